@@ -817,7 +817,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     const long long ids_cap = c.io.ids ? c.io.ids_cap : w.pool_cap;
     CK(launch_k(finalize_kernel, (nq + FIN_WARPS - 1) / FIN_WARPS, 32 * FIN_WARPS, 0, st, pdl, w.d_pool,
                 (const long long*)w.d_cand_off, (const int*)w.d_reg_len, (const int*)w.d_res_count,
-                w.d_out_off, ids, nq, ids_cap, w.d_zb[w.zb_next], w.zb_ints, fs));
+                w.d_out_off, ids, w.d_out, nq, ids_cap, w.d_zb[w.zb_next], w.zb_ints, fs));
     mark(6);
     return RKNN_OK;
 }
@@ -1939,7 +1939,7 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     CK(cudaGetLastError());
     scan_counts_kernel<<<1, 1024, 0, st>>>(L.res_count, L.reg_len, L.region_top, 1, L.out_off, L.counters, nullptr);
     CK(cudaGetLastError());
-    finalize_kernel<<<1, 32 * FIN_WARPS, 0, st>>>(L.pool, L.cand_off, L.reg_len, L.res_count, L.out_off, L.out, 1,
+    finalize_kernel<<<1, 32 * FIN_WARPS, 0, st>>>(L.pool, L.cand_off, L.reg_len, L.res_count, L.out_off, L.out, L.out, 1,
                                                   L.pool_cap, nullptr, 0, FinScan{});
     CK(cudaGetLastError());
 

@@ -93,10 +93,12 @@ struct FinScan {
 // one block per slot: sort the slot's results into out[out_off[s] ...]
 // out may be device-accessible host memory of out_cap ids: a slot whose range
 // would pass out_cap is left out (the caller sees the total and fails the
-// batch).  zero[0 .. zero_n) (another batch's counters, unused by this one)
-// is cleared for the next batch.
+// batch).  stage: device memory for every stored id (at least the total of
+// the result regions), where large sets are sorted; it may be out itself.
+// zero[0 .. zero_n) (another batch's counters, unused by this one) is cleared
+// for the next batch.
 __global__ void finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
-                                int* out_off, int* out, int nq, long long out_cap, int* zero,
+                                int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero,
                                 long long zero_n, FinScan S);
 
 }  // namespace rknn

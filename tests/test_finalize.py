@@ -1,0 +1,41 @@
+"""Result sets of every size class, sorted into each kind of output.
+
+With one facility every user is in its result set, so a set has exactly as
+many ids as there are users, whatever k: the sizes here sit at the edges of
+the sort's classes (32, 64, 128, 256 and 512 ids, and the radix sort beyond).
+"""
+import numpy as np
+import pytest
+
+import rknn
+
+SIZES = [1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 2048, 70_001]
+
+
+def _index(n, ids):
+    rng = np.random.default_rng(n)
+    return rknn.Index(np.array([[500.0, 500.0]], np.float32), rng.uniform(0, 1000, (n, 2)).astype(np.float32),
+                      uid=ids)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", SIZES)
+def test_sorted_ids_in_every_output(n):
+    rng = np.random.default_rng(1000 + n)
+    # ids spread over the whole int32 range, in random order
+    ids = rng.choice(2**32, size=n, replace=False).astype(np.int64) - 2**31
+    ids = ids.astype(np.int32)
+    want = np.tile(np.sort(ids), 3)
+    qs = np.zeros(3, np.int32)
+    with _index(n, ids) as idx:
+        for mode in ("fp32", "fp64"):
+            # page-locked output: staged on the first call, written by the
+            # kernels on the later ones
+            for _ in range(3):
+                got, off = idx.query_batch_flat(qs, 2, mode)
+                assert np.array_equal(off, n * np.arange(4))
+                assert np.array_equal(got, want)
+            # pageable output
+            for got in idx.query_batch(qs, 2, mode):
+                assert np.array_equal(got, want[:n])
+            assert np.array_equal(idx.query(0, 2, mode), want[:n])
