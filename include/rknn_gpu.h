@@ -52,7 +52,9 @@ typedef enum {
 } rknn_status;
 
 typedef enum {
-    RKNN_MODE_FP64 = 0,     /* plain form: predicates filtered in double precision */
+    RKNN_MODE_FP64 = 0,     /* plain form: predicates filtered in double precision (pairs of a
+                               half-plane and a group of users that a certified float test of
+                               the group's bounding box places beyond its error need none) */
     RKNN_MODE_FP32 = 1      /* predicates filtered in float32 with a certified bound */
 } rknn_mode;
 
@@ -97,7 +99,7 @@ typedef struct {
                                facilities offered to the slice heaps) */
     int64_t zone_fp64;      /* intersections computed in double precision */
     int64_t candidates;     /* users tested against the half-planes */
-    int64_t plane_evals;    /* (user, half-plane) evaluations */
+    int64_t plane_evals;    /* (user, half-plane) evaluations, and (box of users, half-plane) ones */
     int64_t survivors;      /* users recounted exactly */
     int64_t fac_checks;     /* (user, facility) comparisons in the exact count */
     int64_t rechecks;       /* comparisons decided by the exact expansion */

@@ -526,9 +526,10 @@ cudaError_t allow_dynamic_smem(const void* fn, int optin)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
 }
 
-// The verification kernel for a users-per-lane setting.
-void (*verify_fn(int upt))(VerifyArgs)
+// The verification kernel for a precision mode and users-per-lane setting.
+void (*verify_fn(int mode, int upt))(VerifyArgs)
 {
+    if (mode == MODE_FP64) return upt == 2 ? verify64_kernel_u2 : upt == 8 ? verify64_kernel_u8 : verify64_kernel;
     return upt == 2 ? verify_kernel_u2 : upt == 8 ? verify_kernel_u8 : verify_kernel;
 }
 
@@ -584,6 +585,7 @@ struct BatchPlan {
     int stage_cap = 0;          // half-planes the verification stages per warp
     int seg_stage = 0;          // user segments it stages per warp
     int vupt = VERIFY_UPT, vwarps = VERIFY_WARPS;
+    int parts = 1;              // parts of 32 vupt users in a verification work item
     bool fuse = false;          // the slice filter verifies its own slots (FP32, every class a slice class)
     size_t vsmem = 0;
     int vgrid = 0;
@@ -613,8 +615,8 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     }
     b.key = {nq, mode, use_order ? 1 : 0};
     // half-planes the verification can stage per warp (128 KB per block at
-    // 32 bytes each: FP64, and the fused filter's pre-duplicated FP32 pairs
-    // for the packed FMA; the verification kernel's FP32 staging is compact)
+    // 32 bytes each: the fused filter's pre-duplicated FP32 pairs for the
+    // packed FMA; the verification kernel's own staging is smaller)
     const int bpp = 32;
     const int stage_max = std::max(1, (128 << 10) / (ix->vwarps * bpp));
     for (auto& c : b.cls) {
@@ -634,6 +636,12 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     // more warps (a lone FP64 query's evaluations are bound by one warp's
     // FP64 issue rate)
     if (nq <= 16 && b.vupt > 2) b.vupt = 2;
+    // batches with more slots than the GPU has verification warps (3,648): a
+    // warp takes up to four parts of a slot in turn and finds the slot, its
+    // segments and half-planes once (verification of 16,384 queries, one part
+    // against four: street layout 1.92 -> 1.75 ms FP32, 3.20 -> 2.94 FP64;
+    // uniform k=10 139 -> 134 us); smaller batches need the items
+    b.parts = nq >= 16384 ? 4 : nq >= 8192 ? 2 : 1;
     b.stage_cap = std::max(1, std::min(b.pstride, stage_max));
     int rm = 0;
     for (auto& c : b.cls) rm = std::max(rm, c.caps.rm);
@@ -653,10 +661,8 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     if (!b.fuse)
         for (auto& c : b.cls) c.zl = zone_launch(ix, c.caps, c.n, c.slice, c.kmax);
     b.key.push_back(b.fuse ? 1 : 0);
-    // (the verification kernel stages FP32 half-planes in 16 bytes)
-    const size_t vbpp = mode == MODE_FP32 ? 16 : (size_t)bpp;
-    b.vsmem = (size_t)b.vwarps * ((size_t)b.stage_cap * vbpp + (size_t)b.seg_stage * sizeof(int2) + 32 * sizeof(float));
-    const int vper = occupancy(ix, (const void*)verify_fn(b.vupt), b.vwarps * 32, b.vsmem);
+    b.vsmem = (size_t)b.vwarps * verify_warp_bytes(b.stage_cap, b.seg_stage);
+    const int vper = occupancy(ix, (const void*)verify_fn(mode, b.vupt), b.vwarps * 32, b.vsmem);
     b.vgrid = vper * ix->num_sms;
     b.key.push_back(b.vupt);
     b.key.push_back(b.vwarps);
@@ -725,6 +731,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     va.qd = w.d_qd; va.planes = w.d_planes; va.bis_pos = w.d_bispos; va.lc = b.pstride;
     va.slice_r = w.d_slice_r;
     va.stage_cap = b.stage_cap;
+    va.parts = b.parts;
     va.segs = w.d_segs; va.seg_cap = w.seg_cap; va.seg_stage = b.seg_stage;
     va.chunk_off = w.d_chunk_off; va.cand_off = w.d_cand_off; va.reg_len = w.d_reg_len; va.nq = nq;
     va.uxy = ix->d_uxy; va.uid = ix->d_uid; va.fxy = ix->d_fxy; va.fstart = ix->d_fstart; va.gf = ix->gf;
@@ -751,7 +758,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
         za.deflist = w.d_deflist;
         za.ndef = w.d_counters + 36;
         za.chunk_off_w = w.d_chunk_off;
-        za.vchunk = 32 * b.vupt;
+        za.vchunk = 32 * b.vupt * b.parts;
         za.done_total = 0;
         for (const ZClass& z : b.cls) za.done_total += z.zl.grid;
         za.v = va;
@@ -794,9 +801,9 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     // and the verification takes only those
     if (!b.fuse)
         CK(launch_k(plan_kernel, 1, 1024, 0, st, pdl && ncls == 1, w.d_qd, nq, w.d_cand_off, w.d_reg_len,
-                    region_top(w), w.d_chunk_off, w.pool_cap, w.rcap, 32 * b.vupt));
+                    region_top(w), w.d_chunk_off, w.pool_cap, w.rcap, 32 * b.vupt * b.parts));
     mark(2);
-    CK(launch_k(verify_fn(b.vupt), b.vgrid, b.vwarps * 32, b.vsmem, st, pdl && (ncls == 1 || !b.fuse), va));
+    CK(launch_k(verify_fn(b.mode, b.vupt), b.vgrid, b.vwarps * 32, b.vsmem, st, pdl && (ncls == 1 || !b.fuse), va));
     mark(3);
     CK(launch_k(recount_kernel, ix->recount_grid, 256, 0, st, pdl, va));
     mark(4);
@@ -1229,9 +1236,9 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
                           (const void*)slice_kernel2_r4, (const void*)slice_kernel2_r8, (const void*)slice_kernel2_r10, (const void*)slice_kernel2_r12,
                           (const void*)slice_kernel2_r16, (const void*)slice_kernel2_r24, (const void*)slice_kernel2_r32})
         CKB(allow_dynamic_smem(f, optin));
-    CKB(allow_dynamic_smem((const void*)verify_kernel, optin));
-    CKB(allow_dynamic_smem((const void*)verify_kernel_u2, optin));
-    CKB(allow_dynamic_smem((const void*)verify_kernel_u8, optin));
+    for (const void* f : {(const void*)verify_kernel, (const void*)verify_kernel_u2, (const void*)verify_kernel_u8,
+                          (const void*)verify64_kernel, (const void*)verify64_kernel_u2, (const void*)verify64_kernel_u8})
+        CKB(allow_dynamic_smem(f, optin));
 
     if (o.users_per_thread != 0 && o.users_per_thread != 2 && o.users_per_thread != 4 && o.users_per_thread != 8)
         return bail(fail(RKNN_ERR_ARG, "users_per_thread must be 2, 4 or 8"));
@@ -1934,8 +1941,8 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     // staging per block); fewer staged planes only send more users to the
     // exact count
     va.stage_cap = std::max(1, std::min(caps.lc, (128 << 10) / (VERIFY_WARPS * 32)));
-    const size_t vsmem = (size_t)VERIFY_WARPS * ((size_t)va.stage_cap * 32 + 32 * sizeof(float));
-    verify_fn(NA_UPT)<<<2 * ix->num_sms, VERIFY_WARPS * 32, vsmem, st>>>(va);
+    const size_t vsmem = (size_t)VERIFY_WARPS * verify_warp_bytes(va.stage_cap, 0);
+    verify_fn(mode, NA_UPT)<<<2 * ix->num_sms, VERIFY_WARPS * 32, vsmem, st>>>(va);
     CK(cudaGetLastError());
     scan_counts_kernel<<<1, 1024, 0, st>>>(L.res_count, L.reg_len, L.region_top, 1, L.out_off, L.counters, nullptr);
     CK(cudaGetLastError());

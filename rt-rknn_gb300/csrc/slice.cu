@@ -232,7 +232,7 @@ __device__ __forceinline__ void fuse_verify(const ZoneArgs& A, int s, const char
     const int wq = NWQ == 2 ? (int)(threadIdx.x >> 5) : 0;
     constexpr int CH = 32 * FUSE_UPT;
     for (int v0 = wq * CH; v0 < d.ncand; v0 += NWQ * CH)
-        vitem::verify_item<FUSE_UPT>(A.v, d, s, v0, smem + FL.planes, sg, Rs, nbs, r0, rl, vc);
+        vitem::verify_item<FUSE_UPT>(A.v, d, s, v0, smem + FL.planes, nbs, nullptr, sg, Rs, nbs, r0, rl, vc);
 }
 
 }  // namespace

@@ -12,7 +12,9 @@
 // exceeds the float (or double) evaluation error of m_f (at most
 // 4.01u(|a x'| + |b y'| + |c|)).  Lanes own users (coalesced float2 loads,
 // four per lane); the warp leaves the half-plane loop as soon as every lane
-// has k certified violations for all its users (__all_sync).
+// has k certified violations for all its users (__all_sync).  In slots of many
+// candidates, and in FP64 always, the users' bounding boxes are tested first
+// (verify_box.cuh).
 //
 // Stage 2 (exact count).  Users that survive stage 1 go to a survivor list,
 // and recount_kernel counts each one exactly, a warp (or a group of up to
@@ -24,16 +26,16 @@
 // error bound, and the undecided ones by the exact expansion predicate.
 // Accepted users are appended to their query's result region.  When the
 // survivor list is full, the warp counts its own survivors, one lane per
-// facility.  The item code itself lives in verify_item.cuh, shared with the
-// slice filter's fused verification.
-#include "verify_item.cuh"
+// facility.  The item code itself lives in verify_item.cuh (the user-by-user
+// form is shared with the slice filter's fused verification).
+#include "verify_box.cuh"
 #include <climits>
 
 namespace rknn {
 
 using namespace vitem;
 
-template <int UPT, bool BITS = false>
+template <int UPT, bool F64>
 __device__ __forceinline__ void verify_body(const VerifyArgs& A)
 {
     extern __shared__ __align__(16) char smem[];
@@ -44,12 +46,12 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
     // a fused batch with no slot left over: nothing to do here
     if (A.deflist && __ldcg(A.ndef) == 0) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // per warp: stage_cap half-planes (16 bytes each in FP32, compact: the
-    // packed pairs are made in registers; 32 in FP64), seg_stage segments,
+    // per warp (verify_warp_bytes): the boxes' scratch, seg_stage segments,
     // the slot's 32 slice bounds
-    const size_t plane_bytes = (size_t)A.stage_cap * (A.mode == MODE_FP32 ? 16 : 32);
-    char* sp = smem + w * (plane_bytes + (size_t)A.seg_stage * sizeof(int2) + 32 * sizeof(float));
-    int2* ssg = (int2*)(sp + plane_bytes);
+    char* wsm = smem + w * verify_warp_bytes(A.stage_cap, A.seg_stage);
+    const BoxScratch BS = {(uint16_t*)(wsm + BOX_STAGE_BYTES + BOX_MASK_BYTES + BOX_QBOX_BYTES), wsm,
+                           (unsigned*)(wsm + BOX_STAGE_BYTES), (float4*)(wsm + BOX_STAGE_BYTES + BOX_MASK_BYTES)};
+    int2* ssg = (int2*)(wsm + verify_box_bytes(A.stage_cap));
     float* sr = (float*)(ssg + A.seg_stage);
     // the listed slots: every slot, or those the fused slice filter left
     const int nl = A.deflist ? __ldcg(A.ndef) : A.nq;
@@ -59,7 +61,8 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
         for (int i = threadIdx.x; i < nsmp; i += blockDim.x) csmp[i] = A.chunk_off[i * st];
     __syncthreads();
     int cur = -1;
-    bool seg_staged = false;
+    bool seg_staged = false, boxed = false;
+    int nsp = 0;
     // per-warp statistics (32-bit here, 64-bit in the totals)
     VCount vc = {};
     const int total = nl > 0 ? A.chunk_off[nl] : 0;
@@ -108,30 +111,38 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
         }
         const int s = A.deflist ? A.deflist[VX(e, A.nq, 222)] : e;
         const QDesc d = A.qd[s];
-        if (s != cur && A.mode == MODE_FP32) {
-            // the slot's half-planes (as many as are staged at most),
-            // seg_stage segments and the slice bounds, each lane's loads
-            // issued together
+        if (s != cur) {
+            // the slot's segments and slice bounds, and the half-planes, each
+            // lane's loads issued together: staged (the first nsp) for the
+            // user-by-user test, brought to L1 (one lane a line) for the boxes
             __syncwarp();
             const float4* src = A.planes + (size_t)s * A.lc;
             const int nst = min(d.nb, A.stage_cap);
-            for (int m0 = lane; m0 < nst; m0 += 32 * 8) {
-                float4 p[8];
+            boxed = F64 || d.ncand >= BOX_MIN_CAND;
+            if (boxed) {
+                if (nst > 0)
+                    for (int m = 8 * lane; m < nst + 7; m += 8 * 32) prefetch_l1(src + min(m, nst - 1));
+            } else {
+                nsp = min(nst, (int)(verify_box_bytes(A.stage_cap) / sizeof(float4)) & ~1);
+                for (int m0 = lane; m0 < nsp; m0 += 32 * 8) {
+                    float4 p[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int m = m0 + 32 * j;
-                    p[j] = m < nst ? src[m] : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+                    for (int j = 0; j < 8; ++j) {
+                        const int m = m0 + 32 * j;
+                        p[j] = m < nsp ? src[m] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int m = m0 + 32 * j;
-                    if (m < nst) ((float4*)sp)[m] = p[j];
+                    for (int j = 0; j < 8; ++j) {
+                        const int m = m0 + 32 * j;
+                        if (m < nsp) ((float4*)wsm)[m] = p[j];
+                    }
                 }
             }
             // the slot's segments (nseg ranges and the terminal entry), when
             // they fit; the record has arrived with the half-planes in flight
             const int2* gsg = A.segs + (size_t)s * A.seg_cap;
-            const int nss = d.nseg + 1 <= A.seg_stage ? d.nseg + 1 : 0;
+            seg_staged = d.nseg + 1 <= A.seg_stage;
+            const int nss = seg_staged ? d.nseg + 1 : 0;
             for (int m0 = lane; m0 < nss; m0 += 32 * 8) {
                 int2 e[8];
 #pragma unroll
@@ -144,45 +155,41 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
                     if (m0 + 32 * j < nss) ssg[m0 + 32 * j] = e[j];
             }
             if (A.slice_r) sr[lane] = A.slice_r[(size_t)s * 32 + lane];
-        }
-        if (s != cur) {
-            if (A.mode == MODE_FP32) {
-                seg_staged = d.nseg + 1 <= A.seg_stage;
-            } else {
-                __syncwarp();
-                const int* bp = A.bis_pos + (size_t)s * A.lc;
-                for (int m = lane; m < min(d.nb, A.stage_cap); m += 32) {
-                    float2 f = A.fxy[VX(bp[m], A.nf, 204)];
-                    double dx = (double)f.x - (double)d.qx, dy = (double)f.y - (double)d.qy;
-                    double* p = (double*)sp + 4 * m;
-                    p[0] = -2.0 * dx;
-                    p[1] = -2.0 * dy;
-                    p[2] = fma(dx, dx, dy * dy);
-                    p[3] = (double)A.planes[(size_t)s * A.lc + m].w;
-                }
-                // the slot's user segments (nseg ranges and the terminal entry)
-                seg_staged = d.nseg + 1 <= A.seg_stage;
-                if (seg_staged) {
-                    const int2* gsg = A.segs + (size_t)s * A.seg_cap;
-                    for (int m = lane; m <= d.nseg; m += 32) ssg[m] = gsg[m];
-                }
-                if (A.slice_r) sr[lane] = A.slice_r[(size_t)s * 32 + lane];
-            }
             cur = s;
             __syncwarp();
         }
-        const int v0 = (g - c_off) * (32 * UPT);
         const int2* sg = seg_staged ? ssg : A.segs + (size_t)s * A.seg_cap;
-        verify_item<UPT, true, BITS>(A, d, s, v0, sp, sg, sr, min(d.nb, A.stage_cap), -1, -1, vc);
+        const int nbs = min(d.nb, A.stage_cap);
+        const float4* gp = A.planes + (size_t)s * A.lc;
+        const float rho2 = item_rho2(d, nbs);
+        // a work item is A.parts parts of 32 UPT users
+        const int vbeg = (g - c_off) * (32 * UPT * A.parts), vend = min(vbeg + 32 * UPT * A.parts, d.ncand);
+        for (int v0 = vbeg; v0 < vend; v0 += 32 * UPT) {
+            if (!boxed) {
+                if constexpr (!F64) verify_item<UPT, true>(A, d, s, v0, wsm, nsp, gp, sg, sr, nbs, -1, -1, vc);
+                continue;
+            }
+            int pos[UPT];
+            float2 u[UPT];
+            bool valid[UPT], direct[UPT], surv[UPT];
+            item_users<UPT>(A, d, s, v0, sg, sr, false, pos, u, valid, vc);
+            filter_boxed<UPT, F64>(A, d, nbs, gp, A.bis_pos + (size_t)s * A.lc, BS, u, valid, direct, surv, vc.evals,
+                                   rho2);
+            item_emit<UPT, F64>(A, d, s, pos, direct, surv, -1, -1, vc);
+        }
     }
     vc.flush(A.vstats);
 }
 
 // The verification kernel with 2, 4 or 8 users per lane per work item
-// (32 * UPT users per item); blocks of up to 16 warps.
-__global__ void __maxnreg__(80) verify_kernel(VerifyArgs a) { verify_body<4>(a); }
-__global__ void __maxnreg__(80) verify_kernel_u2(VerifyArgs a) { verify_body<2, true>(a); }
-__global__ void __launch_bounds__(512) verify_kernel_u8(VerifyArgs a) { verify_body<8>(a); }
+// (32 * UPT users per item), for either precision mode; blocks of up to 16
+// warps.
+__global__ void __maxnreg__(80) verify_kernel(VerifyArgs a) { verify_body<4, false>(a); }
+__global__ void __maxnreg__(80) verify_kernel_u2(VerifyArgs a) { verify_body<2, false>(a); }
+__global__ void __launch_bounds__(512) verify_kernel_u8(VerifyArgs a) { verify_body<8, false>(a); }
+__global__ void __launch_bounds__(512) verify64_kernel(VerifyArgs a) { verify_body<4, true>(a); }
+__global__ void __launch_bounds__(512) verify64_kernel_u2(VerifyArgs a) { verify_body<2, true>(a); }
+__global__ void __launch_bounds__(512) verify64_kernel_u8(VerifyArgs a) { verify_body<8, true>(a); }
 
 // One warp per listed survivor.  Lane r computes the facility range of
 // disc row r (trimmed to the chord), a warp prefix sum flattens the rows,

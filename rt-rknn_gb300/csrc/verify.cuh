@@ -7,7 +7,8 @@ namespace rknn {
 constexpr int VERIFY_UPT = 4;                       // default users per lane per work item
 constexpr int VERIFY_CHUNK = 32 * VERIFY_UPT;       // default users per work item
 constexpr int VERIFY_WARPS = 8;                     // default warps per block
-constexpr int VERIFY_SAMPLES = 4096;                // work-item offsets cached per block
+constexpr int VERIFY_SAMPLES = 1024;                // work-item offsets cached per block
+constexpr int BOX_MIN_CAND = 512;                   // FP32: candidates from which boxes come first
 constexpr int FIN_WARPS = 8;                        // finalize: slots per block (one warp each)
 constexpr int FIN_WCAP = 512;                       // ids one warp sorts in registers
 
@@ -18,8 +19,9 @@ struct VerifyArgs {
     const float4* planes;    // [slot][lc] float half-planes relative to q
     const int* bis_pos;      // [slot][lc] facility positions (FP64 planes are rebuilt from these)
     int lc;                  // row stride of planes / bis_pos
-    int stage_cap;           // half-planes staged per warp (the filter uses the first ones;
+    int stage_cap;           // half-planes used per slot, at most 1024 (the first ones;
                              // fewer only means more users reach the exact recount)
+    int parts = 1;           // parts of 32 * (users per lane) users in a work item
     const int2* segs;        // [slot][seg_cap]
     int seg_cap;
     int seg_stage = 0;       // user segments staged per warp beside the half-planes
@@ -54,9 +56,28 @@ struct VerifyArgs {
     int* done = nullptr;               // fused filter: its blocks finished
 };
 
-__global__ void verify_kernel(VerifyArgs a);        // 4 users per lane per work item
+__global__ void verify_kernel(VerifyArgs a);        // FP32, 4 users per lane per work item
 __global__ void verify_kernel_u2(VerifyArgs a);     // 2
 __global__ void verify_kernel_u8(VerifyArgs a);     // 8
+__global__ void verify64_kernel(VerifyArgs a);      // FP64, 4 users per lane per work item
+__global__ void verify64_kernel_u2(VerifyArgs a);   // 2
+__global__ void verify64_kernel_u8(VerifyArgs a);   // 8
+
+// Shared memory of one warp of a verification kernel: the box filter's 32
+// staged half-planes (three doubles each at most), its masks, boxes and list
+// of half-plane indices; the segments; the slice bounds.
+constexpr int BOX_STAGE_BYTES = 32 * 3 * (int)sizeof(double);
+constexpr int BOX_MASK_BYTES = 4 * 32 * (int)sizeof(unsigned);
+constexpr int BOX_QBOX_BYTES = 4 * 2 * (int)sizeof(float4);
+__host__ __device__ __forceinline__ size_t verify_box_bytes(int stage_cap)
+{
+    return BOX_STAGE_BYTES + BOX_MASK_BYTES + BOX_QBOX_BYTES + (((size_t)stage_cap * sizeof(uint16_t) + 15) & ~(size_t)15);
+}
+__host__ __device__ __forceinline__ size_t verify_warp_bytes(int stage_cap, int seg_stage)
+{
+    const size_t b = verify_box_bytes(stage_cap) + (size_t)seg_stage * sizeof(int2) + 32 * sizeof(float);
+    return (b + 15) & ~(size_t)15;
+}
 
 // exact recount of the listed survivors, one thread each
 __global__ void recount_kernel(VerifyArgs a);

@@ -71,15 +71,23 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
     return cnt;
 }
 
-// Stage 1 over the first nb staged half-planes: cnt = certified
+// Above 4|u - q|^2 with margin, for the user at offset (x, y) from q.
+__device__ __forceinline__ float user_lim(float x, float y)
+{
+    return 4.0f * fmaf(x, x, y * y) * (1.0f + 1e-4f) + 1e-30f;
+}
+
+// Stage 1, FP32, over the slot's first nb half-planes: cnt = certified
 // violations (the loop leaves once every lane's users reached k), und =
-// half-planes the bound could not decide.
-template <typename T, int UPT, bool COMPACT, bool BITS = false>
-__device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char* sp, const int* pos,
+// half-planes the bound could not decide.  sp: the first ns of them staged;
+// gp: all of them in global memory (COMPACT; the loop seldom gets beyond
+// those staged).
+template <int UPT, bool COMPACT>
+__device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char* sp, int ns, const float4* gp,
                                              const float2* u, const bool* valid, int* cnt, int* und,
                                              unsigned& evals, float rho2)
 {
-    T x[UPT], y[UPT], bu[UPT];
+    float x[UPT], y[UPT], bu[UPT];
     // und[t] on return: the half-planes alone do not decide user t, because
     // one was too close to call or the user lies beyond rho/2 of q (then a
     // facility strictly nearer to it need not be a half-plane; rho2 is
@@ -94,72 +102,65 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {
         cnt[t] = valid[t] ? 0 : INT_MAX / 2;
-        und[t] = 0;
         nvalid += valid[t];
-        const float fx = u[t].x - d.qx, fy = u[t].y - d.qy;
-        lim[t] = 4.0f * fmaf(fx, fx, fy * fy) * (1.0f + 1e-4f) + 1e-30f;
-        if (sizeof(T) == 4) {
-            x[t] = fx; y[t] = fy;
-            bu[t] = fmaf(d.k2f, fabsf(fx) + fabsf(fy), d.kf2);
-        } else {
-            double xx = (double)u[t].x - (double)d.qx, yy = (double)u[t].y - (double)d.qy;
-            x[t] = (T)xx; y[t] = (T)yy;
-            bu[t] = (T)fma(d.k2f64, fabs(xx) + fabs(yy), d.kf264);
-        }
+        x[t] = u[t].x - d.qx;
+        y[t] = u[t].y - d.qy;
+        lim[t] = user_lim(x[t], y[t]);
+        bu[t] = fmaf(d.k2f, fabsf(x[t]) + fabsf(y[t]), d.kf2);
     }
     const int k = d.k;
     int m = 0;
-    if constexpr (sizeof(T) == 4) {
-        // FP32: users in pairs through the packed FMA (each half rounds as
-        // fmaf); half-plane m is staged as (a, a, b, b), (c, c, w, w), or,
-        // COMPACT, as (a, b, c, w), the pairs made in registers (half the
-        // shared memory: twice the warps per SM where the staging bounds it).  With
-        // r = fl(mv + bu): mv < -bu exactly when r is negative (a nonzero
-        // exact sum of two floats never rounds to zero, and bu > 0 rules out
-        // -0), and |mv| <= bu implies 0 <= r <= 2bu (rounding is monotone):
-        // the smallest non-negative r, taken as the least unsigned bit
-        // pattern (negative floats have the sign bit set), at most 2bu
-        // (rounded up) flags a half-plane too close to call.  That test may
-        // also flag a few decided ones; such users are only recounted.
-        constexpr int H2 = UPT / 2;
-        float2 X[H2], Y[H2], B[H2];
-        unsigned rmin[UPT];
+    // Users in pairs through the packed FMA (each half rounds as fmaf);
+    // half-plane m is staged as (a, a, b, b), (c, c, w, w), or, COMPACT, as
+    // (a, b, c, w), the pairs made in registers (half the shared memory:
+    // twice the warps per SM where the staging bounds it).  With
+    // r = fl(mv + bu): mv < -bu exactly when r is negative (a nonzero exact
+    // sum of two floats never rounds to zero, and bu > 0 rules out -0), and
+    // |mv| <= bu implies 0 <= r <= 2bu (rounding is monotone): the smallest
+    // non-negative r, taken as the least unsigned bit pattern (negative
+    // floats have the sign bit set), at most 2bu (rounded up) flags a
+    // half-plane too close to call.  That test may also flag a few decided
+    // ones; such users are only recounted.
+    constexpr int H2 = UPT / 2;
+    float2 X[H2], Y[H2], B[H2];
+    unsigned rmin[UPT];
+#pragma unroll
+    for (int h = 0; h < H2; ++h) {
+        X[h] = make_float2(x[2 * h], x[2 * h + 1]);
+        Y[h] = make_float2(y[2 * h], y[2 * h + 1]);
+        B[h] = make_float2(bu[2 * h], bu[2 * h + 1]);
+    }
+#pragma unroll
+    for (int t = 0; t < UPT; ++t) rmin[t] = 0xffffffffu;
+    auto plane = [&](const float4 ab, const float4 cw) {
+        const float2 a2 = make_float2(ab.x, ab.y), b2 = make_float2(ab.z, ab.w), c2 = make_float2(cw.x, cw.y);
 #pragma unroll
         for (int h = 0; h < H2; ++h) {
-            X[h] = make_float2((float)x[2 * h], (float)x[2 * h + 1]);
-            Y[h] = make_float2((float)y[2 * h], (float)y[2 * h + 1]);
-            B[h] = make_float2((float)bu[2 * h], (float)bu[2 * h + 1]);
+            const float2 mv = __ffma2_rn(a2, X[h], __ffma2_rn(b2, Y[h], c2));
+            const float2 r = __fadd2_rn(mv, B[h]);
+            const unsigned rx = __float_as_uint(r.x), ry = __float_as_uint(r.y);
+            cnt[2 * h] += (int)(rx >> 31);
+            cnt[2 * h + 1] += (int)(ry >> 31);
+            rmin[2 * h] = min(rmin[2 * h], rx);
+            rmin[2 * h + 1] = min(rmin[2 * h + 1], ry);
         }
-#pragma unroll
-        for (int t = 0; t < UPT; ++t) rmin[t] = 0xffffffffu;
-        const float4* sp4 = (const float4*)sp;
-        auto plane = [&](const float4 ab, const float4 cw) {
-            const float2 a2 = make_float2(ab.x, ab.y), b2 = make_float2(ab.z, ab.w), c2 = make_float2(cw.x, cw.y);
-#pragma unroll
-            for (int h = 0; h < H2; ++h) {
-                const float2 mv = __ffma2_rn(a2, X[h], __ffma2_rn(b2, Y[h], c2));
-                const float2 r = __fadd2_rn(mv, B[h]);
-                const unsigned rx = __float_as_uint(r.x), ry = __float_as_uint(r.y);
-                cnt[2 * h] += (int)(rx >> 31);
-                cnt[2 * h + 1] += (int)(ry >> 31);
-                rmin[2 * h] = min(rmin[2 * h], rx);
-                rmin[2 * h + 1] = min(rmin[2 * h + 1], ry);
-            }
-        };
-        // two half-planes a trip (the second one's loads overlap the first
-        // one's arithmetic); the early exit is tested after every eighth
-        bool stopped = false;
+    };
+    // two half-planes a trip (the second one's loads overlap the first
+    // one's arithmetic); the early exit is tested after every eighth.  ns is
+    // even unless it is nb.
+    bool stopped = false;
+    auto sweep = [&](const float4* p4, int end) {
         auto load = [&](int i, float4& ab, float4& cw) {
             if constexpr (COMPACT) {
-                const float4 p = sp4[i];
+                const float4 p = p4[i];
                 ab = make_float4(p.x, p.x, p.y, p.y);
                 cw = make_float4(p.z, p.z, p.w, p.w);
             } else {
-                ab = sp4[2 * i];
-                cw = sp4[2 * i + 1];
+                ab = p4[2 * i];
+                cw = p4[2 * i + 1];
             }
         };
-        for (; m + 2 <= nb; m += 2) {
+        for (; m + 2 <= end; m += 2) {
             float4 ab0, cw0, ab1, cw1;
             load(m, ab0, cw0);
             load(m + 1, ab1, cw1);
@@ -172,59 +173,19 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
                 if (__all_sync(FULL, done)) { m += 2; stopped = true; break; }
             }
         }
-        if (!stopped && m < nb) {
+        if (!stopped && m < end) {
             float4 ab, cw;
             load(m, ab, cw);
             plane(ab, cw);
             ++m;
         }
+    };
+    sweep((const float4*)sp, ns);
+    if constexpr (COMPACT)
+        if (!stopped && ns < nb) sweep(gp, nb);
 #pragma unroll
-        for (int t = 0; t < UPT; ++t)
-            und[t] = rmin[t] <= __float_as_uint(__fmul_ru((float)bu[t], 2.0f * (1.0f + 0x1p-20f))) || lim[t] > rho2;
-        evals += (unsigned)(m * nvalid);
-        return;
-    }
-    // FP64 with BITS: the compares of each evaluation on the bits (integer
-    // pipes).  A warp's FP64 instruction holds its sub-partition's FP64 pipe
-    // for about 64 cycles on GB300, so a lone query's evaluations, two FMAs
-    // and three compares each, are bound by that pipe; in large batches the
-    // extra registers cost more than the compares (the kernels with four
-    // and eight users a lane spill).  mv is finite (finite half-planes and
-    // users) and bu >= kf264 > 0, so mv < -bu is order_key(mv) < ~bits(bu),
-    // and -bu <= mv <= bu is |mv| <= bu on the magnitude bits.
-    for (; m < nb; ++m) {
-        T a, b, c;
-        float wm;
-        if (sizeof(T) == 4) {
-            float4 p = ((const float4*)sp)[m];
-            a = (T)p.x; b = (T)p.y; c = (T)p.z;
-            wm = p.w;
-        } else {
-            const double* p = (const double*)sp + 4 * m;
-            a = (T)p[0]; b = (T)p[1]; c = (T)p[2];
-            wm = (float)p[3];       // a float to begin with
-        }
-#pragma unroll
-        for (int t = 0; t < UPT; ++t) {
-            T mv = fma(a, x[t], fma(b, y[t], c));
-            if constexpr (BITS && sizeof(T) == 8) {
-                const long long bb = __double_as_longlong((double)bu[t]);
-                cnt[t] += order_key((double)mv) < ~bb;
-                und[t] += (__double_as_longlong((double)mv) & 0x7fffffffffffffffll) <= bb;
-            } else {
-                cnt[t] += (mv < -bu[t]);
-                und[t] += (mv <= bu[t]) & (mv >= -bu[t]);
-            }
-        }
-        if ((m & 7) == 7) {
-            bool done = true;
-#pragma unroll
-            for (int t = 0; t < UPT; ++t) done &= cnt[t] >= k || wm > lim[t];
-            if (__all_sync(FULL, done)) { ++m; break; }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < UPT; ++t) und[t] |= lim[t] > rho2;
+    for (int t = 0; t < UPT; ++t)
+        und[t] = rmin[t] <= __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f))) || lim[t] > rho2;
     evals += (unsigned)(m * nvalid);
 }
 
@@ -311,15 +272,13 @@ struct VCount {
     }
 };
 
-// Item of slot s starting at candidate v0.  sp: the slot's first nbs
-// half-planes staged (FP32: 32 bytes each as (a, a, b, b), (c, c, w, w);
-// FP64: four doubles), sg: its segments (shared or global memory), sr: its
-// 32 slice bounds.  r0_in/region_in: the slot's result region, or -1 to read
-// it from cand_off/reg_len.
-template <int UPT, bool COMPACT = false, bool BITS = false>
-__device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d, int s, int v0, const char* sp,
-                                            const int2* sg, const float* sr, int nbs, long long r0_in,
-                                            long long region_in, VCount& vc)
+// The item's users: lane's user t is candidate v0 + 32 t + lane of slot s.
+// sg: the slot's segments, sr: its 32 slice bounds.  valid[t] on return: the
+// candidate exists and lies within its slice's bound.
+template <int UPT>
+__device__ __forceinline__ void item_users(const VerifyArgs& A, const QDesc& d, int s, int v0, const int2* sg,
+                                           const float* sr, bool region_known, int* pos, float2* u, bool* valid,
+                                           VCount& vc)
 {
     const int lane = threadIdx.x & 31;
     // user v's segment: the largest i < nseg with sg[i].y <= v (sg[0].y
@@ -335,9 +294,6 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
             if (sg[b[t] + half].y <= v0 + t * 32 + lane) b[t] += half;
         n -= half;
     }
-    int pos[UPT];
-    float2 u[UPT];
-    bool valid[UPT];
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {
         const int v = v0 + t * 32 + lane;
@@ -356,7 +312,7 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
 #pragma unroll
     for (int t = 0; t < UPT; ++t)
         if (valid[t]) prefetch_l1(A.uid + pos[t]);
-    if (lane == 0 && region_in < 0) {
+    if (lane == 0 && !region_known) {
         prefetch_l1(A.cand_off + s);
         prefetch_l1(A.reg_len + s);
     }
@@ -374,19 +330,27 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
             if (fmaf(dx, dx, dy * dy) * (1.0f - 1e-6f) > Rs * Rs) valid[t] = false;
         }
     }
-    int cnt[UPT], und[UPT];
-    // A user within rho/2 of q is decided by the half-planes alone: every
-    // facility strictly nearer to it than q lies within 2|u-q| <= rho of
-    // q, so it is a half-plane.  With no undecided half-plane the
-    // certified count is the exact count.  (All half-planes must be
-    // staged for this.)
-    const float rho2 = (nbs == d.nb) ? d.rho * d.rho * (1.0f - 1e-5f) : 0.0f;
-    if (A.mode == MODE_FP32) filter_users<float, UPT, COMPACT>(d, nbs, sp, pos, u, valid, cnt, und, vc.evals, rho2);
-    else filter_users<double, UPT, false, BITS>(d, nbs, sp, pos, u, valid, cnt, und, vc.evals, rho2);
-    bool direct[UPT];
-#pragma unroll
-    for (int t = 0; t < UPT; ++t) direct[t] = valid[t] && cnt[t] < d.k && und[t] == 0;
+}
 
+// (rho/2)^2 scaled by 4: a user within rho/2 of q is decided by the
+// half-planes alone: every facility strictly nearer to it than q lies within
+// 2|u-q| <= rho of q, so it is a half-plane.  With no undecided half-plane
+// the certified count is the exact count.  (All half-planes must be staged
+// for this: 0 otherwise.)
+__device__ __forceinline__ float item_rho2(const QDesc& d, int nbs)
+{
+    return nbs == d.nb ? d.rho * d.rho * (1.0f - 1e-5f) : 0.0f;
+}
+
+// Stage 2 of an item of slot s: direct[t] users are results, surv[t] users
+// are left to the exact count.  r0_in/region_in: the slot's result region,
+// or -1 to read it from cand_off/reg_len.
+template <int UPT, bool F64>
+__device__ __forceinline__ void item_emit(const VerifyArgs& A, const QDesc& d, int s, const int* pos,
+                                          const bool* direct, const bool* surv, long long r0_in,
+                                          long long region_in, VCount& vc)
+{
+    const int lane = threadIdx.x & 31;
     // stage 2: survivors go to the list for recount_kernel (when it is
     // full, the warp counts them itself, one user at a time); directly
     // accepted users are appended to the slot's results.  The accepted
@@ -398,7 +362,7 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {
         idv[t] = direct[t] ? A.uid[VX(pos[t], A.nu, 207)] : 0;
-        sm[t] = __ballot_sync(FULL, valid[t] && cnt[t] < d.k && !direct[t]);
+        sm[t] = __ballot_sync(FULL, surv[t]);
         am[t] = __ballot_sync(FULL, direct[t]);
         ns += __popc(sm[t]);
         tot += __popc(am[t]);
@@ -444,44 +408,63 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
         vc.res += (lane == 0) ? tot : 0;
     }
     if (!listed && ns) {
-        // survivors the list could not take: counted here, appended with
-        // one more reservation
-        bool acc[UPT];
-#pragma unroll
+        // survivors the list could not take: counted here, one at a time
+        // (rare; one copy of the code for all t)
+#pragma unroll 1
         for (int t = 0; t < UPT; ++t) {
-            acc[t] = false;
-            unsigned m = sm[t];
+            unsigned m = sm[0];
+            int pt = pos[0];
+#pragma unroll
+            for (int i = 1; i < UPT; ++i)
+                if (t == i) { m = sm[i]; pt = pos[i]; }
+            bool acc = false;
             while (m) {
-                int l = __ffs(m) - 1;
+                const int l = __ffs(m) - 1;
                 m &= m - 1;
-                const float2 ul = A.uxy[VX(__shfl_sync(FULL, pos[t], l), A.nu, 219)];
+                const float2 ul = A.uxy[VX(__shfl_sync(FULL, pt, l), A.nu, 219)];
                 unsigned long long fac = 0, rech = 0;
-                int c = (A.mode == MODE_FP32) ? exact_count<float>(ul.x, ul.y, d, A, fac, rech)
-                                              : exact_count<double>(ul.x, ul.y, d, A, fac, rech);
+                const int c = F64 ? exact_count<double>(ul.x, ul.y, d, A, fac, rech)
+                                  : exact_count<float>(ul.x, ul.y, d, A, fac, rech);
                 vc.fac += (unsigned)fac;
                 vc.rech += (unsigned)rech;
-                if (lane == l) acc[t] = c < d.k;
+                if (lane == l) acc = c < d.k;
             }
-        }
-        unsigned bm[UPT];
-        int tot2 = 0;
-#pragma unroll
-        for (int t = 0; t < UPT; ++t) { bm[t] = __ballot_sync(FULL, acc[t]); tot2 += __popc(bm[t]); }
-        if (tot2) {
+            const unsigned bm = __ballot_sync(FULL, acc);
+            if (!bm) continue;
+            const int tot2 = __popc(bm);
             int base = 0;
             if (lane == 0) base = atomicAdd(A.res_count + s, tot2);
             base = __shfl_sync(FULL, base, 0);
             if (lane == 0 && base + tot2 > region) atomicOr(A.dropped, 1);
-            int o = 0;
-#pragma unroll
-            for (int t = 0; t < UPT; ++t) {
-                const long long at = (long long)base + o + __popc(bm[t] & ((1u << lane) - 1));
-                if (acc[t] && at < region) A.res_pool[VX(r0 + at, A.pool_cap, 220)] = A.uid[VX(pos[t], A.nu, 221)];
-                o += __popc(bm[t]);
-            }
+            const long long at = (long long)base + __popc(bm & ((1u << lane) - 1));
+            if (acc && at < region) A.res_pool[VX(r0 + at, A.pool_cap, 220)] = A.uid[VX(pt, A.nu, 221)];
             vc.res += (lane == 0) ? tot2 : 0;
         }
     }
+}
+
+// FP32 item of slot s starting at candidate v0.  sp, ns, gp: the slot's first
+// nbs half-planes (see filter_users), sg: its segments (shared or global
+// memory), sr: its 32 slice bounds.  r0_in/region_in: the slot's result
+// region, or -1 to read it from cand_off/reg_len.
+template <int UPT, bool COMPACT = false>
+__device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d, int s, int v0, const char* sp,
+                                            int ns, const float4* gp, const int2* sg, const float* sr, int nbs,
+                                            long long r0_in, long long region_in, VCount& vc)
+{
+    int pos[UPT];
+    float2 u[UPT];
+    bool valid[UPT];
+    item_users<UPT>(A, d, s, v0, sg, sr, region_in >= 0, pos, u, valid, vc);
+    int cnt[UPT], und[UPT];
+    filter_users<UPT, COMPACT>(d, nbs, sp, ns, gp, u, valid, cnt, und, vc.evals, item_rho2(d, nbs));
+    bool direct[UPT], surv[UPT];
+#pragma unroll
+    for (int t = 0; t < UPT; ++t) {
+        direct[t] = valid[t] && cnt[t] < d.k && und[t] == 0;
+        surv[t] = valid[t] && cnt[t] < d.k && und[t] != 0;
+    }
+    item_emit<UPT, false>(A, d, s, pos, direct, surv, r0_in, region_in, vc);
 }
 
 }  // namespace vitem
