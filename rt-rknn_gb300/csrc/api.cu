@@ -100,7 +100,7 @@ constexpr int FUSE_CAND = 4096;
 constexpr int ZB_VSTATS_INTS = 32;  // room for the statistics after them
 // counter ints: 1 verification work, 2 dropped, 3 listed survivors, 4-8 and
 // 10-14 bounds-check records, 16-31 slice filter work per k class, 36
-// slots the fused filter left over, 37 its blocks done, 40-41 the 64-bit
+// slots the fused filter left over, 37 its blocks done, 38 recount work, 40-41 the 64-bit
 // result-region total
 
 struct Workspace {
@@ -552,16 +552,22 @@ struct ZClass {
 };
 
 // Capacities of the slice filter: a k-entry heap per slice, half-planes of
-// the nearest facilities for the verification (no more than it stages, so
+// the nearest facilities for the verification (no more than it uses, so
 // that all of them take part in its exact shortcut).
-ZoneCaps slice_caps(int kmax, int lc_cap = 512)
+ZoneCaps slice_caps(int kmax)
 {
     ZoneCaps c;
     c.vc = std::max(1, kmax);
     // half-planes: the first 24 k + 60 facilities streamed (more half-planes
     // reach farther: fewer users left to the exact recount; at k=10 on the
-    // uniform workload 0.03 a query instead of 0.53 with 10 k + 60)
-    c.lc = (int)std::max<long long>(1, std::min<long long>(24LL * c.vc + 60, lc_cap));
+    // uniform workload 0.03 a query instead of 0.53 with 10 k + 60), up to
+    // 8 k of them and at least 512, at most the verification's 1024: a user at
+    // the region's edge needs the about 4 k facilities within twice its
+    // distance to q.  Street workload, k up to 100: 68 users a query recounted
+    // with at most 512 (0.81 ms FP32, 2.31 FP64), 2 with 768 (0.03), at 0.04
+    // ms more in the filter.
+    const long long most = std::min<long long>(std::max<long long>(8LL * c.vc, 512), VERIFY_PLANES_MAX);
+    c.lc = (int)std::max<long long>(1, std::min<long long>(24LL * c.vc + 60, most));
     c.pc = 0;
     c.rm = 64;
     return c;
@@ -582,7 +588,7 @@ struct BatchPlan {
     bool use_order = false;
     std::vector<ZClass> cls;
     int pstride = 0;            // half-plane row stride: the largest class lc
-    int stage_cap = 0;          // half-planes the verification stages per warp
+    int stage_cap = 0;          // half-planes the verification uses per slot
     int seg_stage = 0;          // user segments it stages per warp
     int vupt = VERIFY_UPT, vwarps = VERIFY_WARPS;
     int parts = 1;              // parts of 32 vupt users in a verification work item
@@ -614,22 +620,14 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
         b.cls.push_back(ZClass{0, nq, std::max(1, kmax), false, {}, {}});
     }
     b.key = {nq, mode, use_order ? 1 : 0};
-    // half-planes the verification can stage per warp (128 KB per block at
-    // 32 bytes each: the fused filter's pre-duplicated FP32 pairs for the
-    // packed FMA; the verification kernel's own staging is smaller)
-    const int bpp = 32;
-    const int stage_max = std::max(1, (128 << 10) / (ix->vwarps * bpp));
     for (auto& c : b.cls) {
         c.slice = use_slice(ix, c.kmax);
-        c.caps = c.slice ? slice_caps(c.kmax, std::min(512, stage_max)) : caps_fit(ix, caps_for(c.kmax));
+        c.caps = c.slice ? slice_caps(c.kmax) : caps_fit(ix, caps_for(c.kmax));
         b.pstride = std::max(b.pstride, c.caps.lc);
         b.key.push_back(c.n);
         b.key.push_back(c.kmax);
         b.key.push_back(c.slice ? 1 : 0);
     }
-    // the verification stages each query's half-planes in shared memory, at
-    // most 96 KB per block (a longer list is cut: the filter weakens, the
-    // exact recount still decides)
     b.vupt = ix->vupt;
     b.vwarps = ix->vwarps;
     // a handful of queries: smaller work items spread each query's users over
@@ -642,7 +640,9 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     // against four: street layout 1.92 -> 1.75 ms FP32, 3.20 -> 2.94 FP64;
     // uniform k=10 139 -> 134 us); smaller batches need the items
     b.parts = nq >= 16384 ? 4 : nq >= 8192 ? 2 : 1;
-    b.stage_cap = std::max(1, std::min(b.pstride, stage_max));
+    // (half-planes beyond these are left out: the filter weakens, the exact
+    // recount still decides)
+    b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
     int rm = 0;
     for (auto& c : b.cls) rm = std::max(rm, c.caps.rm);
     b.seg_stage = std::min(2 * rm + 2, 512);
@@ -740,6 +740,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     va.nu = (int)ix->nu; va.nf = (int)ix->nf; va.ncf = ix->gf.gx * ix->gf.gy;
     va.pool_cap = w.pool_cap; va.fault = w.d_counters + 10; va.dropped = w.d_counters + 2;
     va.surv = w.d_surv; va.surv_cap = (int)std::min<long long>(w.surv_cap, INT32_MAX); va.surv_count = w.d_counters + 3;
+    va.recount_counter = w.d_counters + 38;
     va.region_top = region_top(w);
     if (b.fuse) {
         // the verification takes only the slots the filter left over
@@ -805,7 +806,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     mark(2);
     CK(launch_k(verify_fn(b.mode, b.vupt), b.vgrid, b.vwarps * 32, b.vsmem, st, pdl && (ncls == 1 || !b.fuse), va));
     mark(3);
-    CK(launch_k(recount_kernel, ix->recount_grid, 256, 0, st, pdl, va));
+    CK(launch_k(b.mode == MODE_FP64 ? recount64_kernel : recount_kernel, ix->recount_grid, 256, 0, st, pdl, va));
     mark(4);
     // the output offsets: in finalize itself for batches of up to
     // FIN_SCAN_MAX slots, else by the scan kernel
@@ -1937,10 +1938,7 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     va.nu = (int)ix->nu; va.nf = (int)ix->nf; va.ncf = ix->gf.gx * ix->gf.gy;
     va.pool_cap = L.pool_cap; va.fault = L.counters + 10; va.dropped = L.counters + 2;
     va.surv = nullptr; va.surv_cap = 0; va.surv_count = L.counters + 3;
-    // at most 512 half-planes staged per warp, as in batches (128 KB of
-    // staging per block); fewer staged planes only send more users to the
-    // exact count
-    va.stage_cap = std::max(1, std::min(caps.lc, (128 << 10) / (VERIFY_WARPS * 32)));
+    va.stage_cap = std::max(1, std::min(caps.lc, VERIFY_PLANES_MAX));
     const size_t vsmem = (size_t)VERIFY_WARPS * verify_warp_bytes(va.stage_cap, 0);
     verify_fn(mode, NA_UPT)<<<2 * ix->num_sms, VERIFY_WARPS * 32, vsmem, st>>>(va);
     CK(cudaGetLastError());

@@ -269,17 +269,38 @@ __device__ __forceinline__ bool closer_f32(float ux, float uy, float fx, float f
     return sign_d2diff_exact(ux, uy, fx, fy, qx, qy) < 0;
 }
 
-// Same decision with a double-precision filter (the plain FP64 form).
-__device__ __forceinline__ bool closer_f64(float ux, float uy, float fx, float fy,
-                                           float qx, float qy, double Dq,
-                                           unsigned long long* rechecks)
+// The double-precision filter of the plain FP64 form, for one user: the
+// squared distance to q and the thresholds that decide the comparison with
+// another one.  Each computed squared distance carries a relative error below
+// (1+u)^5-1, so Df < lo = Dq (1 - 16u) certifies f nearer and Df > hi =
+// Dq (1 + 16u) certifies it not nearer.  Kept as bits: squared distances are
+// not negative, so doubles compare as their bits do, without the FP64 pipe.
+struct Near64 {
+    double ux, uy;
+    long long lo, hi;
+};
+__device__ __forceinline__ Near64 near64(float ux, float uy, float qx, float qy)
 {
-    double dx = (double)ux - (double)fx, dy = (double)uy - (double)fy;
-    double Df = fma(dx, dx, dy * dy);
-    double d = Df - Dq;
-    double bnd = 8.0 * kU64 * (Df + Dq);
-    if (d < -bnd) return true;
-    if (d > bnd) return false;
+    Near64 r;
+    r.ux = f2d_bits(ux);
+    r.uy = f2d_bits(uy);
+    const double dx = r.ux - f2d_bits(qx), dy = r.uy - f2d_bits(qy);
+    const double D = fma(dx, dx, dy * dy);
+    r.lo = __double_as_longlong(D * (1.0 - 16.0 * kU64));
+    r.hi = __double_as_longlong(D * (1.0 + 16.0 * kU64));
+    return r;
+}
+
+// f strictly nearer to u than q, FP64 filter then exact.  Four FP64
+// instructions a test (a warp's FP64 instruction takes its sub-partition's
+// pipe 64 cycles on GB300): two differences, a product and an FMA.
+__device__ __forceinline__ bool closer_f64(const Near64& n, float ux, float uy, float fx, float fy, float qx,
+                                           float qy, unsigned long long* rechecks)
+{
+    const double dx = n.ux - f2d_bits(fx), dy = n.uy - f2d_bits(fy);
+    const long long Df = __double_as_longlong(fma(dx, dx, dy * dy));
+    if (Df < n.lo) return true;
+    if (Df > n.hi) return false;
     ++*rechecks;
     return sign_d2diff_exact(ux, uy, fx, fy, qx, qy) < 0;
 }

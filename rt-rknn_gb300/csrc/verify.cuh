@@ -9,6 +9,7 @@ constexpr int VERIFY_CHUNK = 32 * VERIFY_UPT;       // default users per work it
 constexpr int VERIFY_WARPS = 8;                     // default warps per block
 constexpr int VERIFY_SAMPLES = 1024;                // work-item offsets cached per block
 constexpr int BOX_MIN_CAND = 512;                   // FP32: candidates from which boxes come first
+constexpr int VERIFY_PLANES_MAX = 1024;             // half-planes used per slot (32 box masks of 32)
 constexpr int FIN_WARPS = 8;                        // finalize: slots per block (one warp each)
 constexpr int FIN_WCAP = 512;                       // ids one warp sorts in registers
 
@@ -47,6 +48,7 @@ struct VerifyArgs {
     int2* surv;              // survivors of the half-plane filter: (slot, user position)
     int surv_cap;            // 0: no list (the verification kernel recounts in-warp)
     int* surv_count;
+    int* recount_counter = nullptr;    // recount_kernel's queue
     int* fault;              // checked builds: {flag, array id, index, size, line}
     // slots to verify: chunk_off indexes deflist[0 .. *ndef) when deflist is
     // set (the fused slice filter verified the others), else slots 0 .. nq
@@ -79,8 +81,9 @@ __host__ __device__ __forceinline__ size_t verify_warp_bytes(int stage_cap, int 
     return (b + 15) & ~(size_t)15;
 }
 
-// exact recount of the listed survivors, one thread each
-__global__ void recount_kernel(VerifyArgs a);
+// exact recount of the listed survivors, a warp or a group of warps each
+__global__ void recount_kernel(VerifyArgs a);       // FP32 filter
+__global__ void recount64_kernel(VerifyArgs a);     // FP64 filter
 
 // single block: result regions (min(candidates, rcap) ids at 64-bit offsets,
 // their lengths and *region_top = their total) and work-item offsets from

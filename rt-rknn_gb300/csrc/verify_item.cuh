@@ -34,21 +34,14 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
                                            unsigned long long& fac, unsigned long long& rech)
 {
     const int lane = threadIdx.x & 31;
-    float qx = d.qx, qy = d.qy;
-    T Dq;
-    float r;
+    const float qx = d.qx, qy = d.qy;
     const float slack = 4.0f * kU32 * (fabsf(ux) + fabsf(uy) + fabsf(qx) + fabsf(qy)) + 1e-30f;
-    if (sizeof(T) == 4) {
-        float dx = ux - qx, dy = uy - qy;
-        float D = fmaf(dx, dx, dy * dy);
-        Dq = (T)D;
-        r = sqrtf(D) * (1.0f + 4e-6f) + slack;
-    } else {
-        double dx = (double)ux - (double)qx, dy = (double)uy - (double)qy;
-        double D = fma(dx, dx, dy * dy);
-        Dq = (T)D;
-        r = (float)sqrt_rn64(D) * (1.0f + 4e-6f) + slack;
-    }
+    // the radius of the cells looked at, above |u - q|
+    const float ddx = ux - qx, ddy = uy - qy;
+    const float Dq = fmaf(ddx, ddx, ddy * ddy);
+    const float r = sqrtf(Dq) * (1.0f + 4e-6f) + slack;
+    Near64 near;
+    if (sizeof(T) == 8) near = near64(ux, uy, qx, qy);
     const Grid& g = A.gf;
     int cx0 = cell_coord(ux - r, g.x0, g.inv, g.gx), cx1 = cell_coord(ux + r, g.x0, g.inv, g.gx);
     int cy0 = cell_coord(uy - r, g.y0, g.inv, g.gy), cy1 = cell_coord(uy + r, g.y0, g.inv, g.gy);
@@ -60,8 +53,8 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
             bool c = false;
             if (i < f1 && i != d.qpos) {
                 float2 f = A.fxy[VX(i, A.nf, 203)];
-                if (sizeof(T) == 4) c = closer_f32(ux, uy, f.x, f.y, qx, qy, (float)Dq, &rech);
-                else c = closer_f64(ux, uy, f.x, f.y, qx, qy, (double)Dq, &rech);
+                if (sizeof(T) == 4) c = closer_f32(ux, uy, f.x, f.y, qx, qy, Dq, &rech);
+                else c = closer_f64(near, ux, uy, f.x, f.y, qx, qy, &rech);
             }
             cnt += __popc(__ballot_sync(FULL, c));
             fac += (unsigned long long)min(32, f1 - b);

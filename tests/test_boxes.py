@@ -37,7 +37,7 @@ def test_boxes_match_oracle(engine, sets, layout, upt, warps):
     with engine.Index.of(ds, users_per_thread=upt, verify_warps=warps) as idx:
         # about 66 users a facility: 5 to 8 and 33 to 100 lie on either side
         # of the rule
-        for k in (1, 5, 7, 8, 33, 100):
+        for k in (1, 5, 7, 8, 33, 100, 130):
             want = [o.query(int(q), k) for q in ds.queries]
             for mode in ("fp32", "fp64"):
                 for n in (len(ds.queries), 3):
