@@ -100,8 +100,9 @@ constexpr int FUSE_CAND = 4096;
 constexpr int ZB_VSTATS_INTS = 32;  // room for the statistics after them
 // counter ints: 1 verification work, 2 dropped, 3 listed survivors, 4-8 and
 // 10-14 bounds-check records, 16-31 slice filter work per k class, 36
-// slots the fused filter left over, 37 its blocks done, 38 recount work, 40-41 the 64-bit
-// result-region total
+// slots the fused filter left over, 37 its blocks done, 38 recount work, 39 sets
+// listed for sort_large_kernel, 40-41 the 64-bit result-region total, 42 that
+// kernel's queue
 
 struct Workspace {
     bool last_fuse = false;        // the last batch ran the fused verification
@@ -596,6 +597,7 @@ struct BatchPlan {
     bool fuse = false;          // the slice filter verifies its own slots (FP32, every class a slice class)
     size_t vsmem = 0;
     int vgrid = 0;
+    int sort_grid = 0;          // blocks of sort_large_kernel (0: not launched)
     GraphKey key;
 };
 
@@ -665,6 +667,9 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.vsmem = (size_t)b.vwarps * verify_warp_bytes(b.stage_cap, b.seg_stage);
     const int vper = occupancy(ix, (const void*)verify_fn(mode, b.vupt), b.vwarps * 32, b.vsmem);
     b.vgrid = vper * ix->num_sms;
+    if ((long long)kmax * ix->nu >= (long long)SORT_MIN_MEAN * ix->nf)
+        b.sort_grid = std::min(nq, occupancy(ix, (const void*)sort_large_kernel, SORT_THREADS, sort_large_smem()) * ix->num_sms);
+    b.key.push_back(b.sort_grid);
     b.key.push_back(b.vupt);
     b.key.push_back(b.vwarps);
     return b;
@@ -812,6 +817,10 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     // the output offsets: in finalize itself for batches of up to
     // FIN_SCAN_MAX slots, else by the scan kernel
     FinScan fs;
+    if (b.sort_grid > 0) {
+        fs.large = w.d_deflist;      // (the verification is done with it)
+        fs.nlarge = w.d_counters + 39;
+    }
     if (nq <= FIN_SCAN_MAX) {
         fs.on = 1;
         fs.out_off_host = c.io.off_host;
@@ -827,6 +836,11 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     CK(launch_k(finalize_kernel, (nq + FIN_WARPS - 1) / FIN_WARPS, 32 * FIN_WARPS, 0, st, pdl, w.d_pool,
                 (const long long*)w.d_cand_off, (const int*)w.d_reg_len, (const int*)w.d_res_count,
                 w.d_out_off, ids, w.d_out, nq, ids_cap, w.d_zb[w.zb_next], w.zb_ints, fs));
+    if (b.sort_grid > 0)
+        CK(launch_k(sort_large_kernel, b.sort_grid, SORT_THREADS, sort_large_smem(), st, pdl, w.d_pool,
+                    (const long long*)w.d_cand_off, (const int*)w.d_reg_len, (const int*)w.d_res_count,
+                    (const int*)w.d_out_off, ids, w.d_out, ids_cap, (const int*)w.d_deflist,
+                    (const int*)(w.d_counters + 39), w.d_counters + 42));
     mark(6);
     return RKNN_OK;
 }
@@ -1221,6 +1235,7 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
         ix->recount_grid = std::max(1, per) * ix->num_sms;
     }
     CKB(allow_dynamic_smem((const void*)slice_kernel, optin));
+    CKB(allow_dynamic_smem((const void*)sort_large_kernel, optin));
     for (const void* f : {(const void*)slice_kernel_r4, (const void*)slice_kernel_r8, (const void*)slice_kernel_r10, (const void*)slice_kernel_r12,
                           (const void*)slice_kernel_r16, (const void*)slice_kernel_r24, (const void*)slice_kernel_r32,
                           (const void*)slice_kernel2_r4, (const void*)slice_kernel2_r8, (const void*)slice_kernel2_r10, (const void*)slice_kernel2_r12,

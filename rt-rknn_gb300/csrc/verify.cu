@@ -616,7 +616,8 @@ __device__ __forceinline__ void warp_sort_slot(const unsigned* src, unsigned* ds
 
 // One warp per slot sorts the slot's stored ids into its output range: up to
 // 32 ids by rank counting in registers, up to FIN_WCAP by a bitonic network
-// in registers, larger sets by a radix sort through the slot's pool region.
+// in registers; larger sets are listed for sort_large_kernel where the batch
+// launches it, else radix sorted through the slot's pool region.
 __global__ void __launch_bounds__(32 * FIN_WARPS, 1)
 finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
                 int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero, long long zero_n, FinScan S)
@@ -701,10 +702,205 @@ finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, co
             warp_sort_slot<8>(src, dst, n, lane);
         } else if (n <= FIN_WCAP) {
             warp_sort_slot<16>(src, dst, n, lane);
+        } else if (S.large) {
+            // left to sort_large_kernel
+            if (lane == 0) S.large[atomicAdd(S.nlarge, 1)] = s;
         } else {
             warp_radix_slot(src, (unsigned*)(stage + os), dst, n, lane, bins[w]);
         }
     }
 }
+
+// ------------------------------------------------------- large result sets
+// Sorts one slot's n > 0 ids with a block: LSD radix, SORT_BITS bits a pass
+// over the bits in which the ids differ, in tiles of SORT_TILE ids.  In a pass
+// each thread takes SORT_PT ids at most (a warp's are consecutive runs of 32),
+// ranks them within its warp's digit counts by ballots, and the block's scan of
+// those counts places every id; a set of one tile ping-pongs between two
+// shared-memory buffers, a larger one between src and tmp in device memory,
+// its tiles in order after a histogram of the whole set.  The sorted ids go
+// to out on its 128-byte lines.
+//
+// Why a block: a warp that sorts a set alone is a chain of dependent loads,
+// votes and shared-memory updates (67 rounds a pass at the street workload's
+// mean of 2,140 ids, 400 at its largest), and the last large set that starts
+// ends the batch.  Street workload, 16,384 sets, 35 M ids: finalize 1.42 ms
+// with a warp a set, 0.81 so (0.06 of it because the 140 MB go to page-locked
+// host memory).  Ranking bound: same-digit lanes from a match instruction
+// instead of a ballot a bit took 0.96 ms.
+namespace {
+constexpr int SORT_WARPS = SORT_THREADS / 32;
+constexpr int SORT_PT = SORT_TILE / SORT_THREADS;
+constexpr int SORT_DIGITS = 1 << SORT_BITS;
+static_assert(SORT_THREADS >= SORT_DIGITS && SORT_DIGITS % 32 == 0, "a thread a digit in the scans");
+static_assert(SORT_TILE % SORT_THREADS == 0 && SORT_TILE <= 65536, "whole rounds of ids, 16-bit counts");
+
+struct SortShared {
+    unsigned key[2][SORT_TILE];
+    uint16_t cnt[SORT_WARPS][SORT_DIGITS];      // a warp's digit counts, then its first places
+    unsigned base[SORT_DIGITS];                 // tiled sets: where a digit's next id goes
+    unsigned place[SORT_DIGITS];                // where the tile's first id of a digit goes
+    unsigned ws[SORT_WARPS], mn, mx;
+    int slot;
+};
+
+// Exclusive scan of v over the block's first SORT_DIGITS threads (the others
+// pass 0); begins and ends at a barrier.
+__device__ __forceinline__ unsigned sort_scan(unsigned v, SortShared& sh)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sh.ws[w] = x;
+    __syncthreads();
+    unsigned b = 0;
+#pragma unroll
+    for (int j = 0; j < SORT_DIGITS / 32; ++j)
+        if (j < w) b += sh.ws[j];
+    __syncthreads();
+    return b + x - v;
+}
+
+__device__ __forceinline__ void sort_slot(SortShared& sh, const unsigned* src0, unsigned* tmp, unsigned* out, int n)
+{
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    unsigned* src = (unsigned*)src0;
+    const bool one = n <= SORT_TILE;
+    // keys with the ids' order, their range, and (one tile) their copy
+    unsigned mn = 0xffffffffu, mx = 0u;
+    if (tid == 0) { sh.mn = 0xffffffffu; sh.mx = 0u; }
+    for (int i = tid; i < n; i += SORT_THREADS) {
+        const unsigned k = okey((int)src[i]);
+        if (one) sh.key[0][i] = k;
+        else src[i] = k;
+        mn = min(mn, k);
+        mx = max(mx, k);
+    }
+    mn = __reduce_min_sync(FULL, mn);
+    mx = __reduce_max_sync(FULL, mx);
+    __syncthreads();
+    if (lane == 0) { atomicMin(&sh.mn, mn); atomicMax(&sh.mx, mx); }
+    __syncthreads();
+    mn = sh.mn;
+    const unsigned span = sh.mx - mn;
+    const int passes = span ? (32 - __clz((int)span) + SORT_BITS - 1) / SORT_BITS : 0;
+    int cur = 0;                        // one tile: the buffer that holds the keys
+    unsigned *a = src, *b = tmp;        // more: the arrays, a holding the keys
+    for (int p = 0; p < passes; ++p) {
+        const int shift = SORT_BITS * p;
+        if (!one) {
+            // the whole set's digit counts place its tiles
+            for (int i = tid; i < SORT_DIGITS; i += SORT_THREADS) sh.base[i] = 0u;
+            __syncthreads();
+            for (int i = tid; i < n; i += SORT_THREADS)
+                atomicAdd(&sh.base[((a[i] - mn) >> shift) & (SORT_DIGITS - 1)], 1u);
+            __syncthreads();
+            const unsigned e = sort_scan(tid < SORT_DIGITS ? sh.base[tid] : 0u, sh);
+            if (tid < SORT_DIGITS) sh.base[tid] = e;
+            __syncthreads();
+        }
+        for (int t0 = 0; t0 < n; t0 += SORT_TILE) {
+            const int m = min(SORT_TILE, n - t0);
+            for (int i = lane; i < SORT_DIGITS / 2; i += 32) ((unsigned*)sh.cnt[w])[i] = 0u;
+            __syncwarp();
+            unsigned key[SORT_PT];
+            uint16_t rank[SORT_PT];
+            const int pt = (m + SORT_THREADS - 1) / SORT_THREADS;      // ids a thread takes
+            const int i0 = w * (32 * pt) + lane;
+#pragma unroll
+            for (int j = 0; j < SORT_PT; ++j) {
+                if (j >= pt) break;
+                const int i = i0 + 32 * j;
+                const bool ok = i < m;
+                key[j] = ok ? (one ? sh.key[cur][i] : a[t0 + i]) : 0u;
+                const unsigned d = ((key[j] - mn) >> shift) & (SORT_DIGITS - 1);
+                // lanes with the same digit, a ballot a bit
+                unsigned mm = __ballot_sync(FULL, ok);
+#pragma unroll
+                for (int t = 0; t < SORT_BITS; ++t) {
+                    const bool bit = (d >> t) & 1u;
+                    const unsigned v = __ballot_sync(FULL, bit);
+                    mm &= bit ? v : ~v;
+                }
+                const int r = __popc(mm & ((1u << lane) - 1));
+                const int old = ok ? sh.cnt[w][d] : 0;
+                __syncwarp();
+                if (ok && r == 0) sh.cnt[w][d] = (uint16_t)(old + __popc(mm));
+                __syncwarp();
+                rank[j] = (uint16_t)(old + r);
+            }
+            __syncthreads();
+            // a digit's ids: warp by warp, after those of smaller digits
+            unsigned tot = 0;
+            if (tid < SORT_DIGITS) {
+#pragma unroll
+                for (int j = 0; j < SORT_WARPS; ++j) {
+                    const unsigned c = sh.cnt[j][tid];
+                    sh.cnt[j][tid] = (uint16_t)tot;
+                    tot += c;
+                }
+            }
+            unsigned first = 0;
+            if (one) {
+                first = sort_scan(tot, sh);
+            } else if (tid < SORT_DIGITS) {
+                first = sh.base[tid];
+                sh.base[tid] = first + tot;
+            }
+            if (tid < SORT_DIGITS) sh.place[tid] = first;
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < SORT_PT; ++j) {
+                const int i = i0 + 32 * j;
+                if (j < pt && i < m) {
+                    const unsigned d = ((key[j] - mn) >> shift) & (SORT_DIGITS - 1);
+                    const unsigned at = sh.place[d] + sh.cnt[w][d] + rank[j];
+                    if (one) sh.key[cur ^ 1][at] = key[j];
+                    else b[at] = key[j];
+                }
+            }
+            __syncthreads();
+        }
+        cur ^= 1;
+        unsigned* t = a;
+        a = b;
+        b = t;
+    }
+    const int lead = (int)(((unsigned long long)out >> 2) & 31ull);
+    for (int i = tid - lead; i < n; i += SORT_THREADS)
+        if (i >= 0) out[i] = (one ? sh.key[cur][i] : a[i]) ^ 0x80000000u;
+    __syncthreads();
+}
+}  // namespace
+
+// Blocks take the slots of more than FIN_WCAP ids that finalize_kernel listed.
+__global__ void __launch_bounds__(SORT_THREADS)
+sort_large_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
+                  const int* out_off, int* out, int* stage, long long out_cap, const int* list, const int* nlist,
+                  int* queue)
+{
+    extern __shared__ __align__(16) char smem[];
+    SortShared& sh = *(SortShared*)smem;
+    pdl_wait();
+    pdl_trigger();
+    const int nl = *nlist;
+    for (int e = blockIdx.x; e < nl;) {
+        const int s = list[e];
+        const int n = min(res_count[s], reg_len[s]), os = out_off[s];
+        if ((long long)os + n <= out_cap)
+            sort_slot(sh, (const unsigned*)(res_pool + cand_off[s]), (unsigned*)(stage + os), (unsigned*)(out + os), n);
+        if (nl <= (int)gridDim.x) break;
+        if (threadIdx.x == 0) sh.slot = (int)gridDim.x + atomicAdd(queue, 1);
+        __syncthreads();
+        e = sh.slot;
+        __syncthreads();
+    }
+}
+
+size_t sort_large_smem() { return sizeof(SortShared); }
 
 }  // namespace rknn

@@ -112,7 +112,24 @@ struct FinScan {
     int* out_off_host = nullptr;
     const long long* region_top = nullptr;
     const int* counters = nullptr;
+    // sets above FIN_WCAP ids are listed here for sort_large_kernel (null:
+    // sorted by their warps)
+    int* large = nullptr;
+    int* nlarge = nullptr;
 };
+
+// Sets above FIN_WCAP ids, a block each (persistent blocks, *queue counts the
+// slots taken after each block's first).  Launched for batches whose largest k
+// gives SORT_MIN_MEAN results on average: below it large sets are few, and the
+// launch would cost more than their warps' sorts.
+// (finalize of the street workload, ms, threads / tile: 256 / 4096 0.84,
+// 256 / 8192 0.94, 512 / 4096 0.87, 512 / 8192 0.81, 1024 / 12288 1.03)
+constexpr int SORT_BITS = 8, SORT_THREADS = 512, SORT_TILE = 8192;
+constexpr int SORT_MIN_MEAN = 1024;
+__global__ void sort_large_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
+                                  const int* out_off, int* out, int* stage, long long out_cap, const int* list,
+                                  const int* nlist, int* queue);
+size_t sort_large_smem();
 
 // one block per slot: sort the slot's results into out[out_off[s] ...]
 // out may be device-accessible host memory of out_cap ids: a slot whose range

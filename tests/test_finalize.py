@@ -2,32 +2,35 @@
 
 With one facility every user is in its result set, so a set has exactly as
 many ids as there are users, whatever k: the sizes here sit at the edges of
-the sort's classes (32, 64, 128, 256 and 512 ids, and the radix sort beyond).
+the sort's classes (32, 64, 128, 256 and 512 ids, and the block's radix sort
+beyond, by tiles of 8192).  Beside a few hundred facilities far from every
+user the same sets are few in their batch, and warps sort the large ones.
 """
 import numpy as np
 import pytest
 
 import rknn
 
-SIZES = [1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 2048, 70_001]
+SIZES = [1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 2048, 8192, 8193, 16_385, 70_001]
 
 
-def _index(n, ids):
+def _index(n, ids, far):
     rng = np.random.default_rng(n)
-    return rknn.Index(np.array([[500.0, 500.0]], np.float32), rng.uniform(0, 1000, (n, 2)).astype(np.float32),
-                      uid=ids)
+    fxy = np.concatenate([[[500.0, 500.0]], rng.uniform(90_000, 100_000, (far, 2))]).astype(np.float32)
+    return rknn.Index(fxy, rng.uniform(0, 1000, (n, 2)).astype(np.float32), uid=ids)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("far", [0, 300])
 @pytest.mark.parametrize("n", SIZES)
-def test_sorted_ids_in_every_output(n):
+def test_sorted_ids_in_every_output(n, far):
     rng = np.random.default_rng(1000 + n)
     # ids spread over the whole int32 range, in random order
     ids = rng.choice(2**32, size=n, replace=False).astype(np.int64) - 2**31
     ids = ids.astype(np.int32)
     want = np.tile(np.sort(ids), 3)
     qs = np.zeros(3, np.int32)
-    with _index(n, ids) as idx:
+    with _index(n, ids, far) as idx:
         for mode in ("fp32", "fp64"):
             # page-locked output: staged on the first call, written by the
             # kernels on the later ones
