@@ -97,6 +97,9 @@ constexpr int ZB_COUNTERS = 64;     // counter ints at the head of the zeroed bl
 // most candidates the fused slice filter verifies itself (more go to the
 // verification kernel, which spreads a slot over the whole GPU)
 constexpr int FUSE_CAND = 4096;
+// segments kept in shared memory for a slot's verification (slots with more
+// read them from L1)
+constexpr int SEG_STAGE_MAX = 130;
 constexpr int ZB_VSTATS_INTS = 32;  // room for the statistics after them
 // counter ints: 1 verification work, 2 dropped, 3 listed survivors, 4-8 and
 // 10-14 bounds-check records, 16-31 slice filter work per k class, 36
@@ -571,7 +574,7 @@ ZoneCaps slice_caps(int kmax)
     const long long most = std::min<long long>(std::max<long long>(8LL * c.vc, 512), VERIFY_PLANES_MAX);
     c.lc = (int)std::max<long long>(1, std::min<long long>(24LL * c.vc + 60, most));
     c.pc = 0;
-    c.rm = 64;
+    c.rm = 128;
     return c;
 }
 
@@ -648,7 +651,7 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
     int rm = 0;
     for (auto& c : b.cls) rm = std::max(rm, c.caps.rm);
-    b.seg_stage = std::min(2 * rm + 2, 512);
+    b.seg_stage = std::min(2 * rm + 2, SEG_STAGE_MAX);
     // Fused verification for FP32 batches whose every class runs the slice
     // filter two warps a query (batches that fit resident): there it takes
     // the verification kernel's latency off each query's path.  Larger

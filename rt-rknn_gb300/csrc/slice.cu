@@ -128,6 +128,16 @@ __device__ __forceinline__ float box_bound(float X0, float X1, float Y0, float Y
     return r;
 }
 
+// Whether every facility in a box (relative to q, not around it) lies beyond
+// twice the reach of its slice (Rs: the slices' reach, slice_reach).
+__device__ __forceinline__ bool plane_only(float X0, float X1, float Y0, float Y1, const float* Rs)
+{
+    const float dx = fmaxf(fmaxf(X0, -X1), 0.0f), dy = fmaxf(fmaxf(Y0, -Y1), 0.0f);
+    const float L2 = fmaf(dx, dx, dy * dy) * (1.0f - 4e-6f);     // |box - q|^2, rounded down
+    const float R = box_bound(X0, X1, Y0, Y1, Rs);
+    return R < INFINITY && 0.25f * L2 > R * R * (1.0f + 4e-6f);
+}
+
 // Cell ri of the square ring at Chebyshev distance ring around (qcx, qcy):
 // bottom row, top row, then the left and right columns without corners.
 __device__ __forceinline__ void ring_cell(int ring, int ri, int qcx, int qcy, int& cxx, int& cyy)
@@ -288,7 +298,8 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
     float* H = (float*)(wsm + LY.heap);
     float* Rs = (float*)(wsm + LY.R);
     int* lpos = (int*)(wsm + LY.lpos);
-    uint32_t* bitmap = (uint32_t*)(wsm + LY.bitmap);
+    int* rowlo = (int*)(wsm + LY.rows);
+    int* rowhi = rowlo + 2 * A.rmax + 1;
     // NWQ = 2: both warps' lists ([warp][entry][lane]) and a few ints passed
     // between the warps
     float* xl = (float*)(smem + (size_t)NWQ * LY.bytes);
@@ -516,10 +527,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                             // the cell's box widened for the cell function's rounding
                             const float X0 = A.gf.x0 + (float)cxx * A.gf.cs - cmargin, X1 = A.gf.x0 + (float)(cxx + 1) * A.gf.cs + cmargin;
                             const float Y0 = A.gf.y0 + (float)cyy * A.gf.cs - cmargin, Y1 = A.gf.y0 + (float)(cyy + 1) * A.gf.cs + cmargin;
-                            const float ddx = fmaxf(fmaxf(X0 - qf.x, qf.x - X1), 0.0f), ddy = fmaxf(fmaxf(Y0 - qf.y, qf.y - Y1), 0.0f);
-                            const float Lc2 = fmaf(ddx, ddx, ddy * ddy) * (1.0f - 4e-6f);     // |box - q|^2, rounded down
-                            const float Rc = box_bound(X0 - qf.x, X1 - qf.x, Y0 - qf.y, Y1 - qf.y, Rs);
-                            if (Rc < INFINITY && 0.25f * Lc2 > Rc * Rc * (1.0f + 4e-6f)) po = true;
+                            po = plane_only(X0 - qf.x, X1 - qf.x, Y0 - qf.y, Y1 - qf.y, Rs);
                         }
                         // once the half-planes are full (a facility of rho_ring
                         // was left out), a plane-only cell has nothing to give:
@@ -747,65 +755,71 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         int nseg = 0, ncand = 0;
         int qflags = QF_SLICE_R;
         if (NWQ == 1 || wq == 1) {
-        // ---- ring scan over user cells --------------------------------------
+        // ---- user rows ------------------------------------------------------
+        // The kept region is the union of the slices' sectors (radius R(P)).
+        // Each lane walks the user-grid rows its sector meets and widens the
+        // rows' column ranges to the sector's in that row's band: in the
+        // quadrant's reflection, a point of the sector with y in [lo, hi] has
+        //     lo cot(b) <= x <= min(hi cot(a), R cos(a), sqrt(R^2 - lo^2)),
+        // a and b its lower and upper edge angle.  (slice_of decides quadrants
+        // by the signs, exactly; within one the widened edges hold every user
+        // it may name the slice for.)  A ring scan over the cells, with the
+        // bounds of the slices a cell spans, took 7.0 k cycles a query on the
+        // uniform workload at k=10 and 31 k on the street workload, against
+        // 2.9 k and 7.0 k, kept 5 % more candidates on the former, and gave up
+        // (every user a candidate) beyond 64 cells: 11,171 candidates a query
+        // on the clustered workload, now 1,095.
         const Grid gu = A.gu;
-        const int ucx = cell_coord(qf.x, gu.x0, gu.inv, gu.gx);
         const int ucy = cell_coord(qf.y, gu.y0, gu.inv, gu.gy);
         const int RM = A.rmax;
-        const int W = 2 * RM + 1;
-        const int nwords = (W * W + 31) / 32;
-        for (int i = lane; i < nwords; i += 32) bitmap[SX(i, nwords, 320)] = 0u;
+        const int NR = 2 * RM + 1;          // rows ucy - RM .. ucy + RM
+        for (int i = lane; i < NR; i += 32) {
+            rowlo[SX(i, NR, 320)] = INT_MAX;
+            rowhi[SX(i, NR, 320)] = -1;
+        }
         __syncwarp();
         const float delta = 8.0f * kU32 * (fabsf(gu.x0) + fabsf(gu.y0) + gu.cs * (float)max(gu.gx, gu.gy) + fabsf(qf.x) + fabsf(qf.y) + gu.cs) + 1e-30f;
-        const int rmaxu = max(max(ucx, gu.gx - 1 - ucx), max(ucy, gu.gy - 1 - ucy));
-        bool all_users = false;
-        int rend = -1;
+        int ylo = ucy, yhi = ucy;           // the rows the region meets
+        bool row_span = false;              // too many of them: one range of whole rows
         if (A.nu > 0) {
-            for (int r = 0;; ++r) {
-                if (r > rmaxu) { rend = r - 1; break; }
-                if (r > RM) { all_users = true; break; }
-                const int ncell = r == 0 ? 1 : 8 * r;
-                bool anykeep = false;
-                for (int t0 = 0; t0 < ncell; t0 += 32) {
-                    const int t = t0 + lane;
-                    int dx = 0, dy = 0;
-                    bool ok = t < ncell;
-                    if (ok && r > 0) {
-                        const int side = 2 * r + 1;
-                        if (t < side) { dx = -r + t; dy = -r; }
-                        else if (t < 2 * side) { dx = -r + (t - side); dy = r; }
-                        else if (t < 2 * side + (2 * r - 1)) { dx = -r; dy = -r + 1 + (t - 2 * side); }
-                        else { dx = r; dy = -r + 1 + (t - 2 * side - (2 * r - 1)); }
+            // the user test keeps |u - q| up to R (1 + 1e-6)
+            const float R = Rs[lane] * (1.0f + 4e-6f) + 1e-30f;
+            const bool xpos = lane < 8 || lane >= 24, ypos = lane < 16;
+            const bool even = ((lane >> 3) & 1) == 0;       // the lower edge of the reflection is e1
+            const float sxf = xpos ? 1.0f : -1.0f, syf = ypos ? 1.0f : -1.0f;
+            const float cA = sxf * (even ? e1x : e2x), sA = syf * (even ? e1y : e2y);
+            const float cB = sxf * (even ? e2x : e1x), sB = syf * (even ? e2y : e1y);
+            // an edge past an axis is the axis
+            const float cotA = sA > 0.0f ? __fdividef(cA, sA) * (1.0f + 1e-6f) : INFINITY;
+            const float cosA = sA > 0.0f ? cA * (1.0f + 1e-6f) : 1.0f;
+            const float cotB = cB > 0.0f ? __fdividef(cB, sB) * (1.0f - 1e-6f) : 0.0f;
+            const float Ymax = cB > 0.0f ? R * fminf(sB * (1.0f + 1e-6f), 1.0f) : R;
+            const float Xmax = R * cosA;
+            const int ra = ypos ? cell_coord(qf.y - delta, gu.y0, gu.inv, gu.gy)
+                                : cell_coord(qf.y - Ymax - delta, gu.y0, gu.inv, gu.gy);
+            const int rb = ypos ? cell_coord(qf.y + Ymax + delta, gu.y0, gu.inv, gu.gy)
+                                : cell_coord(qf.y + delta, gu.y0, gu.inv, gu.gy);
+            ylo = __reduce_min_sync(FULL, ra);
+            yhi = __reduce_max_sync(FULL, rb);
+            row_span = ylo < ucy - RM || yhi > ucy + RM;
+            if (!row_span) {
+                for (int r = ra; r <= rb; ++r) {
+                    const float Y0 = (gu.y0 + (float)r * gu.cs) - qf.y - delta;
+                    const float Y1 = (gu.y0 + (float)(r + 1) * gu.cs) - qf.y + delta;
+                    const float lo = fmaxf(ypos ? Y0 : -Y1, 0.0f), hi = fminf(ypos ? Y1 : -Y0, Ymax);
+                    if (lo > hi) continue;
+                    const float xa = lo * cotB;
+                    const float xc = sqrtf((R - lo) * (R + lo)) * (1.0f + 1e-6f);   // (lo <= hi <= R)
+                    const float xb = fminf(fminf(hi * cotA, Xmax), xc);     // (0 times infinity: xb from the others)
+                    const int c0 = cell_coord(xpos ? qf.x + xa - delta : qf.x - xb - delta, gu.x0, gu.inv, gu.gx);
+                    const int c1 = cell_coord(xpos ? qf.x + xb + delta : qf.x - xa + delta, gu.x0, gu.inv, gu.gx);
+                    if (c0 <= c1) {
+                        atomicMin(&rowlo[SX(r - (ucy - RM), NR, 321)], c0);
+                        atomicMax(&rowhi[SX(r - (ucy - RM), NR, 321)], c1);
                     }
-                    const int cxx = ucx + dx, cyy = ucy + dy;
-                    ok = ok && cxx >= 0 && cxx < gu.gx && cyy >= 0 && cyy < gu.gy;
-                    bool keep = false;
-                    if (ok) {
-                        const float X0 = (gu.x0 + (float)cxx * gu.cs) - qf.x - delta;
-                        const float X1 = (gu.x0 + (float)(cxx + 1) * gu.cs) - qf.x + delta;
-                        const float Y0 = (gu.y0 + (float)cyy * gu.cs) - qf.y - delta;
-                        const float Y1 = (gu.y0 + (float)(cyy + 1) * gu.cs) - qf.y + delta;
-                        if (X0 <= 0.0f && X1 >= 0.0f && Y0 <= 0.0f && Y1 >= 0.0f) keep = true;
-                        else {
-                            // nearest point of the cell against the largest
-                            // bound of the slices the cell spans
-                            const float ddx = fmaxf(fmaxf(X0, -X1), 0.0f), ddy = fmaxf(fmaxf(Y0, -Y1), 0.0f);
-                            const float dmin2 = fmaf(ddx, ddx, ddy * ddy) * (1.0f - 4.0f * kU32);
-                            const float Rmax = box_bound(X0, X1, Y0, Y1, Rs);
-                            keep = !(dmin2 > Rmax * Rmax);
-                        }
-                    }
-                    if (keep) {
-                        const int bit = (dy + RM) * W + (dx + RM);
-                        atomicOr(&bitmap[SX(bit >> 5, nwords, 321)], 1u << (bit & 31));
-                    }
-                    anykeep |= keep;
                 }
-                anykeep = __any_sync(FULL, anykeep);
-                if (!anykeep && r >= 1) { rend = r - 1; break; }
-                rend = r;
             }
-            zs.rings = rend + 1;
+            zs.rings = max(ucy - ylo, yhi - ucy) + 1;
         }
         __syncwarp();
         zs.cyc[2] += clock64() - tph;
@@ -818,29 +832,20 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             seg[i] = v;
             if (FUSED && i < A.fuse_ss) fzs[i] = v;
         };
-        if (all_users) {
-            put_seg(0, make_int2(0, 0));
-            put_seg(1, make_int2(0, A.nu));
+        if (A.nu > 0 && row_span) {
+            const int st = A.ustart[SX((long long)ylo * gu.gx, NCU + 1, 322)];
+            ncand = A.ustart[SX((long long)(yhi + 1) * gu.gx, NCU + 1, 322)] - st;
+            put_seg(0, make_int2(st, 0));
+            put_seg(1, make_int2(0, ncand));
             nseg = 1;
-            ncand = A.nu;
-            qflags |= QF_ALL_USERS;
-        } else if (rend >= 0) {
-            const int y0 = max(0, ucy - rend), y1 = min(gu.gy - 1, ucy + rend);
-            const int xl0 = max(0, ucx - rend), xl1 = min(gu.gx - 1, ucx + rend);
-            for (int r0 = y0; r0 <= y1; r0 += 32) {
+            if (ncand == A.nu) qflags |= QF_ALL_USERS;
+        } else if (A.nu > 0) {
+            for (int r0 = ylo; r0 <= yhi; r0 += 32) {
                 const int row = r0 + lane;
                 int st = 0, len = 0;
-                if (row <= y1) {
-                    const int dy = row - ucy;
-                    int xmin = INT_MAX, xmax = -1;
-                    for (int cxx = xl0; cxx <= xl1; ++cxx) {
-                        const int bit = (dy + RM) * W + (cxx - ucx + RM);
-                        if (bitmap[SX(bit >> 5, nwords, 322)] & (1u << (bit & 31))) {
-                            xmin = min(xmin, cxx);
-                            xmax = cxx;
-                        }
-                    }
-                    if (xmax >= 0) {
+                if (row <= yhi) {
+                    const int xmin = rowlo[SX(row - (ucy - RM), NR, 322)], xmax = rowhi[SX(row - (ucy - RM), NR, 322)];
+                    if (xmax >= xmin) {
                         st = A.ustart[SX((long long)row * gu.gx + xmin, NCU + 1, 323)];
                         len = A.ustart[SX((long long)row * gu.gx + xmax + 1, NCU + 1, 324)] - st;
                     }
@@ -870,7 +875,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         } else if (lane == 0) {
             put_seg(0, make_int2(0, 0));
         }
-        }   // ring scan and segments
+        }   // user rows and segments
         zs.cyc[7] += clock64() - tph;
         zs.nb = nL;
         if constexpr (NWQ == 2) {
@@ -929,14 +934,17 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
 
 #undef SLICE_KTH
 
+// The one-warp variants' registers are capped where more queries in flight pay
+// for shorter chains (filter of 16,384 uniform queries at k=10: 133 registers
+// 254 us, 121 (16 blocks an SM) 212, 104 (18) 196, 20 blocks 196, 24 201).
 __global__ void __launch_bounds__(32, 1) slice_kernel(ZoneArgs A) { slice_body<0, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r4(ZoneArgs A) { slice_body<4, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r8(ZoneArgs A) { slice_body<8, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r10(ZoneArgs A) { slice_body<10, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r12(ZoneArgs A) { slice_body<12, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r16(ZoneArgs A) { slice_body<16, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r24(ZoneArgs A) { slice_body<24, 1>(A); }
-__global__ void __launch_bounds__(32, 1) slice_kernel_r32(ZoneArgs A) { slice_body<32, 1>(A); }
+__global__ void __launch_bounds__(32, 18) slice_kernel_r4(ZoneArgs A) { slice_body<4, 1>(A); }
+__global__ void __launch_bounds__(32, 18) slice_kernel_r8(ZoneArgs A) { slice_body<8, 1>(A); }
+__global__ void __launch_bounds__(32, 18) slice_kernel_r10(ZoneArgs A) { slice_body<10, 1>(A); }
+__global__ void __launch_bounds__(32, 18) slice_kernel_r12(ZoneArgs A) { slice_body<12, 1>(A); }
+__global__ void __launch_bounds__(32, 14) slice_kernel_r16(ZoneArgs A) { slice_body<16, 1>(A); }
+__global__ void __launch_bounds__(32, 14) slice_kernel_r24(ZoneArgs A) { slice_body<24, 1>(A); }
+__global__ void __launch_bounds__(32, 14) slice_kernel_r32(ZoneArgs A) { slice_body<32, 1>(A); }
 __global__ void __launch_bounds__(64, 7) slice_kernel2_r4(ZoneArgs A) { slice_body<4, 2>(A); }
 __global__ void __launch_bounds__(64, 7) slice_kernel2_r8(ZoneArgs A) { slice_body<8, 2>(A); }
 __global__ void __launch_bounds__(64, 7) slice_kernel2_r10(ZoneArgs A) { slice_body<10, 2>(A); }

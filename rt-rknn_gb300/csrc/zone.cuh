@@ -78,20 +78,20 @@ __host__ __device__ inline ZoneLayout zone_layout(const ZoneCaps& c)
 
 // Angular-slice filter (slice_kernel): 32 slices around q, one per lane.
 // caps.vc = heap entries per slice (the batch class's largest k), caps.lc =
-// half-planes kept for the verification, caps.rm = user ring scan radius.
+// half-planes kept for the verification, caps.rm = user rows on either side of
+// q's (rows: their column ranges).
 struct SliceLayout {
-    size_t heap, R, lpos, bitmap, bytes;
+    size_t heap, R, lpos, rows, bytes;
 };
 
 __host__ __device__ inline SliceLayout slice_layout(const ZoneCaps& c)
 {
     SliceLayout L;
     size_t o = 0;
-    const size_t W = 2 * (size_t)c.rm + 1;
     L.heap = o;   o = zl_align(o + 4 * 32 * ((size_t)c.vc + ZL_SPARE));
     L.R = o;      o = zl_align(o + 4 * 32);
     L.lpos = o;   o = zl_align(o + 4 * ((size_t)c.lc + ZL_SPARE));
-    L.bitmap = o; o = zl_align(o + 4 * ((W * W + 31) / 32 + ZL_SPARE));
+    L.rows = o;   o = zl_align(o + 4 * 2 * (2 * (size_t)c.rm + 1));
     L.bytes = o;
     return L;
 }

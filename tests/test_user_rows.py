@@ -1,0 +1,46 @@
+"""The slice filter's kept region as user-grid rows: regions of more rows than
+it lists one by one, regions cut by the data's box, points on a line, users far
+from every facility.  Every answer equals the exact oracle's."""
+import numpy as np
+import pytest
+
+import datagen
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(layout):
+    rng = np.random.default_rng(91)
+    if layout == "wide":                    # about 190 user rows, regions from a few to all of them
+        f, u = rng.uniform(0, 1000, (60, 2)), rng.uniform(0, 1000, (300_007, 2))
+    elif layout == "vertical":              # one column of cells
+        f = np.stack([np.full(200, 3.0), rng.uniform(-50, 50, 200)], 1)
+        u = np.stack([np.full(20_011, 3.0), rng.uniform(-50, 50, 20_011)], 1)
+    elif layout == "horizontal":
+        f = np.stack([rng.uniform(-50, 50, 200), np.full(200, -7.0)], 1)
+        u = np.stack([rng.uniform(-50, 50, 20_011), np.full(20_011, -7.0)], 1)
+    else:                                   # users in a corner, facilities in the opposite one
+        f = rng.uniform(0, 10, (150, 2))
+        u = np.concatenate([rng.uniform(900, 1000, (30_000, 2)), rng.uniform(0, 10, (500, 2))])
+    f, u = f.astype(np.float32), u.astype(np.float32)
+    return datagen.Dataset(f, u, np.arange(len(f), dtype=np.int32), np.arange(len(f), len(f) + len(u), dtype=np.int32))
+
+
+@pytest.mark.parametrize("layout", ["wide", "vertical", "horizontal", "corner"])
+def test_regions_match_oracle(engine, layout):
+    ds = _points(layout)
+    o = O.Oracle.of(ds)
+    # the facilities nearest to the box's sides and corners, and a few others
+    near = [np.argmin(ds.fxy @ np.array(d, np.float32)) for d in [(1, 0), (-1, 0), (0, 1), (0, -1), (1, 1), (-1, -1)]]
+    qs = np.unique(np.concatenate([near, np.arange(0, ds.nf, 9)])).astype(np.int32)
+    big = np.tile(qs, 1 + 1300 // qs.size)          # one warp a query instead of two
+    with engine.Index.of(ds, filter="slice") as idx:
+        for k in (1, 7, 20, 45):
+            want = [o.query(int(q), k) for q in qs]
+            for mode in ("fp32", "fp64"):
+                for got, w in zip(idx.query_batch(qs, k, mode), want):
+                    assert np.array_equal(got, w), (layout, k, mode)
+            if layout != "corner":
+                for got, w in zip(idx.query_batch(big, k, "fp32"), want * (big.size // qs.size)):
+                    assert np.array_equal(got, w), (layout, k)
