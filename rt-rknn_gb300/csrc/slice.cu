@@ -129,13 +129,20 @@ __device__ __forceinline__ float box_bound(float X0, float X1, float Y0, float Y
 }
 
 // Whether every facility in a box (relative to q, not around it) lies beyond
-// twice the reach of its slice (Rs: the slices' reach, slice_reach).
-__device__ __forceinline__ bool plane_only(float X0, float X1, float Y0, float Y1, const float* Rs)
+// twice the need of its slice (Ns: the slices' need).
+__device__ __forceinline__ bool box_idle(float X0, float X1, float Y0, float Y1, const float* Ns)
 {
     const float dx = fmaxf(fmaxf(X0, -X1), 0.0f), dy = fmaxf(fmaxf(Y0, -Y1), 0.0f);
     const float L2 = fmaf(dx, dx, dy * dy) * (1.0f - 4e-6f);     // |box - q|^2, rounded down
-    const float R = box_bound(X0, X1, Y0, Y1, Rs);
+    const float R = box_bound(X0, X1, Y0, Y1, Ns);
     return R < INFINITY && 0.25f * L2 > R * R * (1.0f + 4e-6f);
+}
+
+// Whether a facility at offset (vx, vy), |v|^2 = d2, lies beyond twice a reach
+// or need.
+__device__ __forceinline__ bool beyond(float d2, float r)
+{
+    return 0.25f * d2 * (1.0f - 4.0f * kU32) >= r * r;
 }
 
 // Cell ri of the square ring at Chebyshev distance ring around (qcx, qcy):
@@ -153,25 +160,40 @@ __device__ __forceinline__ void ring_cell(int ring, int ri, int qcx, int qcy, in
     }
 }
 
-// Reach of a slice: a facility whose direction lies in slice s can lower no
-// slice's bound unless half its distance is below reach(s).  Its arc in the
-// slice j places away is |f-q| / (2 cos a) with a, the angle to that slice's
-// far edge, at least j slice widths (the slices' widening exceeds slice_of's
-// uncertainty at the edges), and infinite from the eighth on:
-//     reach(s) = max over |j| <= 7 of cos(j 11.25 degrees) R(s + j),
-// rounded up.  R: the lane's slice's bound.  (Beside the plain maximum of the
-// bounds within 8 slices: 64 instead of 80 facilities offered a query on the
-// uniform workload at k=10, filter 243 -> 233 us for 16,384 queries; 141
-// instead of 292 on the clustered one, 1.92 -> 1.49 ms for 2000.)
-__device__ __forceinline__ float slice_reach(float R, int lane)
+// How far from q a facility can matter, by its slice; R: the lane's slice's
+// bound (min(k-th smallest arc, clip)).  Both are rounded up.
+// reach: a facility whose direction lies in slice s can lower no slice's bound
+// unless half its distance is below reach(s).  Its arc in the slice j places
+// away is |f-q| / (2 cos a) with a, the angle to that slice's far edge, at
+// least j slice widths (the slices' widening exceeds slice_of's uncertainty at
+// the edges), and infinite from the eighth on:
+//     reach(s) = max over |j| <= 7 of cos(j 11.25 degrees) R(s + j).
+// need: a facility strictly nearer to a user u than q has |f-q| < 2 |u-q|
+// cos a, a the angle between them, at least |j| - 1 widths from slice s to u's
+// slice s + j; a kept user's |u-q| is at most its slice's bound, inflated past
+// the user test's margins.  So only facilities with half their distance below
+//     need(s) = max over |j| <= 8 of cos(max(|j| - 1, 0) 11.25 degrees) R(s + j)
+// can be nearer than q to a kept user: the others are no half-planes at all.
+// (at least 1e-6 of the largest bound, for directions a rounding short of 90
+// degrees).  Stored per slice.
+__device__ __forceinline__ void store_reach(float R, int lane, float* reach, float* need)
 {
-    constexpr float C[8] = {1.0f, 0.980785280f, 0.923879533f, 0.831469612f, 0.707106781f, 0.555570233f,
-                            0.382683432f, 0.195090322f};
-    float t = R;
+    constexpr float C[9] = {1.0f, 0.980785280f, 0.923879533f, 0.831469612f, 0.707106781f, 0.555570233f,
+                            0.382683432f, 0.195090322f, 0.0f};
+    float t = R, n = R;
 #pragma unroll
-    for (int j = 1; j < 8; ++j)
-        t = fmaxf(t, C[j] * fmaxf(__shfl_sync(FULL, R, (lane + j) & 31), __shfl_sync(FULL, R, (lane - j) & 31)));
-    return t * (1.0f + 1e-6f);
+    for (int j = 1; j <= 8; ++j) {
+        const float m = fmaxf(__shfl_sync(FULL, R, (lane + j) & 31), __shfl_sync(FULL, R, (lane - j) & 31));
+        if (j < 8) t = fmaxf(t, C[j] * m);
+        n = fmaxf(n, C[j - 1] * m);
+    }
+    float top = R;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
+    __syncwarp();               // the last ones have been read
+    if (reach) reach[lane] = t * (1.0f + 1e-6f);
+    need[lane] = fmaxf(n * (1.0f + 2e-5f), 1e-6f * top);
+    __syncwarp();
 }
 
 // Max-heap of one slice, interleaved across lanes: entry i of lane l at
@@ -219,6 +241,30 @@ __device__ __forceinline__ void list_insert(float (&L)[KR], float v)
 #pragma unroll
     for (int i = KR - 1; i > 0; --i) L[i] = fminf(L[i], fmaxf(L[i - 1], v));
     L[0] = fminf(L[0], v);
+}
+
+// Drops from lpos[0 .. n) the facilities beyond the current need, keeping the
+// order; returns how many are left.
+__device__ __forceinline__ int trim_planes(const float2* fxy, int nf, int* lpos, int n, float2 q, const float* Ns, int lane)
+{
+    int k = 0;
+    for (int m0 = 0; m0 < n; m0 += 32) {
+        const int m = m0 + lane;
+        int pos = 0;
+        float dx = 0.0f, dy = 0.0f;
+        if (m < n) {
+            pos = lpos[m];
+            const float2 f = fxy[SX(pos, nf, 334)];
+            dx = f.x - q.x;
+            dy = f.y - q.y;
+        }
+        const bool keep = m < n && !beyond(fmaf(dx, dx, dy * dy), Ns[slice_of(dx, dy)]);
+        const unsigned km = __ballot_sync(FULL, keep);          // (every lane has read its entry)
+        if (keep) lpos[k + __popc(km & ((1u << lane) - 1))] = pos;
+        k += __popc(km);
+        __syncwarp();
+    }
+    return k;
 }
 
 constexpr int FUSE_UPT = 4;     // users per lane per item of the fused verification
@@ -296,7 +342,8 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
     const SliceLayout LY = slice_layout(A.caps);
     char* wsm = smem + (size_t)wq * LY.bytes;           // this warp's region
     float* H = (float*)(wsm + LY.heap);
-    float* Rs = (float*)(wsm + LY.R);
+    float* Rs = (float*)(wsm + LY.R);          // the slices' bounds (while streaming: their reach)
+    float* Ns = Rs + 32;                        // the slices' need
     int* lpos = (int*)(wsm + LY.lpos);
     int* rowlo = (int*)(wsm + LY.rows);
     int* rowhi = rowlo + 2 * A.rmax + 1;
@@ -466,6 +513,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             pf_fe = A.fstart[SX(cid + 1, NCF + 1, 331)];
         }
         int ring = 0;
+        bool cut = false;       // the budget ended the stream
         for (; ring <= rmaxf; ++ring) {
             long long tp = clock64();
             const int cur_fs = pf_fs, cur_fe = pf_fe;
@@ -497,14 +545,14 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             // Every heap top is an upper bound at any time, so the stream may
             // stop early; past a budget the remaining (sparse-direction)
             // slices keep their bounds and the kept region grows instead.
-            if ((NWQ == 2 ? pts_all : zs.pts) >= fbudget) break;
-            // The slices' reach for the ring: a cell whose facilities are all
-            // farther than twice the largest reach of the slices it spans can
-            // lower no bound: its facilities become half-planes without being
-            // loaded or offered (plane-only).  (Rs serves as scratch until
-            // the stream ends.)
-            Rs[lane] = slice_reach(Rl, lane);
-            __syncwarp();
+            if ((NWQ == 2 ? pts_all : zs.pts) >= fbudget) {
+                cut = true;
+                break;
+            }
+            // The slices' reach and need for the ring: a cell whose
+            // facilities are all beyond the need of the slices it spans is
+            // passed over.
+            store_reach(Rl, lane, Rs, Ns);
             zs.cyc[3] += clock64() - tp;
             tp = clock64();
             // the ring's cells (8 ring of them, 1 for ring 0), one range each
@@ -512,7 +560,6 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             for (int r0 = 0; r0 < nrange; r0 += 32) {
                 const int ri = r0 + lane;
                 int fs = 0, fe = 0;
-                bool po = false;        // plane-only: the cell's facilities can enter no heap
                 if (ri < nrange && (NWQ == 1 || (ri & 1) == wq)) {
                     int cxx, cyy;
                     ring_cell(ring, ri, qcx, qcy, cxx, cyy);
@@ -523,18 +570,14 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                             fs = cur_fs;
                             fe = cur_fe;
                         }
+                        bool idle = false;
                         if (ring > 0 && (!ahead || fe > fs)) {
                             // the cell's box widened for the cell function's rounding
                             const float X0 = A.gf.x0 + (float)cxx * A.gf.cs - cmargin, X1 = A.gf.x0 + (float)(cxx + 1) * A.gf.cs + cmargin;
                             const float Y0 = A.gf.y0 + (float)cyy * A.gf.cs - cmargin, Y1 = A.gf.y0 + (float)(cyy + 1) * A.gf.cs + cmargin;
-                            po = plane_only(X0 - qf.x, X1 - qf.x, Y0 - qf.y, Y1 - qf.y, Rs);
+                            idle = box_idle(X0 - qf.x, X1 - qf.x, Y0 - qf.y, Y1 - qf.y, Ns);
                         }
-                        // once the half-planes are full (a facility of rho_ring
-                        // was left out), a plane-only cell has nothing to give:
-                        // its range is not even loaded (the far rings of a
-                        // query at a cluster's edge: the clustered
-                        // workload's slowest query 3.1 -> 2.3 M cycles)
-                        if (po && rho_ring >= 0) {
+                        if (idle) {
                             fs = fe = 0;
                         } else if (!ahead) {
                             fs = A.fstart[SX(cid, NCF + 1, 312)];
@@ -570,55 +613,53 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                     const int rs = __shfl_sync(FULL, fs, lo);
                     const int rincl = __shfl_sync(FULL, incl, lo);
                     const int rlen = __shfl_sync(FULL, len, lo);
-                    const bool rpo = __shfl_sync(FULL, (int)po, lo) != 0;
                     const int fidx = rs + (j - (rincl - rlen));
                     bool ok = j < total && fidx != qpos;
                     float vx = 0.0f, vy = 0.0f;
-                    if (ok && !rpo) {
+                    if (ok) {
                         const float2 f = A.fxy[SX(fidx, A.nf, 314)];
                         vx = f.x - qf.x;
                         vy = f.y - qf.y;
                         // a facility at q's position is never strictly nearer
-                        // (float differences are zero only for equal floats;
-                        // such a facility lies in q's cell, never plane-only)
+                        // (float differences are zero only for equal floats)
                         ok = vx != 0.0f || vy != 0.0f;
                     }
-                    // half-planes: the first LC facilities of the rings, in
-                    // ring order, those of plane-only cells included (so that
-                    // rho is limited only by the rings, below)
-                    const unsigned pm = __ballot_sync(FULL, ok);
+                    const int np = __popc(__ballot_sync(FULL, ok));
+                    zs.pts += np;
+                    if constexpr (NWQ == 2)
+                        if (lane == 0 && np) atomicAdd(xs + 7, np);
+                    // Offered to the bounds only within its slice's reach, a
+                    // half-plane only within its need.  Bounds only shrink, so
+                    // those taken before the batch are conservative.
+                    if constexpr (NWQ == 1) {
+                        // one warp: fresh ones from a ring's second batch on
+                        if (r0 + t0 > 0) store_reach(fminf(SLICE_KTH(), clip), lane, Rs, Ns);
+                    }
+                    const int sj = slice_of(vx, vy);
+                    const float rj = Rs[sj], nj = Ns[sj];
+                    const float d2 = fmaf(vx, vx, vy * vy);
+                    const bool hp = ok && !beyond(d2, nj);
+                    unsigned m = __ballot_sync(FULL, ok && !beyond(d2, rj));
+                    // half-planes: the first LC of them, in ring order
+                    const unsigned pm = __ballot_sync(FULL, hp);
                     int at0 = nL;       // this batch's first half-plane slot
                     if constexpr (NWQ == 2) {
                         int a = 0;
                         if (lane == 0 && pm) a = atomicAdd(xs + 6, __popc(pm));
                         at0 = __shfl_sync(FULL, a, 0);
+                    } else {
+                        // no room: those taken under looser bounds go
+                        if (nL + __popc(pm) > LC && rho_ring < 0) {
+                            nL = trim_planes(A.fxy, A.nf, lpos0, nL, qf, Ns, lane);
+                            at0 = nL;
+                        }
                     }
-                    if (ok) {
+                    if (hp) {
                         const int at = at0 + __popc(pm & ((1u << lane) - 1));
                         if (at < LC) lpos0[SX(at, LC, 315)] = fidx;
                     }
                     if (at0 + __popc(pm) > LC && rho_ring < 0) rho_ring = ring;
                     if constexpr (NWQ == 1) nL = min(LC, nL + __popc(pm));
-                    const unsigned om = __ballot_sync(FULL, ok && !rpo);      // offered to the bounds
-                    zs.pts += __popc(om);
-                    if constexpr (NWQ == 2)
-                        if (lane == 0 && om) atomicAdd(xs + 7, __popc(om));
-                    // Offered only within its slice's reach.  Bounds only shrink,
-                    // so the reaches taken before the batch are conservative.
-                    unsigned m = om;
-                    {
-                        const int sj = ok ? slice_of(vx, vy) : 0;
-                        float Rwj;
-                        if constexpr (NWQ == 2) {
-                            // the ring top's, over both warps' lists
-                            Rwj = Rs[sj];
-                        } else {
-                            // (arcs beyond the clip change no effective bound)
-                            Rwj = __shfl_sync(FULL, slice_reach(fminf(SLICE_KTH(), clip), lane), sj);
-                        }
-                        const bool useful = ok && !rpo && !(0.25f * fmaf(vx, vx, vy * vy) * (1.0f - 4.0f * kU32) >= Rwj * Rwj);
-                        m = __ballot_sync(FULL, useful);
-                    }
                     // every lane offers every useful facility to its slice
                     zs.cand += __popc(m);
                     const long long t_offer = clock64();
@@ -675,16 +716,15 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             nL = min(LC, xs[6]);
             zs.pts = xs[7];
         }
-        // rho: every facility outside the half-planes lies in ring rho_ring or
-        // beyond, at least (rho_ring - 1) cs from q (less the rounding slack)
-        float rho;
-        {
-            if (rho_ring < 0) rho_ring = ring;          // every streamed facility is a half-plane
-            if (rho_ring > rmaxf) rho = INFINITY;
-            else {
-                const float Lr = __fsub_rd(__fmul_rd((float)(rho_ring - 1), A.gf.cs), slack_f);
-                rho = Lr > 0.0f ? Lr : 0.0f;
-            }
+        // rho: every facility nearer to q than rho that can be nearer than q to
+        // a kept user is a half-plane: all of them when the stream ended by
+        // itself and none was left out, else those before ring rho_ring (or
+        // the ring the budget ended at), at least (rho_ring - 1) cs from q
+        // (less the rounding slack)
+        float rho = INFINITY;
+        if (rho_ring >= 0 || cut) {
+            const float Lr = __fsub_rd(__fmul_rd((float)((rho_ring < 0 ? ring : rho_ring) - 1), A.gf.cs), slack_f);
+            rho = Lr > 0.0f ? Lr : 0.0f;
         }
         zs.cyc[0] += clock64() - tph;
         tph = clock64();
@@ -701,21 +741,38 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         if (NWQ == 1 || wq == 0) {
         float4* planes = A.planes + (size_t)s * A.pstride;
         float cmax = 0.0f;
-        for (int m = lane; m < nL; m += 32) {
-            const int pos = lpos[SX(m, LC, 316)];
-            const float2 f = A.fxy[SX(pos, A.nf, 317)];
-            const float dx = f.x - qf.x, dy = f.y - qf.y;
-            const float c = fmaf(dx, dx, dy * dy);
-            planes[SX(m, A.pstride, 318)] = make_float4(-2.0f * dx, -2.0f * dy, c, 0.0f);
-            if (FUSED && m < A.fuse_sc) {
-                fzp[2 * m] = make_float4(-2.0f * dx, -2.0f * dx, -2.0f * dy, -2.0f * dy);
-                fzp[2 * m + 1] = make_float4(c, c, 0.0f, 0.0f);
+        // only those within the final bounds' need, in order
+        store_reach(Rs[lane], lane, nullptr, Ns);
+        int nk = 0;
+        for (int m0 = 0; m0 < nL; m0 += 32) {
+            const int m = m0 + lane;
+            int pos = 0;
+            float dx = 0.0f, dy = 0.0f;
+            if (m < nL) {
+                pos = lpos[SX(m, LC, 316)];
+                const float2 f = A.fxy[SX(pos, A.nf, 317)];
+                dx = f.x - qf.x;
+                dy = f.y - qf.y;
             }
-            A.bis_pos[(size_t)s * A.pstride + SX(m, A.pstride, 319)] = pos;
-            cmax = fmaxf(cmax, c);
-            // the slot is free now: |f - q|^2 rounded well down
-            lpos[SX(m, LC, 316)] = __float_as_int(__fmul_rd(c, 1.0f - 1e-6f));
+            const float c = fmaf(dx, dx, dy * dy);
+            const bool keep = m < nL && !beyond(c, Ns[slice_of(dx, dy)]);
+            const unsigned km = __ballot_sync(FULL, keep);      // (every lane has read its entry)
+            if (keep) {
+                const int o = nk + __popc(km & ((1u << lane) - 1));
+                planes[SX(o, A.pstride, 318)] = make_float4(-2.0f * dx, -2.0f * dy, c, 0.0f);
+                if (FUSED && o < A.fuse_sc) {
+                    fzp[2 * o] = make_float4(-2.0f * dx, -2.0f * dx, -2.0f * dy, -2.0f * dy);
+                    fzp[2 * o + 1] = make_float4(c, c, 0.0f, 0.0f);
+                }
+                A.bis_pos[(size_t)s * A.pstride + SX(o, A.pstride, 319)] = pos;
+                cmax = fmaxf(cmax, c);
+                // the slot is free now: |f - q|^2 rounded well down
+                lpos[SX(o, LC, 316)] = __float_as_int(__fmul_rd(c, 1.0f - 1e-6f));
+            }
+            nk += __popc(km);
+            __syncwarp();
         }
+        nL = nk;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(FULL, cmax, o));
         __syncwarp();

@@ -89,7 +89,7 @@ __host__ __device__ inline SliceLayout slice_layout(const ZoneCaps& c)
     SliceLayout L;
     size_t o = 0;
     L.heap = o;   o = zl_align(o + 4 * 32 * ((size_t)c.vc + ZL_SPARE));
-    L.R = o;      o = zl_align(o + 4 * 32);
+    L.R = o;      o = zl_align(o + 4 * 64);       // the slices' bounds and need
     L.lpos = o;   o = zl_align(o + 4 * ((size_t)c.lc + ZL_SPARE));
     L.rows = o;   o = zl_align(o + 4 * 2 * (2 * (size_t)c.rm + 1));
     L.bytes = o;

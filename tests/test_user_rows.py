@@ -1,6 +1,6 @@
 """The slice filter's kept region as user-grid rows: regions of more rows than
 it lists one by one, regions cut by the data's box, points on a line, users far
-from every facility.  Every answer equals the exact oracle's."""
+from every facility, more facilities in a cell than half-planes are kept.  Every answer equals the exact oracle's."""
 import numpy as np
 import pytest
 
@@ -20,6 +20,9 @@ def _points(layout):
     elif layout == "horizontal":
         f = np.stack([rng.uniform(-50, 50, 200), np.full(200, -7.0)], 1)
         u = np.stack([rng.uniform(-50, 50, 20_011), np.full(20_011, -7.0)], 1)
+    elif layout == "dense":                 # cells of thousands of facilities beside empty ones
+        f = np.concatenate([rng.normal((400, 400), 0.3, (4000, 2)), rng.uniform(0, 1000, (400, 2))])
+        u = np.concatenate([rng.normal((400, 400), 0.4, (8000, 2)), rng.uniform(0, 1000, (30_000, 2))])
     else:                                   # users in a corner, facilities in the opposite one
         f = rng.uniform(0, 10, (150, 2))
         u = np.concatenate([rng.uniform(900, 1000, (30_000, 2)), rng.uniform(0, 10, (500, 2))])
@@ -27,13 +30,13 @@ def _points(layout):
     return datagen.Dataset(f, u, np.arange(len(f), dtype=np.int32), np.arange(len(f), len(f) + len(u), dtype=np.int32))
 
 
-@pytest.mark.parametrize("layout", ["wide", "vertical", "horizontal", "corner"])
+@pytest.mark.parametrize("layout", ["wide", "vertical", "horizontal", "dense", "corner"])
 def test_regions_match_oracle(engine, layout):
     ds = _points(layout)
     o = O.Oracle.of(ds)
     # the facilities nearest to the box's sides and corners, and a few others
     near = [np.argmin(ds.fxy @ np.array(d, np.float32)) for d in [(1, 0), (-1, 0), (0, 1), (0, -1), (1, 1), (-1, -1)]]
-    qs = np.unique(np.concatenate([near, np.arange(0, ds.nf, 9)])).astype(np.int32)
+    qs = np.unique(np.concatenate([near, np.arange(0, ds.nf, max(9, ds.nf // 25))])).astype(np.int32)
     big = np.tile(qs, 1 + 1300 // qs.size)          # one warp a query instead of two
     with engine.Index.of(ds, filter="slice") as idx:
         for k in (1, 7, 20, 45):
