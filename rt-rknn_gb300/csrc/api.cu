@@ -122,6 +122,7 @@ struct Workspace {
     ZStats* d_zst = nullptr;
     long long* d_cand_off = nullptr;   // result region of each slot (64-bit offsets)
     int* d_reg_len = nullptr;          // and its length
+    int* d_ncand = nullptr;            // candidate users of each slot
     int* d_deflist = nullptr;          // slots the fused filter leaves to the verification kernel
     int *d_chunk_off = nullptr, *d_res_count = nullptr, *d_out_off = nullptr;
     int rcap = 1 << 18;            // ids a slot's region holds at most (raised when exceeded)
@@ -262,7 +263,7 @@ void free_ws(Workspace& w)
     cudaFree(w.d_qko);
     cudaFree(w.d_qd); cudaFree(w.d_planes); cudaFree(w.d_bispos); cudaFree(w.d_segs); cudaFree(w.d_zst);
     cudaFree(w.d_slice_r);
-    cudaFree(w.d_cand_off); cudaFree(w.d_reg_len); cudaFree(w.d_deflist); cudaFree(w.d_chunk_off);
+    cudaFree(w.d_cand_off); cudaFree(w.d_reg_len); cudaFree(w.d_deflist); cudaFree(w.d_chunk_off); cudaFree(w.d_ncand);
     cudaFree(w.d_out_off);
     cudaFree(w.d_zb[0]);        // the counters, statistics and result counts
     cudaFree(w.d_zb[1]);
@@ -498,6 +499,7 @@ rknn_status grow_ws(Workspace& w, int nqc, int lc, int sc)
         CK(dalloc(w.d_zst, nqc));
         CK(dalloc(w.d_cand_off, nqc + 1)); CK(dalloc(w.d_reg_len, nqc + 1)); CK(dalloc(w.d_chunk_off, nqc + 1));
         CK(dalloc(w.d_deflist, nqc));
+        CK(dalloc(w.d_ncand, nqc));
         // counters, statistics and per-slot result counts in one block, two
         // of them for alternate batches, both zero to begin with
         static_assert(sizeof(VStats) <= ZB_VSTATS_INTS * sizeof(int), "VStats outgrew its room");
@@ -733,7 +735,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     za.skip_coincident = ix->skip_coincident;
     za.vertex_test = ix->zone_vertex_test;
     za.seg_cap = w.seg_cap;
-    za.qd = w.d_qd; za.planes = w.d_planes; za.bis_pos = w.d_bispos; za.segs = w.d_segs; za.zst = w.d_zst;
+    za.qd = w.d_qd; za.ncand = w.d_ncand; za.planes = w.d_planes; za.bis_pos = w.d_bispos; za.segs = w.d_segs; za.zst = w.d_zst;
     za.slice_r = w.d_slice_r;
     za.pstride = b.pstride;
     VerifyArgs va;
@@ -810,7 +812,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     // fused batches: the filter's last block planned the left-over slots,
     // and the verification takes only those
     if (!b.fuse)
-        CK(launch_k(plan_kernel, 1, 1024, 0, st, pdl && ncls == 1, w.d_qd, nq, w.d_cand_off, w.d_reg_len,
+        CK(launch_k(plan_kernel, scan_blocks(nq), SCAN_THREADS, 0, st, pdl && ncls == 1, w.d_qd, (const int*)w.d_ncand, nq, w.d_cand_off, w.d_reg_len,
                     region_top(w), w.d_chunk_off, w.pool_cap, w.rcap, 32 * b.vupt * b.parts));
     mark(2);
     CK(launch_k(verify_fn(b.mode, b.vupt), b.vgrid, b.vwarps * 32, b.vsmem, st, pdl && (ncls == 1 || !b.fuse), va));
@@ -830,7 +832,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
         fs.region_top = region_top(w);
         fs.counters = w.d_counters;
     } else {
-        CK(launch_k(scan_counts_kernel, 1, 1024, 0, st, pdl, (const int*)w.d_res_count, (const int*)w.d_reg_len,
+        CK(launch_k(scan_counts_kernel, scan_blocks(nq), SCAN_THREADS, 0, st, pdl, (const int*)w.d_res_count, (const int*)w.d_reg_len,
                     (const long long*)region_top(w), nq, w.d_out_off, (const int*)w.d_counters, c.io.off_host));
     }
     mark(5);
@@ -1832,7 +1834,7 @@ std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_ptr[NOALLOC_MAX_DEVICES] = {};
 
 struct NoallocLayout {
-    int *counters, *q, *k, *chunk_off, *res_count, *out_off, *bispos, *pool, *out, *reg_len;
+    int *counters, *q, *k, *ncand, *chunk_off, *res_count, *out_off, *bispos, *pool, *out, *reg_len;
     long long *cand_off, *region_top;
     QDesc* qd;
     ZStats* zst;
@@ -1852,6 +1854,7 @@ NoallocLayout noalloc_layout(unsigned char* base, int lc, int seg_cap)
     L.counters = (int*)take(sizeof(int) * 16);
     L.q = (int*)take(sizeof(int));
     L.k = (int*)take(sizeof(int));
+    L.ncand = (int*)take(sizeof(int));
     L.cand_off = (long long*)take(sizeof(long long) * 2);
     L.region_top = (long long*)take(sizeof(long long));
     L.reg_len = (int*)take(sizeof(int));
@@ -1943,7 +1946,7 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     za.seg_cap = seg_cap;
     za.pstride = caps.lc;
     za.slice_r = nullptr;
-    za.qd = L.qd; za.planes = L.planes; za.bis_pos = L.bispos; za.segs = L.segs; za.zst = L.zst;
+    za.qd = L.qd; za.ncand = L.ncand; za.planes = L.planes; za.bis_pos = L.bispos; za.segs = L.segs; za.zst = L.zst;
     za.fault = L.counters + 4;
     // the kernels rknn_query picks for one query: the zone over a block
     // (when its capacities allow it, as in zone_launch) and the verification
@@ -1956,7 +1959,7 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     else zone_kernel_smem<<<1, 32 * ZONE_WARPS, zl * ZONE_WARPS, st>>>(za);
     CK(cudaGetLastError());
     constexpr int NA_UPT = 2;
-    plan_kernel<<<1, 1024, 0, st>>>(L.qd, 1, L.cand_off, L.reg_len, L.region_top, L.chunk_off, L.pool_cap,
+    plan_kernel<<<1, SCAN_THREADS, 0, st>>>(L.qd, L.ncand, 1, L.cand_off, L.reg_len, L.region_top, L.chunk_off, L.pool_cap,
                                     (int)std::min<long long>(L.pool_cap, INT32_MAX), 32 * NA_UPT);
     CK(cudaGetLastError());
 
@@ -1975,7 +1978,7 @@ extern "C" rknn_status rknn_query_noalloc(rknn_index* ix, int32_t q, int32_t k, 
     const size_t vsmem = (size_t)VERIFY_WARPS * verify_warp_bytes(va.stage_cap, 0);
     verify_fn(mode, NA_UPT)<<<2 * ix->num_sms, VERIFY_WARPS * 32, vsmem, st>>>(va);
     CK(cudaGetLastError());
-    scan_counts_kernel<<<1, 1024, 0, st>>>(L.res_count, L.reg_len, L.region_top, 1, L.out_off, L.counters, nullptr);
+    scan_counts_kernel<<<1, SCAN_THREADS, 0, st>>>(L.res_count, L.reg_len, L.region_top, 1, L.out_off, L.counters, nullptr);
     CK(cudaGetLastError());
     finalize_kernel<<<1, 32 * FIN_WARPS, 0, st>>>(L.pool, L.cand_off, L.reg_len, L.res_count, L.out_off, L.out, L.out, 1,
                                                   L.pool_cap, nullptr, 0, FinScan{});

@@ -406,6 +406,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 d.flags = QF_BAD_QUERY;
                 if (FUSED) fuse_claim(A, s, d, smem, FL, false);
                 *qd = d;
+                A.ncand[s] = d.ncand;
                 A.zst[s] = zs;
                 A.segs[(size_t)s * A.seg_cap] = make_int2(0, 0);
             }
@@ -430,6 +431,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 d.flags = QF_ALL_USERS;
                 if (FUSED) fuse_claim(A, s, d, smem, FL, false);
                 *qd = d;
+                A.ncand[s] = d.ncand;
                 A.zst[s] = zs;
                 int2* seg = A.segs + (size_t)s * A.seg_cap;
                 seg[0] = make_int2(0, 0);
@@ -1036,6 +1038,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
             d.pad = 0;
             if (FUSED) fuse_claim(A, s, d, smem, FL, true);
             *qd = d;
+            A.ncand[s] = d.ncand;
             if (!FUSED) put_stats();
         }
         if (FUSED) {

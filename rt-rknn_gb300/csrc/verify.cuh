@@ -85,13 +85,17 @@ __host__ __device__ __forceinline__ size_t verify_warp_bytes(int stage_cap, int 
 __global__ void recount_kernel(VerifyArgs a);       // FP32 filter
 __global__ void recount64_kernel(VerifyArgs a);     // FP64 filter
 
-// single block: result regions (min(candidates, rcap) ids at 64-bit offsets,
-// their lengths and *region_top = their total) and work-item offsets from
-// QDesc.ncand; flags slots whose region does not fit the pool
-__global__ void plan_kernel(QDesc* qd, int nq, long long* cand_off, int* reg_len, long long* region_top,
-                            int* chunk_off, long long pool_cap, int rcap, int chunk);
+// slots a block of the two scan kernels takes
+constexpr int SCAN_THREADS = 1024;
+inline int scan_blocks(int nq) { return (nq + SCAN_THREADS - 1) / SCAN_THREADS; }
 
-// single block: exclusive scan of the stored result counts into out_off
+// result regions (min(candidates, rcap) ids at 64-bit offsets, their lengths
+// and *region_top = their total) and work-item offsets from the slots'
+// candidate counts; flags slots whose region does not fit the pool
+__global__ void plan_kernel(QDesc* qd, const int* ncand, int nq, long long* cand_off, int* reg_len,
+                            long long* region_top, int* chunk_off, long long pool_cap, int rcap, int chunk);
+
+// exclusive scan of the stored result counts into out_off
 // out_off: nq+1 offsets, then OFF_TAIL ints: the region total (low and high
 // halves of *region_top), the dropped flag and the listed survivors
 // (counters[2], counters[3]), so that one copy brings back all of them.

@@ -87,6 +87,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                 d.k = k;
                 d.flags = QF_BAD_QUERY;
                 *qd = d;
+                A.ncand[s] = d.ncand;
                 A.zst[s] = zs;
                 A.segs[(size_t)s * A.seg_cap] = make_int2(0, 0);
             }
@@ -899,6 +900,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             d.rho = 0.0f;           // the zone's bisectors need not cover any disc
             d.pad = 0;
             *qd = d;
+            A.ncand[s] = d.ncand;
             A.zst[s] = zs;
         }
         WSYNC();

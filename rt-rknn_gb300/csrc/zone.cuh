@@ -125,6 +125,7 @@ struct ZoneArgs {
     int seg_cap;             // segments per query slot (>= 2*rmax+2)
     // outputs (per slot)
     QDesc* qd;
+    int* ncand;              // [slot]: the descriptor's candidate count, for plan_kernel
     float4* planes;          // [slot][pstride]
     int* bis_pos;            // [slot][pstride] facility positions of the bisectors
     int pstride;             // >= caps.lc: row stride of planes / bis_pos

@@ -426,6 +426,7 @@ __device__ __forceinline__ void zone_cta_body(const ZoneArgs& A)
                 d.k = k;
                 d.flags = QF_BAD_QUERY;
                 *qd = d;
+                A.ncand[s] = d.ncand;
                 A.zst[s] = zs;
                 A.segs[(size_t)s * A.seg_cap] = make_int2(0, 0);
             }
@@ -1285,6 +1286,7 @@ __device__ __forceinline__ void zone_cta_body(const ZoneArgs& A)
             d.rho = 0.0f;
             d.pad = 0;
             *qd = d;
+            A.ncand[s] = d.ncand;
             A.zst[s] = zs;
         }
     }

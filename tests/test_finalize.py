@@ -42,3 +42,18 @@ def test_sorted_ids_in_every_output(n, far):
             for got in idx.query_batch(qs, 2, mode):
                 assert np.array_equal(got, want[:n])
             assert np.array_equal(idx.query(0, 2, mode), want[:n])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq", [1023, 1024, 1025, 2049, 4097])
+def test_regions_past_the_pool(nq):
+    """Every query returns 9001 ids: more than a fresh workspace's pool (4096 a
+    query) holds, so the first launch skips the slots past its end and the
+    batch runs again; the scans' blocks take 1024 slots each."""
+    n = 9001
+    ids = np.random.default_rng(nq).permutation(n).astype(np.int32)
+    with _index(n, ids, 0) as idx:
+        for mode in ("fp64", "fp32"):
+            got, off = idx.query_batch_flat(np.zeros(nq, np.int32), 3, mode)
+            assert np.array_equal(off, n * np.arange(nq + 1))
+            assert np.array_equal(got.reshape(nq, n), np.tile(np.arange(n, dtype=np.int32), (nq, 1)))
