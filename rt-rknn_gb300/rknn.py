@@ -195,9 +195,9 @@ _fast = None
 
 
 def _fast_call():
-    """The CPython entry point for rknn_query_batch (host/pycall.c, built
-    beside the library where the interpreter's headers are installed), or
-    False: ctypes then makes the same call."""
+    """The CPython entry points for the calls made most often (host/pycall.c,
+    built beside the library where the interpreter's headers are installed), or
+    False: ctypes then makes the same calls."""
     global _fast
     if _fast is None:
         load()                  # the module links against the loaded library
@@ -321,9 +321,14 @@ class Index:
 
     def query(self, q: int, k: int, mode="fp64", stats: bool = False):
         """Sorted user ids of RkNN_k(q) (rknn_query: one query, one launch)."""
-        L = load()
         cap = max(16, self.nu)
         out = np.empty(cap, np.int32)
+        fast = _fast if _fast is not None else _fast_call()
+        if fast and not stats:
+            rc, n = fast.query(self.h.value if self.h else 0, int(q), int(k), _MODES[mode], out)
+            _check(rc)
+            return out[:n].copy()
+        L = load()
         n = C.c_int64(0)
         st = Stats()
         _check(L.rknn_query(self.h, int(q), int(k), _MODES[mode], out.ctypes.data, cap,
@@ -481,25 +486,34 @@ class Server:
         _check(L.rknn_serve_start(index.h, C.byref(o), C.byref(self.h)))
 
     def submit(self, q: int, k: int, mode="fp32") -> int:
+        fast = _fast if _fast is not None else _fast_call()
+        if fast:
+            rc, t = fast.serve_submit(self.h.value or 0, int(q), int(k), _MODES[mode])
+            _check(rc)
+            return t
         t = C.c_uint64(0)
         _check(load().rknn_serve_submit(self.h, int(q), int(k), _MODES[mode], C.byref(t)))
         return t.value
 
     def wait(self, ticket: int, timeout_ms: int = -1, latency: bool = False):
+        fast = _fast if _fast is not None else _fast_call()
         L = load()
-        n = C.c_int64(0)
-        lat = C.c_double(0)
         cap = 1024
         while True:
             out = np.empty(cap, np.int32)
-            rc = L.rknn_serve_wait(self.h, C.c_uint64(ticket), int(timeout_ms), out.ctypes.data, cap,
-                                   C.byref(n), C.byref(lat))
-            if rc == 5 and n.value > cap:            # RKNN_ERR_CAPACITY: request kept
-                cap = int(n.value)
+            if fast:
+                rc, n, lat = fast.serve_wait(self.h.value or 0, ticket, int(timeout_ms), out)
+            else:
+                nn, ll = C.c_int64(0), C.c_double(0)
+                rc = L.rknn_serve_wait(self.h, C.c_uint64(ticket), int(timeout_ms), out.ctypes.data, cap,
+                                       C.byref(nn), C.byref(ll))
+                n, lat = nn.value, ll.value
+            if rc == 5 and n > cap:                  # RKNN_ERR_CAPACITY: request kept
+                cap = n
                 continue
             _check(rc)
-            ids = out[: n.value].copy()
-            return (ids, lat.value) if latency else ids
+            ids = out[:n].copy()
+            return (ids, lat) if latency else ids
 
     def replay(self, q, k, mode, arrival_s):
         """Open-loop load: request i at arrival_s[i] s; returns (latency_ms, n_results)."""
