@@ -608,8 +608,8 @@ __device__ __forceinline__ void warp_sort_regs(unsigned (&x)[E], int lane)
     }
 }
 
-template <int E>
-__device__ __forceinline__ void warp_sort_slot(const unsigned* src, unsigned* dst, int n, int lane)
+template <int E, bool TWIN>
+__device__ __forceinline__ void warp_sort_slot(const unsigned* src, unsigned* dst, unsigned* twin, int n, int lane)
 {
     unsigned x[E];
 #pragma unroll
@@ -621,7 +621,10 @@ __device__ __forceinline__ void warp_sort_slot(const unsigned* src, unsigned* ds
 #pragma unroll
     for (int t = 0; t < E; ++t) {
         const int i = (t << 5) | lane;
-        if (i < n) dst[i] = x[t] ^ 0x80000000u;
+        if (i < n) {
+            dst[i] = x[t] ^ 0x80000000u;
+            if (TWIN && twin) twin[i] = x[t] ^ 0x80000000u;
+        }
     }
 }
 }  // namespace
@@ -630,9 +633,10 @@ __device__ __forceinline__ void warp_sort_slot(const unsigned* src, unsigned* ds
 // 32 ids by rank counting in registers, up to FIN_WCAP by a bitonic network
 // in registers; larger sets are listed for sort_large_kernel where the batch
 // launches it, else radix sorted through the slot's pool region.
-__global__ void __launch_bounds__(32 * FIN_WARPS, 1)
-finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
-                int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero, long long zero_n, FinScan S)
+template <bool TWIN>
+__device__ __forceinline__ void finalize_body(int* res_pool, const long long* cand_off, const int* reg_len,
+                                              const int* res_count, int* out_off, int* out, int* stage, int nq,
+                                              long long out_cap, int* zero, long long zero_n, const FinScan& S)
 {
     // the next batch's counters (no kernel of this batch uses them), while
     // the predecessor drains
@@ -695,6 +699,7 @@ finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, co
         const int os = S.on ? s_off[w] : out_off[s];
         unsigned* src = (unsigned*)(res_pool + cand_off[s]);
         unsigned* dst = (unsigned*)(out + os);
+        unsigned* twin = TWIN && (long long)os + n <= S.twin_cap ? (unsigned*)(S.twin + os) : nullptr;
         if ((long long)os + n > out_cap) {
             // past the output's capacity: left out (the batch fails on the host)
         } else if (n <= 32) {
@@ -705,22 +710,41 @@ finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, co
                 const unsigned o = __shfl_sync(FULL, key, j);
                 rank += (o < key) || (o == key && j < lane);
             }
-            if (lane < n) dst[rank] = key ^ 0x80000000u;
+            if (lane < n) {
+                dst[rank] = key ^ 0x80000000u;
+                if (TWIN && twin) twin[rank] = key ^ 0x80000000u;
+            }
         } else if (n <= 64) {
-            warp_sort_slot<2>(src, dst, n, lane);
+            warp_sort_slot<2, TWIN>(src, dst, twin, n, lane);
         } else if (n <= 128) {
-            warp_sort_slot<4>(src, dst, n, lane);
+            warp_sort_slot<4, TWIN>(src, dst, twin, n, lane);
         } else if (n <= 256) {
-            warp_sort_slot<8>(src, dst, n, lane);
+            warp_sort_slot<8, TWIN>(src, dst, twin, n, lane);
         } else if (n <= FIN_WCAP) {
-            warp_sort_slot<16>(src, dst, n, lane);
+            warp_sort_slot<16, TWIN>(src, dst, twin, n, lane);
         } else if (S.large) {
             // left to sort_large_kernel
             if (lane == 0) S.large[atomicAdd(S.nlarge, 1)] = s;
         } else {
             warp_radix_slot(src, (unsigned*)(stage + os), dst, n, lane, bins[w]);
+            __syncwarp();
+            if (TWIN && twin)
+                for (int i = lane; i < n; i += 32) twin[i] = dst[i];
         }
     }
+}
+
+__global__ void __launch_bounds__(32 * FIN_WARPS, 1)
+finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
+                int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero, long long zero_n, FinScan S)
+{
+    finalize_body<false>(res_pool, cand_off, reg_len, res_count, out_off, out, stage, nq, out_cap, zero, zero_n, S);
+}
+__global__ void __launch_bounds__(32 * FIN_WARPS, 1)
+finalize_twin_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
+                     int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero, long long zero_n, FinScan S)
+{
+    finalize_body<true>(res_pool, cand_off, reg_len, res_count, out_off, out, stage, nq, out_cap, zero, zero_n, S);
 }
 
 // ------------------------------------------------------- large result sets

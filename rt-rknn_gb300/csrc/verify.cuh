@@ -120,6 +120,11 @@ struct FinScan {
     // sorted by their warps)
     int* large = nullptr;
     int* nlarge = nullptr;
+    // a second copy of the sorted ids, in device-accessible host memory of
+    // twin_cap ids (null: none; not with large): slots that would pass its end
+    // are left out of it
+    int* twin = nullptr;
+    long long twin_cap = 0;
 };
 
 // Sets above FIN_WCAP ids, a block each (persistent blocks, *queue counts the
@@ -145,5 +150,10 @@ size_t sort_large_smem();
 __global__ void finalize_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
                                 int* out_off, int* out, int* stage, int nq, long long out_cap, int* zero,
                                 long long zero_n, FinScan S);
+// the same with the second copy (S.twin)
+__global__ void finalize_twin_kernel(int* res_pool, const long long* cand_off, const int* reg_len,
+                                     const int* res_count, int* out_off, int* out, int* stage, int nq,
+                                     long long out_cap, int* zero, long long zero_n, FinScan S);
+
 
 }  // namespace rknn
