@@ -602,6 +602,7 @@ struct BatchPlan {
     int stage_cap = 0;          // half-planes the verification uses per slot
     int seg_stage = 0;          // user segments it stages per warp
     int vupt = VERIFY_UPT, vwarps = VERIFY_WARPS;
+    int list_cand = -1;         // see LIST_CAND
     int parts = 1;              // parts of 32 vupt users in a verification work item
     bool fuse = false;          // the slice filter verifies its own slots (FP32, every class a slice class)
     size_t vsmem = 0;
@@ -655,6 +656,8 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     // (half-planes beyond these are left out: the filter weakens, the exact
     // recount still decides)
     b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
+    if (nq <= LIST_QUERIES && std::none_of(b.cls.begin(), b.cls.end(), [](const ZClass& c) { return c.slice; }))
+        b.list_cand = LIST_CAND;
     int rm = 0;
     for (auto& c : b.cls) rm = std::max(rm, c.caps.rm);
     b.seg_stage = std::min(2 * rm + 2, SEG_STAGE_MAX);
@@ -747,6 +750,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     va.slice_r = w.d_slice_r;
     va.stage_cap = b.stage_cap;
     va.parts = b.parts;
+    va.list_cand = b.list_cand;
     va.segs = w.d_segs; va.seg_cap = w.seg_cap; va.seg_stage = b.seg_stage;
     va.chunk_off = w.d_chunk_off; va.cand_off = w.d_cand_off; va.reg_len = w.d_reg_len; va.nq = nq;
     va.uxy = ix->d_uxy; va.uid = ix->d_uid; va.fxy = ix->d_fxy; va.fstart = ix->d_fstart; va.gf = ix->gf;

@@ -61,7 +61,7 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
         for (int i = threadIdx.x; i < nsmp; i += blockDim.x) csmp[i] = A.chunk_off[i * st];
     __syncthreads();
     int cur = -1;
-    bool seg_staged = false, boxed = false;
+    bool seg_staged = false, boxed = false, listed = false;
     int nsp = 0;
     // per-warp statistics (32-bit here, 64-bit in the totals)
     VCount vc = {};
@@ -118,8 +118,11 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
             __syncwarp();
             const float4* src = A.planes + (size_t)s * A.lc;
             const int nst = min(d.nb, A.stage_cap);
-            boxed = F64 || d.ncand >= BOX_MIN_CAND;
-            if (boxed) {
+            listed = A.list_cand >= d.ncand;
+            boxed = listed || F64 || d.ncand >= BOX_MIN_CAND;
+            if (listed) {
+                // no half-planes needed
+            } else if (boxed) {
                 if (nst > 0)
                     for (int m = 8 * lane; m < nst + 7; m += 8 * 32) prefetch_l1(src + min(m, nst - 1));
             } else {
@@ -173,6 +176,10 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
             float2 u[UPT];
             bool valid[UPT], direct[UPT], surv[UPT];
             item_users<UPT>(A, d, s, v0, sg, sr, false, pos, u, valid, vc);
+            if (listed) {
+#pragma unroll
+                for (int t = 0; t < UPT; ++t) { direct[t] = false; surv[t] = valid[t]; }
+            } else
             filter_boxed<UPT, F64>(A, d, nbs, gp, A.bis_pos + (size_t)s * A.lc, BS, u, valid, direct, surv, vc.evals,
                                    rho2);
             item_emit<UPT, F64>(A, d, s, pos, direct, surv, -1, -1, vc);

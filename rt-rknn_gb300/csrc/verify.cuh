@@ -9,6 +9,14 @@ constexpr int VERIFY_CHUNK = 32 * VERIFY_UPT;       // default users per work it
 constexpr int VERIFY_WARPS = 8;                     // default warps per block
 constexpr int VERIFY_SAMPLES = 1024;                // work-item offsets cached per block
 constexpr int BOX_MIN_CAND = 512;                   // FP32: candidates from which boxes come first
+// Most queries of an influence-zone batch, and candidates of a query, that go
+// to the recount without a half-plane test.  The zone's half-planes reject
+// about half of the candidates and accept none (its pruning may have dropped a
+// needed facility, so those left are counted anyway), and a few queries leave
+// most warps idle: counting all candidates takes the recount no longer, and the
+// half-plane tests' chain is saved (one FP64 query at k=10: verification
+// 26 -> 8 us).
+constexpr int LIST_QUERIES = 16, LIST_CAND = 4096;
 constexpr int VERIFY_PLANES_MAX = 1024;             // half-planes used per slot (32 box masks of 32)
 constexpr int FIN_WARPS = 8;                        // finalize: slots per block (one warp each)
 constexpr int FIN_WCAP = 512;                       // ids one warp sorts in registers
@@ -22,6 +30,7 @@ struct VerifyArgs {
     int lc;                  // row stride of planes / bis_pos
     int stage_cap;           // half-planes used per slot, at most 1024 (the first ones;
                              // fewer only means more users reach the exact recount)
+    int list_cand = -1;      // slots of up to this many candidates go to the recount whole
     int parts = 1;           // parts of 32 * (users per lane) users in a work item
     const int2* segs;        // [slot][seg_cap]
     int seg_cap;
