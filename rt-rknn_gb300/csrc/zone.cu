@@ -23,6 +23,15 @@
 // bisectors are discarded before the FP64 division: the reference creates and
 // then erases them in the same step.
 //
+// What bounds it: the chain of one warp's dependent steps (a batch of 1000 keeps
+// 6.6 warps on an SM), FP64 instructions of about 65 cycles each among them.  So
+// the queue is a sorted array that the whole warp merges into and a pop reads
+// (a heap popped by one lane: 131 k cycles a query, now 36 k), the live
+// candidates are listed and counted by groups of lanes, the farthest vertex
+// comes from passes that run anyway, without its square root, and compares and
+// conversions of doubles run on their bits.  999 queries at k=10: 1.69 -> 1.35
+// ms.  (Loading each pass's next vertices ahead gained nothing: 1.38.)
+//
 // Epilogue: the bisectors become exact half-planes relative to q for the
 // verification kernel, and a ring scan over the user grid keeps every cell
 // that is not certified to lie on the strict far side of >= k bisectors.  The
@@ -42,6 +51,92 @@ namespace rknn {
 // Lanes hand zone state to each other through shared memory between warp
 // barriers.
 #define WSYNC() __syncwarp()
+
+namespace {
+// The priority queue: (K, C)[0 .. n) in descending (key, code) order, so the
+// next entry is the last one and a pop is one read.  Merges the batch
+// tk/tc[0 .. m), m <= 32: from the end on, each old entry moves past the new
+// ones greater than it, 32 at a time, and each new one counts the old and new
+// ones greater than itself.  Entries beyond cap are not taken (*over is set).
+// Codes are unique, so the sequence of entries taken is a heap's.
+__device__ __forceinline__ void wq_merge(uint64_t* K, uint32_t* C, int& n, const uint64_t* tk, const uint32_t* tc,
+                                         int m, int cap, bool& over)
+{
+    const int lane = threadIdx.x & 31;
+    WSYNC();
+    if (n + m > cap) {
+        over = true;
+        m = cap - n;
+    }
+    if (m <= 0) return;
+    const uint64_t nk = lane < m ? tk[lane] : 0;
+    const uint32_t nc = lane < m ? tc[lane] : 0;
+    int pos = 0;
+    for (int e = 0; e < m; ++e) pos += pq_less(nk, nc, tk[e], tc[e]);
+    for (int c0 = (n - 1) & ~31; c0 >= 0; c0 -= 32) {
+        const int j = c0 + lane;
+        const bool in = j < n;
+        const uint64_t k = in ? K[j] : 0;
+        const uint32_t c = in ? C[j] : 0;
+        int shift = 0;
+        for (int e = 0; e < m; ++e) {
+            const bool less = pq_less(k, c, tk[e], tc[e]);
+            shift += less;
+            const int g = __popc(__ballot_sync(FULL, in && !less));
+            if (lane == e) pos += g;
+        }
+        WSYNC();
+        if (in && shift) { K[j + shift] = k; C[j + shift] = c; }
+        // every entry here is greater than every new one: so are those before
+        if (!__any_sync(FULL, in && shift)) { pos += c0; break; }
+    }
+    WSYNC();
+    if (lane < m) { K[pos] = nk; C[pos] = nc; }
+    n += m;
+    WSYNC();
+}
+
+// Extreme boundary points (inf.cpp:283-321): extreme j (left min/max y, right
+// min/max y, bottom min/max x, top min/max x) is the first strict minimum or
+// maximum over the list of boundary vertices in vertex order: the least key
+// (largest for a maximum), the earliest vertex among equal keys.  Each lane
+// keeps its best, then 32-bit warp minima of the key's words (the sign bit
+// flipped; all bits flipped for a maximum) and of the vertex index.  ext[j] =
+// vertex index or -1.
+__device__ __forceinline__ void warp_extremes(const Slice& S, int nB, int (&ext)[8])
+{
+    const int lane = threadIdx.x & 31;
+    long long bk[8];
+    int bp[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { bk[j] = 0; bp[j] = INT_MAX; }
+    for (int t = lane; t < nB; t += 32) {
+        const int vi = IX(S.blist, t);
+        const uint32_t fl = vfl_of(IX(S.v4, vi).w);
+        const double2 p = IX(S.vd, vi);
+        const long long kx = order_key(p.x), ky = order_key(p.y);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t ebit = j < 2 ? VB_EL : j < 4 ? VB_ER : j < 6 ? VB_EB : VB_ET;
+            if (!(fl & ebit)) continue;
+            const long long kk = j < 4 ? ky : kx;
+            if (bp[j] == INT_MAX || ((j & 1) == 0 ? kk < bk[j] : kk > bk[j])) { bk[j] = kk; bp[j] = vi; }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const bool has = bp[j] != INT_MAX;
+        unsigned long long u = (unsigned long long)bk[j] ^ 0x8000000000000000ull;
+        if (j & 1) u = ~u;
+        const unsigned hi = has ? (unsigned)(u >> 32) : 0xffffffffu;
+        const unsigned lo = has ? (unsigned)u : 0xffffffffu;
+        const bool c1 = hi == __reduce_min_sync(FULL, hi);
+        const unsigned mlo = __reduce_min_sync(FULL, c1 ? lo : 0xffffffffu);
+        const unsigned at = __reduce_min_sync(FULL, c1 && lo == mlo ? (unsigned)bp[j] : (unsigned)INT_MAX);
+        ext[j] = at == (unsigned)INT_MAX ? -1 : (int)at;
+    }
+}
+}  // namespace
 
 __device__ __forceinline__ void zone_body(const ZoneArgs& A)
 {
@@ -66,6 +161,8 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
     const float fsx0 = __double2float_rd(sx0), fsy0 = __double2float_rd(sy0);
     const float fsx1 = __double2float_ru(sx1), fsy1 = __double2float_ru(sy1);
     const double slack = 1e-5 * ((double)A.gf.cs + fmax(fmax(fabs(sx0), fabs(sx1)), fmax(fabs(sy0), fabs(sy1))));
+    const float slack_ru = __double2float_ru(slack);
+    const long long kx0 = order_key(sx0), kx1 = order_key(sx1), ky0 = order_key(sy0), ky1 = order_key(sy1);
     // coordinates within EPS in double are within EPS + 2E as floats
     const float tolE = (1e-9f + 2.0f * E) * (1.0f + 0x1p-20f);
 
@@ -100,7 +197,8 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
         // Warp-uniform scalars live in registers (identical in every lane);
         // lane 0 alone touches the heap and broadcasts what it changes.
         int nV = 4, nL = 0, nP = 0, nCons = -1, flags = 0;
-        double far_ = 0.0, nearb = DBL_MAX;
+        double nearb = DBL_MAX;
+        float nearf = INFINITY;         // nearb rounded up
 
         // ---- init: four space corners (inf.cpp:211-226) -------------------
         double d2c = 0.0;
@@ -113,9 +211,12 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                                          vpack(0, VB_BND | edge_bits(x, y, sx0, sy0, sx1, sy1)));
         }
         WSYNC();
-        far_ = __dsqrt_rn(warp_max(d2c));
-        // integer thresholds of rules 1 and 2 on the queue keys
-        Cut K1 = sqrt_cut(2.0 * far_, false);
+        // the farthest vertex's squared distance (bits), and what rule 1 and
+        // the ring gate derive from it without its square root; rule 2's
+        // integer thresholds on the queue keys
+        long long far2 = __double_as_longlong(warp_max(d2c));
+        Cut K1 = far_cut(far2);
+        float ring_T = ring_limit32(far2, slack_ru);
         Cut K2 = sqrt_cut(2.0 * DBL_MAX, true);  // nearest bisector: none yet (threshold +inf)
 
         long long tph = clock64();
@@ -126,19 +227,14 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
         int ring = 0;        // next facility ring to expand
         bool ring_open;
         uint64_t ring_key;
-        ring_gate(ring, rmaxf, (double)A.gf.cs, slack, far_, ring_open, ring_key);
+        ring_gate32(ring, rmaxf, A.gf.cs, slack_ru, ring_T, ring_open, ring_key);
 
         // ---- best-first search --------------------------------------------
         for (;;) {
             // make the top poppable: expand rings whose cells could precede it
             for (;;) {
                 if (!ring_open) break;
-                if (nP > 0) {
-                    uint64_t top = 0;
-                    if (lane == 0) top = IX(S.pqk, 0);
-                    top = __shfl_sync(FULL, top, 0);
-                    if (top < ring_key) break;
-                }
+                if (nP > 0 && IX(S.pqk, nP - 1) < ring_key) break;
                 // expand ring `ring`: 8*ring cells (1 for ring 0)
                 const int ncell = ring == 0 ? 1 : 8 * ring;
                 for (int t0 = 0; t0 < ncell; t0 += 32) {
@@ -165,31 +261,21 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                     const unsigned m = __ballot_sync(FULL, ok);
                     const int rank = __popc(m & ((1u << lane) - 1));
                     if (ok) { IX(S.tk, rank) = (uint64_t)__double_as_longlong(key); IX(S.tc, rank) = (uint32_t)cid; }
-                    WSYNC();
-                    if (lane == 0) {
-                        for (int i = 0; i < __popc(m); ++i)
-                            if (!pq_push(S.pqk.p, S.pqc.p, nP, PC, IX(S.tk, i), IX(S.tc, i))) { flags |= QF_ZONE_PQ_OVERFLOW; break; }
-                    }
-                    nP = __shfl_sync(FULL, nP, 0);
-                    flags = __shfl_sync(FULL, flags, 0);
-                    WSYNC();
+                    bool over = false;
+                    wq_merge(S.pqk.p, S.pqc.p, nP, S.tk.p, S.tc.p, __popc(m), PC, over);
+                    if (over) { flags |= QF_ZONE_PQ_OVERFLOW; break; }
                 }
                 ring++;
-                ring_gate(ring, rmaxf, (double)A.gf.cs, slack, far_, ring_open, ring_key);
+                ring_gate32(ring, rmaxf, A.gf.cs, slack_ru, ring_T, ring_open, ring_key);
                 if (flags) break;
             }
             PHASE(0);
             if (flags || nP == 0) break;
-            uint64_t keybits = 0;
-            uint32_t code = 0;
-            if (lane == 0) {
-                keybits = IX(S.pqk, 0);
-                code = IX(S.pqc, 0);
-                pq_pop(S.pqk.p, S.pqc.p, nP);
-            }
-            keybits = __shfl_sync(FULL, keybits, 0);
-            code = __shfl_sync(FULL, code, 0);
-            nP = __shfl_sync(FULL, nP, 0);
+            // pop: the last entry (nothing writes the queue until a merge, which
+            // starts at a warp barrier)
+            --nP;
+            const uint64_t keybits = IX(S.pqk, nP);
+            const uint32_t code = IX(S.pqc, nP);
             const double key = __longlong_as_double((long long)keybits);
 
             const bool is_point = (code & KIND_POINT) != 0;
@@ -217,7 +303,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             bool r1;
             if (keybits >= K1.hi) r1 = true;
             else if (keybits <= K1.lo) r1 = false;
-            else r1 = sqrt_rn64(key) > 2.0 * far_;
+            else r1 = sqrt_rn64(key) > 2.0 * sqrt_rn64(__longlong_as_double(far2));
             if (r1) break;
             // rule 2: keep when nearer than twice the nearest bisector
             bool r2;
@@ -252,47 +338,11 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                         nB += __popc(mb);
                     }
                     WSYNC();
-                    // Extreme boundary points (inf.cpp:283-321): lane j < 8 keeps
-                    // extreme j over the list in vertex order, the first strict
-                    // min / max winning as the reference's pointer updates do:
-                    // left min/max y, right min/max y, bottom min/max x, top min/max x.
-                    // The list is read 32 entries at a time and broadcast.
-                    int best = -1;
-                    {
-                        const bool byY = lane < 4;
-                        const bool wantMin = (lane & 1) == 0;
-                        const uint32_t ebit = lane < 2 ? VB_EL : lane < 4 ? VB_ER : lane < 6 ? VB_EB : VB_ET;
-                        long long bk = 0;
-                        for (int t0 = 0; t0 < nB; t0 += 32) {
-                            const int t = t0 + lane;
-                            int vi = 0;
-                            uint32_t fl = 0;
-                            long long kx = 0, ky = 0;
-                            if (t < nB) {
-                                vi = IX(S.blist, t);
-                                fl = vfl_of(IX(S.v4, vi).w);
-                                const double2 p = IX(S.vd, vi);
-                                kx = order_key(p.x);
-                                ky = order_key(p.y);
-                            }
-                            const int n = min(32, nB - t0);
-                            for (int u = 0; u < n; ++u) {
-                                const int ui = __shfl_sync(FULL, vi, u);
-                                const uint32_t uf = __shfl_sync(FULL, fl, u);
-                                const long long ukx = __shfl_sync(FULL, kx, u);
-                                const long long uky = __shfl_sync(FULL, ky, u);
-                                if (lane < 8 && (uf & ebit)) {
-                                    const long long kk = byY ? uky : ukx;
-                                    if (best < 0 || (wantMin ? kk < bk : kk > bk)) { best = ui; bk = kk; }
-                                }
-                            }
-                        }
-                    }
                     int ext[8];
+                    warp_extremes(S, nB, ext);
                     float ex[8], ey[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        ext[j] = __shfl_sync(FULL, best, j);
                         ex[j] = 0.0f; ey[j] = 0.0f;
                         if (ext[j] >= 0) {
                             const float4 e = IX(S.v4, ext[j]);
@@ -313,7 +363,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                                 for (int j = 0; j < 8; ++j) {
                                     if (c || ext[j] < 0 || fabsf(v.x - ex[j]) > tolE || fabsf(v.y - ey[j]) > tolE) continue;
                                     const double2 a = IX(S.vd, vi), b = IX(S.vd, ext[j]);
-                                    if (fabs(__dsub_rn(a.x, b.x)) < EPS && fabs(__dsub_rn(a.y, b.y)) < EPS) c = true;
+                                    if (within_eps(a.x, b.x) && within_eps(a.y, b.y)) c = true;
                                 }
                             }
                         }
@@ -364,15 +414,9 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                         IX(S.tk, lane) = (uint64_t)__double_as_longlong(d2_64(qx, qy, (double)pf.x, (double)pf.y));
                         IX(S.tc, lane) = KIND_POINT | (uint32_t)t;
                     }
-                    WSYNC();
-                    if (lane == 0) {
-                        const int cnt = min(32, p1 - t0);
-                        for (int i = 0; i < cnt; ++i)
-                            if (!pq_push(S.pqk.p, S.pqc.p, nP, PC, IX(S.tk, i), IX(S.tc, i))) { flags |= QF_ZONE_PQ_OVERFLOW; break; }
-                    }
-                    nP = __shfl_sync(FULL, nP, 0);
-                    flags = __shfl_sync(FULL, flags, 0);
-                    WSYNC();
+                    bool over = false;
+                    wq_merge(S.pqk.p, S.pqc.p, nP, S.tk.p, S.tc.p, min(32, p1 - t0), PC, over);
+                    if (over) { flags |= QF_ZONE_PQ_OVERFLOW; break; }
                 }
                 if (flags) break;
                 continue;
@@ -386,36 +430,52 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             nb.b = __shfl_sync(FULL, nb.b, 0);
             nb.vert = __shfl_sync(FULL, nb.vert, 0);
             nb.valid = __shfl_sync(FULL, nb.valid, 0);
-            const float na32 = (float)nb.a, nb32 = (float)nb.b;
+            const float na32 = d2f_bits<0>(nb.a), nb32 = d2f_bits<0>(nb.b);
             const float nab = fabsf(na32);
             zs.nb++;
 
-            // (1) count pass over the existing vertices (inf.cpp:359-364)
+            // (1) count pass over the existing vertices (inf.cpp:359-364); it
+            //     lists the vertices near the new line for (3) and finds the
+            //     float maximum of the squared distances of those that stay
+            //     for (7)
             const int nV0 = nV;
-            for (int i = lane; i < nV0; i += 32) {
-                const float4 v = IX(S.v4, i);
-                float r32, err;
-                if (nb.vert) {
-                    r32 = v.x - nb32;
-                    err = 3.0f * kU32 * (fabsf(v.x) + fabsf(nb32)) + 1e-37f;
-                } else {
-                    const float t = nab * fabsf(v.x);
-                    r32 = v.y - fmaf(na32, v.x, nb32);
-                    err = 5.0f * kU32 * (fabsf(v.y) + t + fabsf(nb32)) + 1e-37f;
+            int nOn = 0;
+            float m32 = 0.0f;
+            nCons = -1;   // the considered list must be rebuilt: its room is free
+            for (int i0 = 0; i0 < nV0; i0 += 32) {
+                const int i = i0 + lane;
+                bool on = false;
+                if (i < nV0) {
+                    const float4 v = IX(S.v4, i);
+                    float r32, err;
+                    if (nb.vert) {
+                        r32 = v.x - nb32;
+                        err = 3.0f * kU32 * (fabsf(v.x) + fabsf(nb32)) + 1e-37f;
+                    } else {
+                        const float t = nab * fabsf(v.x);
+                        r32 = v.y - fmaf(na32, v.x, nb32);
+                        err = 5.0f * kU32 * (fabsf(v.y) + t + fabsf(nb32)) + 1e-37f;
+                    }
+                    bool valid;
+                    if (r32 > err) valid = nb.valid == 1;
+                    else if (r32 < -err) valid = nb.valid == 0;
+                    else {
+                        const double2 p = IX(S.vd, i);
+                        valid = valid64k(nb.a, nb.b, nb.vert, nb.valid, p.x, p.y);
+                    }
+                    // near the new line: may coincide (within 1e-9) with one of its intersections
+                    const float tol = (1.0f + nab) * 1.2e-9f + err;
+                    on = fabsf(r32) <= tol || !(fabsf(r32) < FLT_MAX);
+                    const uint32_t nc = vcnt_of(v.w) + (valid ? 0u : 1u);
+                    IX(S.v4, i).w = vpack(nc, vfl_of(v.w));
+                    if (nc < ku) m32 = fmaxf(m32, v.z);
                 }
-                bool valid;
-                if (r32 > err) valid = nb.valid == 1;
-                else if (r32 < -err) valid = nb.valid == 0;
-                else {
-                    const double2 p = IX(S.vd, i);
-                    valid = valid64(nb.a, nb.b, nb.vert, nb.valid, p.x, p.y);
-                }
-                // near the new line: may coincide (within 1e-9) with one of its intersections
-                const float tol = (1.0f + nab) * 1.2e-9f + err;
-                uint32_t fl = vfl_of(v.w) & ~VB_ON;
-                if (fabsf(r32) <= tol || !(fabsf(r32) < FLT_MAX)) fl |= VB_ON;
-                IX(S.v4, i).w = vpack(vcnt_of(v.w) + (valid ? 0u : 1u), fl);
+                const unsigned mo = __ballot_sync(FULL, on);
+                if (on) IX(S.cons, nOn + __popc(mo & ((1u << lane) - 1))) = (uint16_t)i;
+                nOn += __popc(mo);
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m32 = fmaxf(m32, __shfl_xor_sync(FULL, m32, o));
             WSYNC();
 
             PHASE(3);
@@ -423,26 +483,27 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             //     right; inf.h:340-374) then every earlier bisector in order
             const int C = 4 + nL;
             // float interval of the new line's coefficients (directed rounding)
-            const float a1l = __double2float_rd(nb.a), a1h = __double2float_ru(nb.a);
-            const float b1l = __double2float_rd(nb.b), b1h = __double2float_ru(nb.b);
+            const float a1l = d2f_bits<-1>(nb.a), a1h = d2f_bits<1>(nb.a);
+            const float b1l = d2f_bits<-1>(nb.b), b1h = d2f_bits<1>(nb.b);
             for (int c = lane; c < C; c += 32) {
                 double x = 0, y = 0;
                 bool ok = false;
                 uint8_t cf = 0;
-                if (c < 4) {
-                    const double ea = 0, eb = (c == 0) ? sy0 : (c == 1) ? sy1 : (c == 2) ? sx0 : sx1;
-                    const int ev = c >= 2;
-                    if (intersect64(nb.a, nb.b, nb.vert, ea, eb, ev, x, y)) {
-                        ok = (c < 2) ? (x >= sx0 && x <= sx1) : (y >= sy0 && y <= sy1);
-                    }
+                // the other line: an edge of the space (c < 4) or a bisector
+                const bool edge = c < 4;
+                double2 e = make_double2(0.0, 0.0);
+                uint32_t lf = 0;
+                bool need64 = true;
+                if (edge) {
+                    e.y = (c == 0) ? sy0 : (c == 1) ? sy1 : (c == 2) ? sx0 : sx1;
+                    lf = c >= 2 ? LB_VERT : 0u;
                     cf = VB_BND;
-                    zs.cand += ok;
                 } else {
                     const int j = c - 4;
-                    const double2 e = IX(S.ld, j);
+                    e = IX(S.ld, j);
                     const float4 e4 = IX(S.l4, j);
-                    const int ev = (__float_as_uint(e4.w) & LB_VERT) ? 1 : 0;
-                    bool need64 = true;
+                    lf = __float_as_uint(e4.w);
+                    const int ev = (lf & LB_VERT) ? 1 : 0;
                     if (!nb.vert && !ev) {
                         // float interval of the intersection (directed rounding)
                         const float a2l = lo32(e4.x), a2h = hi32(e4.x);
@@ -496,15 +557,25 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                             }
                         }
                     }
-                    if (need64) {
-                        zs.cand64++;
-                        if (intersect64(nb.a, nb.b, nb.vert, e.x, e.y, ev, x, y))
-                            ok = x >= sx0 && x <= sx1 && y >= sy0 && y <= sy1;
-                    }
                     zs.cand++;
+                    zs.cand64 += need64;
+                }
+                if (need64 && intersect64(nb.a, nb.b, nb.vert, e.x, e.y, (lf & LB_VERT) ? 1 : 0, x, y)) {
+                    const long long xk = order_key(x), yk = order_key(y);
+                    const bool inx = xk >= kx0 && xk <= kx1, iny = yk >= ky0 && yk <= ky1;
+                    if (edge) {
+                        ok = c < 2 ? inx : iny;
+                        zs.cand += ok;
+                    } else {
+                        ok = inx && iny;
+                        // the generating bisector passes through the candidate:
+                        // its side is a rounding question, decided in FP64
+                        // (0x40: the invalid one) and counted by (4)
+                        if (ok && !valid64k(e.x, e.y, lf & LB_VERT, (lf & LB_VALID) ? 1 : 0, x, y)) cf = 0x40;
+                    }
                 }
                 IX(S.cd, c) = make_double2(x, y);
-                IX(S.c2, c) = make_float2((float)x, (float)y);
+                IX(S.c2, c) = make_float2(d2f_bits<0>(x), d2f_bits<0>(y));
                 IX(S.cfl, c) = ok ? (uint8_t)(cf | 0x80) : (uint8_t)0;
             }
             WSYNC();
@@ -513,17 +584,6 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             // (3) deduplicate (|dx| < 1e-9 and |dy| < 1e-9) against existing
             //     vertices near the new line and against earlier candidates
             {
-                // online vertices
-                int nOn = 0;
-                for (int i0 = 0; i0 < nV0; i0 += 32) {
-                    const int i = i0 + lane;
-                    const bool on = i < nV0 && (vfl_of(IX(S.v4, i).w) & VB_ON);
-                    const unsigned m = __ballot_sync(FULL, on);
-                    if (on) IX(S.cons, nOn + __popc(m & ((1u << lane) - 1))) = (uint16_t)i;   // cons reused as scratch
-                    nOn += __popc(m);
-                }
-                WSYNC();
-                nCons = -1;   // considered list must be rebuilt
                 if (nOn > 0) {
                     for (int c = lane; c < C; c += 32) {
                         if (!(IX(S.cfl, c) & 0x80)) continue;
@@ -534,7 +594,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                             const float4 v = IX(S.v4, i);
                             if (fabsf(v.x - c32.x) > tolE || fabsf(v.y - c32.y) > tolE) continue;
                             const double2 p = IX(S.vd, i), q = IX(S.cd, c);
-                            if (fabs(__dsub_rn(p.x, q.x)) < EPS && fabs(__dsub_rn(p.y, q.y)) < EPS) dup = true;
+                            if (within_eps(p.x, q.x) && within_eps(p.y, q.y)) dup = true;
                         }
                         if (dup) IX(S.cfl, c) &= 0x7f;
                     }
@@ -543,74 +603,92 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             }
 
             PHASE(5);
-            // (4) counts of the surviving candidates over earlier bisectors:
-            //     a float pass counts certain violations (and stops at k, which
-            //     erases the candidate anyway); bisectors it cannot decide are
-            //     evaluated in FP64 in a second pass
-            for (int c = lane; c < C; c += 32) {
-                int cnt = k;
-                if (IX(S.cfl, c) & 0x80) {
-                    const double2 p = IX(S.cd, c);
-                    const float2 c32 = IX(S.c2, c);
-                    const float KX = kU32 * fabsf(c32.x) * (1.0f + kU32) + 3.01f * kU32 * fabsf(c32.x);
-                    const float KY = kU32 * fabsf(c32.y) + 3.01f * kU32 * fabsf(c32.y) + 1e-37f;
-                    cnt = 0;
-                    // the bisector that generated this candidate passes through
-                    // it: its side is a rounding question, decided in FP64
-                    const int gen = c - 4;
-                    if (gen >= 0) {
-                        const double2 g = IX(S.ld, gen);
-                        const uint32_t lf = __float_as_uint(IX(S.l4, gen).w);
-                        cnt += !valid64(g.x, g.y, lf & LB_VERT, (lf & LB_VALID) ? 1 : 0, p.x, p.y);
-                    }
-                    int undec = 0;
-                    int m = 0;
-                    for (; m + 4 <= nL && cnt < k; m += 4) {
-                        const float4 q0 = IX(S.l4, m), q1 = IX(S.l4, m + 1);
-                        const float4 q2 = IX(S.l4, m + 2), q3 = IX(S.l4, m + 3);
+            // (4) counts of the live candidates over earlier bisectors.  They
+            //     are listed first (about 11 of 27 are live at k=10), and a
+            //     group of up to four lanes takes each: a float pass counts
+            //     certain violations, the bisectors it cannot decide are
+            //     evaluated in FP64.  (Counts past k only erase the candidate.)
+            // (4b) a kept candidate closer than 1e-9 to an earlier live one is
+            //     not added (the reference keeps the first): the float prefilter
+            //     runs beside the counts; any hit triggers the exact sequential
+            //     resolution over all candidates.
+            int nlive = 0;
+            for (int c0 = 0; c0 < C; c0 += 32) {
+                const int c = c0 + lane;
+                const bool lv = c < C && (IX(S.cfl, c) & 0x80);
+                const unsigned m = __ballot_sync(FULL, lv);
+                // the list: the low halves of ccnt; the counts: the high ones
+                if (lv) IX(S.ccnt, nlive + __popc(m & ((1u << lane) - 1))) = c;
+                nlive += __popc(m);
+            }
+            WSYNC();
+            bool anyclose = false;
+            const int G = nlive <= 8 ? 4 : nlive <= 16 ? 2 : 1;      // lanes a candidate
+            for (int u0 = 0; u0 < nlive; u0 += 32 / G) {
+                const int u = u0 + lane / G, gl = lane % G;
+                const bool live = u < nlive;
+                const int c = live ? IX(S.ccnt, u) & 0xffff : 0;
+                int cnt = 0, undec = 0;
+                double2 p = make_double2(0, 0);
+                float2 c32 = make_float2(0, 0);
+                float KX = 0, KY = 0;
+                const int gen = c - 4;
+                if (live) {
+                    p = IX(S.cd, c);
+                    c32 = IX(S.c2, c);
+                    KX = kU32 * fabsf(c32.x) * (1.0f + kU32) + 3.01f * kU32 * fabsf(c32.x);
+                    KY = kU32 * fabsf(c32.y) + 3.01f * kU32 * fabsf(c32.y) + 1e-37f;
+                    if (gen >= 0 && gl == 0) cnt += (IX(S.cfl, c) & 0x40) ? 1 : 0;
+                    int m = gl;
+                    for (; m + 3 * G < nL; m += 4 * G) {
+                        const float4 q0 = IX(S.l4, m), q1 = IX(S.l4, m + G);
+                        const float4 q2 = IX(S.l4, m + 2 * G), q3 = IX(S.l4, m + 3 * G);
                         const int s0 = (m == gen) ? -1 : side32(q0, c32.x, c32.y, KX, KY);
-                        const int s1 = (m + 1 == gen) ? -1 : side32(q1, c32.x, c32.y, KX, KY);
-                        const int s2 = (m + 2 == gen) ? -1 : side32(q2, c32.x, c32.y, KX, KY);
-                        const int s3 = (m + 3 == gen) ? -1 : side32(q3, c32.x, c32.y, KX, KY);
+                        const int s1 = (m + G == gen) ? -1 : side32(q1, c32.x, c32.y, KX, KY);
+                        const int s2 = (m + 2 * G == gen) ? -1 : side32(q2, c32.x, c32.y, KX, KY);
+                        const int s3 = (m + 3 * G == gen) ? -1 : side32(q3, c32.x, c32.y, KX, KY);
                         cnt += (s0 > 0) + (s1 > 0) + (s2 > 0) + (s3 > 0);
                         undec += (s0 == 0) + (s1 == 0) + (s2 == 0) + (s3 == 0);
                     }
-                    for (; m < nL && cnt < k; ++m) {
+                    for (; m < nL; m += G) {
                         const int sm = (m == gen) ? -1 : side32(IX(S.l4, m), c32.x, c32.y, KX, KY);
                         cnt += sm > 0;
                         undec += sm == 0;
                     }
-                    if (cnt < k && undec > 0) {
-                        for (int j = 0; j < nL && cnt < k; ++j) {
+                }
+                for (int o = 1; o < G; o <<= 1) {
+                    cnt += __shfl_xor_sync(FULL, cnt, o);
+                    undec += __shfl_xor_sync(FULL, undec, o);
+                }
+                const bool need = live && cnt < k && undec > 0;
+                if (__any_sync(FULL, need)) {
+                    int extra = 0;
+                    if (need) {
+                        for (int j = gl; j < nL; j += G) {
                             if (j == gen) continue;
                             const float4 q = IX(S.l4, j);
                             if (side32(q, c32.x, c32.y, KX, KY) != 0) continue;
                             const double2 g = IX(S.ld, j);
                             const uint32_t lf = __float_as_uint(q.w);
-                            cnt += !valid64(g.x, g.y, lf & LB_VERT, (lf & LB_VALID) ? 1 : 0, p.x, p.y);
+                            extra += !valid64k(g.x, g.y, lf & LB_VERT, (lf & LB_VALID) ? 1 : 0, p.x, p.y);
                         }
                     }
+                    for (int o = 1; o < G; o <<= 1) extra += __shfl_xor_sync(FULL, extra, o);
+                    cnt += extra;
                 }
-                IX(S.ccnt, c) = cnt;
-            }
-            WSYNC();
-            // (4b) a candidate closer than 1e-9 to an earlier one is not added
-            // (the reference keeps the first).  Only a kept candidate can change
-            // the vertex set, so the float prefilter runs for those; any hit
-            // triggers the exact sequential resolution over all candidates.
-            {
-                bool anyclose = false;
-                for (int c = lane; c < C; c += 32) {
-                    if (!(IX(S.cfl, c) & 0x80) || IX(S.ccnt, c) >= k) continue;
+                if (live && gl == 0) IX(S.ccnt, c) = (IX(S.ccnt, c) & 0xffff) | (min(cnt, 0x7fff) << 16);
+                WSYNC();
+                if (live && cnt < k) {
                     // doubles within 1e-9 give floats within 1e-9 + u(|x1|+|x2|)
-                    const float2 c32 = IX(S.c2, c);
                     const float tx = 3.0f * kU32 * fabsf(c32.x) + 2e-9f, ty = 3.0f * kU32 * fabsf(c32.y) + 2e-9f;
-                    for (int c2 = 0; c2 < c; ++c2) {
-                        if (!(IX(S.cfl, c2) & 0x80)) continue;
-                        const float2 o = IX(S.c2, c2);
-                        if (fabsf(o.x - c32.x) <= tx && fabsf(o.y - c32.y) <= ty) { anyclose = true; break; }
+                    for (int u2 = gl; u2 < u && !anyclose; u2 += G) {
+                        const float2 o = IX(S.c2, IX(S.ccnt, u2) & 0xffff);
+                        if (fabsf(o.x - c32.x) <= tx && fabsf(o.y - c32.y) <= ty) anyclose = true;
                     }
                 }
+            }
+            WSYNC();
+            {
                 if (__any_sync(FULL, anyclose)) {
                     if (lane == 0) {
                         for (int c = 0; c < C; ++c) {
@@ -619,7 +697,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                             for (int c2 = 0; c2 < c; ++c2) {
                                 if (!(IX(S.cfl, c2) & 0x80)) continue;
                                 const double2 o = IX(S.cd, c2);
-                                if (fabs(__dsub_rn(o.x, p.x)) < EPS && fabs(__dsub_rn(o.y, p.y)) < EPS) { IX(S.cfl, c) &= 0x7f; break; }
+                                if (within_eps(o.x, p.x) && within_eps(o.y, p.y)) { IX(S.cfl, c) &= 0x7f; break; }
                             }
                         }
                     }
@@ -629,6 +707,10 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
 
             // (5) erase old vertices with count >= k (order kept), then append
             //     the new vertices with count < k in candidate order
+            //     mx: this lane's candidates for (7), as bits: the FP64 value of
+            //     the old vertices whose float value is the float maximum
+            //     found by (1) (rounding is monotone), and of every new one
+            long long mx = 0;
             int w = 0;
             for (int i0 = 0; i0 < nV0; i0 += 32) {
                 const int i = i0 + lane;
@@ -644,9 +726,11 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                 WSYNC();
                 if (keep) {
                     const int o = w + __popc(m & ((1u << lane) - 1));
-                    v.w = vpack(vcnt_of(v.w), vfl_of(v.w) & ~VB_ON);
-                    IX(S.vd, o) = p;
-                    IX(S.v4, o) = v;
+                    if (v.z == m32) mx = max(mx, __double_as_longlong(d2_64(p.x, p.y, qx, qy)));
+                    if (o != i) {
+                        IX(S.vd, o) = p;
+                        IX(S.v4, o) = v;
+                    }
                 }
                 w += __popc(m);
                 WSYNC();
@@ -654,16 +738,20 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             int nnew = 0;
             for (int c0 = 0; c0 < C; c0 += 32) {
                 const int c = c0 + lane;
-                const bool keep = c < C && (IX(S.cfl, c) & 0x80) && IX(S.ccnt, c) < k;
+                const bool keep = c < C && (IX(S.cfl, c) & 0x80) && (IX(S.ccnt, c) >> 16) < k;
                 const unsigned m = __ballot_sync(FULL, keep);
                 const int o = w + nnew + __popc(m & ((1u << lane) - 1));
-                if (keep && o < VC) {
+                if (keep) {
                     const double2 p = IX(S.cd, c);
-                    const float2 c32 = IX(S.c2, c);
-                    IX(S.vd, o) = p;
-                    IX(S.v4, o) = make_float4(c32.x, c32.y, (float)d2_64(p.x, p.y, qx, qy),
-                                              vpack((uint32_t)IX(S.ccnt, c),
-                                                    (IX(S.cfl, c) & VB_BND) | edge_bits(p.x, p.y, sx0, sy0, sx1, sy1)));
+                    const double d2 = d2_64(p.x, p.y, qx, qy);
+                    mx = max(mx, __double_as_longlong(d2));
+                    if (o < VC) {
+                        const float2 c32 = IX(S.c2, c);
+                        uint32_t fl = 0;
+                        if (IX(S.cfl, c) & VB_BND) fl = VB_BND | edge_bits(p.x, p.y, sx0, sy0, sx1, sy1);   // read for boundary vertices only
+                        IX(S.vd, o) = p;
+                        IX(S.v4, o) = make_float4(c32.x, c32.y, d2f_bits<0>(d2), vpack((uint32_t)(IX(S.ccnt, c) >> 16), fl));
+                    }
                 }
                 nnew += __popc(m);
             }
@@ -679,7 +767,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                 double dl = nearb;
                 if (lane == 0) {
                     bool need = true;
-                    if (nearb < DBL_MAX) {
+                    if (nearf < INFINITY) {
                         float est, err;
                         if (nb.vert) {
                             est = fabsf(qf.x - nb32);
@@ -689,7 +777,8 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                             est = fabsf(fmaf(na32, qf.x, nb32 - qf.y)) / den;
                             err = 8.0f * kU32 * ((fabsf(na32 * qf.x) + fabsf(qf.y) + fabsf(nb32)) / den + est) + 1e-30f;
                         }
-                        if ((double)__fsub_rd(est, err) > nearb) need = false;   // NaN keeps need
+                        // (a float above nearb rounded up; NaN keeps need)
+                        if (__fsub_rd(est, err) > nearf) need = false;
                     }
                     if (need) {
                         const double d = line_dist64(qx, qy, nb.a, nb.b, nb.vert);
@@ -697,9 +786,10 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
                     }
                 }
                 dl = __shfl_sync(FULL, dl, 0);
-                if (dl != nearb) {
+                if (__double_as_longlong(dl) != __double_as_longlong(nearb)) {
                     nearb = dl;
-                    K2 = sqrt_cut(2.0 * nearb, true);
+                    nearf = d2f_bits<1>(dl);
+                    K2 = near_cut(dl);
                 }
             }
             if (lane == 0) {
@@ -712,29 +802,14 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             if (vover) flags |= QF_ZONE_V_OVERFLOW;
             if (nV > zs.vmax) zs.vmax = nV;
             WSYNC();
-            // (7) furthest remaining vertex (inf.cpp:445-451).  The float
-            //     squared distances are the FP64 ones rounded to nearest, a
-            //     monotone map: the FP64 maximum is among the vertices whose
-            //     float value is the float maximum.
-            {
-                float m32 = 0.0f;
-                for (int i = lane; i < nV; i += 32) m32 = fmaxf(m32, IX(S.v4, i).z);
+            // (7) furthest remaining vertex (inf.cpp:445-451), from (5)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) m32 = fmaxf(m32, __shfl_xor_sync(FULL, m32, o));
-                long long m = 0;
-                for (int i = lane; i < nV; i += 32)
-                    if (IX(S.v4, i).z == m32) {
-                        const double2 p = IX(S.vd, i);
-                        m = max(m, __double_as_longlong(d2_64(p.x, p.y, qx, qy)));
-                    }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
-                const double f = sqrt_rn64(__longlong_as_double(m));
-                if (f != far_) {
-                    far_ = f;
-                    K1 = sqrt_cut(2.0 * far_, false);
-                    ring_gate(ring, rmaxf, (double)A.gf.cs, slack, far_, ring_open, ring_key);
-                }
+            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, o));
+            if (mx != far2) {
+                far2 = mx;
+                K1 = far_cut(far2);
+                ring_T = ring_limit32(far2, slack_ru);
+                ring_gate32(ring, rmaxf, A.gf.cs, slack_ru, ring_T, ring_open, ring_key);
             }
             WSYNC();
             PHASE(6);

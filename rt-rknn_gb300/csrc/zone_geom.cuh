@@ -186,47 +186,13 @@ struct Arr {
 #define IX(a, i) (a).p[(i)]
 #endif
 
-// ---- priority queue (lane 0 only) ------------------------------------------
+// ---- priority queue ---------------------------------------------------------
 // Keys are squared distances (non-negative doubles), stored as their bit
 // patterns: for non-negative doubles the integer order is the numeric order,
 // so the heap needs no floating-point comparison.
 __device__ __forceinline__ bool pq_less(uint64_t k1, uint32_t c1, uint64_t k2, uint32_t c2)
 {
     return k1 < k2 || (k1 == k2 && c1 < c2);
-}
-
-__device__ __forceinline__ bool pq_push(uint64_t* K, uint32_t* C, int& n, int cap, uint64_t key, uint32_t code)
-{
-    if (n >= cap) return false;
-    int i = n++;
-    while (i > 0) {
-        int p = (i - 1) >> 1;
-        if (!pq_less(key, code, K[p], C[p])) break;
-        K[i] = K[p];
-        C[i] = C[p];
-        i = p;
-    }
-    K[i] = key;
-    C[i] = code;
-    return true;
-}
-
-__device__ __forceinline__ void pq_pop(uint64_t* K, uint32_t* C, int& n)
-{
-    uint64_t lk = K[n - 1];
-    uint32_t lc = C[n - 1];
-    --n;
-    int i = 0;
-    for (;;) {
-        int l = 2 * i + 1;
-        if (l >= n) break;
-        int c = (l + 1 < n && pq_less(K[l + 1], C[l + 1], K[l], C[l])) ? l + 1 : l;
-        if (!pq_less(K[c], C[c], lk, lc)) break;
-        K[i] = K[c];
-        C[i] = C[c];
-        i = c;
-    }
-    if (n > 0) { K[i] = lk; C[i] = lc; }
 }
 
 constexpr uint32_t KIND_POINT = 0x80000000u;
@@ -346,10 +312,12 @@ __device__ __forceinline__ Cut near_cut(double dl)
     return c;
 }
 
-// FP32 form of ring_gate (below), conservative: Lr rounded down and the
-// threshold T >= 2 far (1 + 1e-9) + slack rounded up, so a ring opens no
-// later than the FP64 gate opens it (an earlier expansion only puts cells in
-// the queue sooner; the order of the entries taken is the same).
+// Whether facility ring `ring` (cells at Chebyshev distance `ring` from q's
+// cell) may still hold entries that rule 1 keeps, and the squared lower bound
+// of its cells' distances to q, as key bits.  Conservative in float: Lr rounded
+// down and the threshold T >= 2 far (1 + 1e-9) + slack rounded up, so a ring
+// never opens too late (an earlier expansion only puts cells in the queue
+// sooner; the order of the entries taken is the same).
 __device__ __forceinline__ float ring_limit32(long long far2bits, float slack_ru)
 {
     const float f = __fmul_ru(__fsqrt_ru(d2f_bits<1>(__longlong_as_double(far2bits))), 1.0f + 0x1p-22f);
@@ -362,18 +330,6 @@ __device__ __forceinline__ void ring_gate32(int ring, int rmaxf, float cs, float
     if (!(Lr > 0.0f)) Lr = 0.0f;
     open = ring <= rmaxf && !(Lr > T_ru);
     key = (uint64_t)__double_as_longlong((double)__fmul_rd(Lr, Lr));
-}
-
-// Whether facility ring `ring` (cells at Chebyshev distance `ring` from q's
-// cell) may still hold entries that rule 1 keeps, and the squared lower
-// bound of its cells' distances to q, as key bits.
-__device__ __forceinline__ void ring_gate(int ring, int rmaxf, double cs, double slack, double far_,
-                                          bool& open, uint64_t& key)
-{
-    double Lr = ring == 0 ? 0.0 : (double)(ring - 1) * cs - slack;
-    if (!(Lr > 0.0)) Lr = 0.0;
-    open = ring <= rmaxf && !(Lr > 2.0 * far_ * (1.0 + 1e-9) + slack);
-    key = (uint64_t)__double_as_longlong(Lr * Lr);
 }
 
 // Float bounds of the double that rounded (to nearest) to v.
