@@ -66,13 +66,15 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
     // per-warp statistics (32-bit here, 64-bit in the totals)
     VCount vc = {};
     const int total = nl > 0 ? A.chunk_off[nl] : 0;
-    // Warp gw's first item is item gw; later items come from the counter,
+    // A warp's first item is its number, counted over the blocks first so that
+    // a small batch's items spread over all SMs (FP64, 1000 queries of about
+    // two items: 47 -> 43 us); later items come from the counter,
     // numbered after the nwarps taken that way, and only when items
     // outnumber warps.  (Thousands of warps taking even their first item
     // from one counter queue their atomics on one address for many
     // microseconds, and a small batch's few items wait behind them.)
     const int nwarps = gridDim.x * (blockDim.x >> 5);
-    int g = blockIdx.x * (blockDim.x >> 5) + w;
+    int g = w * gridDim.x + blockIdx.x;
     for (bool first = true;; first = false) {
         if (!first) {
             if (total <= nwarps) break;
@@ -190,12 +192,15 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
 
 // The verification kernel with 2, 4 or 8 users per lane per work item
 // (32 * UPT users per item), for either precision mode; blocks of up to 16
-// warps.
+// warps.  80 registers (24 warps an SM): FP64 needs the warps to issue beside
+// the FP64 pipe (street layout with 126 / 80 / 64 registers: 2.49 / 2.27 /
+// 2.25 ms; 1000 uniform queries: 41 / 43 / 45 us), FP32 with 64 spills more
+// (1.46 -> 1.54 ms).
 __global__ void __maxnreg__(80) verify_kernel(VerifyArgs a) { verify_body<4, false>(a); }
 __global__ void __maxnreg__(80) verify_kernel_u2(VerifyArgs a) { verify_body<2, false>(a); }
 __global__ void __launch_bounds__(512) verify_kernel_u8(VerifyArgs a) { verify_body<8, false>(a); }
-__global__ void __launch_bounds__(512) verify64_kernel(VerifyArgs a) { verify_body<4, true>(a); }
-__global__ void __launch_bounds__(512) verify64_kernel_u2(VerifyArgs a) { verify_body<2, true>(a); }
+__global__ void __maxnreg__(80) verify64_kernel(VerifyArgs a) { verify_body<4, true>(a); }
+__global__ void __maxnreg__(80) verify64_kernel_u2(VerifyArgs a) { verify_body<2, true>(a); }
 __global__ void __launch_bounds__(512) verify64_kernel_u8(VerifyArgs a) { verify_body<8, true>(a); }
 
 // One warp per listed survivor.  Lane r computes the facility range of

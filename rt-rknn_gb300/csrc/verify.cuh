@@ -74,10 +74,14 @@ __global__ void verify64_kernel(VerifyArgs a);      // FP64, 4 users per lane pe
 __global__ void verify64_kernel_u2(VerifyArgs a);   // 2
 __global__ void verify64_kernel_u8(VerifyArgs a);   // 8
 
-// Shared memory of one warp of a verification kernel: the box filter's 32
+// Shared memory of one warp of a verification kernel: the box filter's
 // staged half-planes (three doubles each at most), its masks, boxes and list
 // of half-plane indices; the segments; the slice bounds.
-constexpr int BOX_STAGE_BYTES = 32 * 3 * (int)sizeof(double);
+constexpr int BOX_STAGE = 34;          // staged entries: one that decides nothing, 32 half-planes, padding
+// FP32: half-planes a lane evaluates between two tests (street layout, ms: two
+// 1.55, three 1.53, four 1.52, six 1.56)
+constexpr int BOX_TRIP = 4;
+constexpr int BOX_STAGE_BYTES = BOX_STAGE * 3 * (int)sizeof(double);
 constexpr int BOX_MASK_BYTES = 4 * 32 * (int)sizeof(unsigned);
 constexpr int BOX_QBOX_BYTES = 4 * 2 * (int)sizeof(float4);
 __host__ __device__ __forceinline__ size_t verify_box_bytes(int stage_cap)

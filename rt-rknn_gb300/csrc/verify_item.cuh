@@ -6,6 +6,7 @@
 // verifies its own slot's users when their count is small.
 #pragma once
 #include "verify.cuh"
+#include <cfloat>
 #include <climits>
 
 namespace rknn {
@@ -329,10 +330,11 @@ __device__ __forceinline__ void item_users(const VerifyArgs& A, const QDesc& d, 
 // half-planes alone: every facility strictly nearer to it than q lies within
 // 2|u-q| <= rho of q, so it is a half-plane.  With no undecided half-plane
 // the certified count is the exact count.  (All half-planes must be staged
-// for this: 0 otherwise.)
+// for this: 0 otherwise.)  Finite even for an unbounded rho: a user so far
+// from q that lim overflows is counted.
 __device__ __forceinline__ float item_rho2(const QDesc& d, int nbs)
 {
-    return nbs == d.nb ? d.rho * d.rho * (1.0f - 1e-5f) : 0.0f;
+    return nbs == d.nb ? fminf(d.rho * d.rho * (1.0f - 1e-5f), FLT_MAX) : 0.0f;
 }
 
 // Stage 2 of an item of slot s: direct[t] users are results, surv[t] users

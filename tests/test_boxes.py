@@ -56,3 +56,24 @@ def test_items_of_several_parts(engine, sets, nq):
         for mode in ("fp32", "fp64"):
             for q, k, got in zip(qs, ks, idx.query_batch(qs, ks, mode)):
                 assert np.array_equal(got, want[(int(q), int(k))]), (int(q), int(k), mode)
+
+
+@pytest.mark.parametrize("tight", [0.0, 0.3, 0.9])
+def test_quarters(engine, tight):
+    """Users in clumps of eight, some of no extent, some wide: of a group's
+    quarters one, two or more stay open after the boxes."""
+    rng = np.random.default_rng(int(100 * tight) + 5)
+    nc, nf = 4_003, 300
+    centre = rng.random((nc, 1, 2)) * 1000
+    wide = np.where(rng.random((nc, 1, 1)) < tight, 0.0, rng.choice([0.5, 8.0, 40.0], size=(nc, 1, 1)))
+    uxy = (centre + wide * rng.standard_normal((nc, 8, 2))).reshape(-1, 2).astype(np.float32)
+    fxy = (rng.random((nf, 2)) * 1000).astype(np.float32)
+    ds = datagen.Dataset(fxy, uxy, np.arange(nf, dtype=np.int32), np.arange(nf, nf + 8 * nc, dtype=np.int32),
+                         rng.choice(nf, size=12, replace=False).astype(np.int64))
+    o = O.Oracle.of(ds)
+    with engine.Index.of(ds) as idx:
+        for k in (6, 17, 60):
+            want = [o.query(int(q), k) for q in ds.queries]
+            for mode in ("fp32", "fp64"):
+                for got, w in zip(idx.query_batch(ds.queries, k, mode), want):
+                    assert np.array_equal(got, w), (tight, k, mode)
