@@ -1121,9 +1121,16 @@ rknn_status build_grids(rknn_index* ix, float fac_per_cell, float usr_per_cell)
     CK(dalloc(ix->d_uxy, nu));
     CK(dalloc(ix->d_uid, nu));
     CK(dalloc(ix->d_ustart, ncu + 1));
-    CK(grid_sort(ix->d_fin, nullptr, (int)nf, ix->gf, ix->d_fxy, nullptr, ix->d_fidx, ix->d_fpos, ix->d_fstart, st));
+    // both sorts' scratch (from the stream-ordered pool, which gives its memory
+    // back at each wait, a build over 10 M users took 170 us more)
+    struct Scratch {
+        char* p = nullptr;
+        ~Scratch() { cudaFree(p); }
+    } ws;
+    CK(dalloc(ws.p, std::max(grid_sort_bytes((int)nf, ix->gf), grid_sort_bytes((int)nu, ix->gu))));
+    CK(grid_sort(ix->d_fin, nullptr, (int)nf, ix->gf, ws.p, ix->d_fxy, ix->d_fidx, ix->d_fpos, ix->d_fstart, st));
     CK(cell_mbrs(ix->d_fxy, ix->d_fstart, ix->gf, ix->d_fmbr, st));
-    CK(grid_sort(ix->d_uin, ix->d_uidin, (int)nu, ix->gu, ix->d_uxy, ix->d_uid, nullptr, nullptr, ix->d_ustart, st));
+    CK(grid_sort(ix->d_uin, ix->d_uidin, (int)nu, ix->gu, ws.p, ix->d_uxy, ix->d_uid, nullptr, ix->d_ustart, st));
     if (ix->order_est) {
         ix->h_fstart.resize(ncf + 1);
         ix->h_ustart.resize(ncu + 1);

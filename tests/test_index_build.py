@@ -3,6 +3,9 @@ points and ids given back by a snapshot."""
 import numpy as np
 import pytest
 
+import datagen
+import oracle as O
+
 pytestmark = pytest.mark.gpu
 
 
@@ -45,3 +48,23 @@ def test_snapshot_keeps_points_and_ids(engine, tmp_path, given):
     f, i, u, j = engine.snapshot_read(path)
     assert np.array_equal(f, fxy) and np.array_equal(u, uxy) and np.array_equal(j, want_uid)
     assert np.array_equal(i, fid if given else np.arange(513))
+
+
+@pytest.mark.parametrize("nu", [1, 255, 2047, 2048, 2049, 70_001])
+@pytest.mark.parametrize("per_cell", [1e9, 300.0, 4.0, 1e-6])
+def test_cells(engine, nu, per_cell):
+    """Sort passes (1 to 4 digits: one cell, and up to 8192 x 8192), tiles'
+    remainders, cells of many users and none: the answers are the oracle's."""
+    rng = np.random.default_rng(nu)
+    uxy = rng.uniform(0, 1000, size=(nu, 2))
+    uxy[: nu // 2] = np.round(uxy[: nu // 2] / 250) * 250       # half in crowded points
+    fxy = rng.uniform(0, 1000, size=(400, 2)).astype(np.float32)
+    fxy[:40] = fxy[0]                                           # coincident facilities
+    ds = datagen.Dataset(fxy, uxy.astype(np.float32), np.arange(400, dtype=np.int32),
+                         np.arange(400, 400 + nu, dtype=np.int32), np.arange(0, 400, 37).astype(np.int64))
+    o = O.Oracle.of(ds)
+    with engine.Index.of(ds, usr_per_cell=per_cell, fac_per_cell=min(per_cell, 1e3)) as idx:
+        for k in (1, 9):
+            want = [o.query(int(q), k) for q in ds.queries]
+            for got, w in zip(idx.query_batch(ds.queries, k, "fp32"), want):
+                assert np.array_equal(got, w), (nu, per_cell, k)
