@@ -760,32 +760,39 @@ finalize_twin_kernel(int* res_pool, const long long* cand_off, const int* reg_le
 }
 
 // ------------------------------------------------------- large result sets
-// Sorts one slot's n > 0 ids with a block: LSD radix, SORT_BITS bits a pass
-// over the bits in which the ids differ, in tiles of SORT_TILE ids.  In a pass
-// each thread takes SORT_PT ids at most (a warp's are consecutive runs of 32),
-// ranks them within its warp's digit counts by ballots, and the block's scan of
-// those counts places every id; a set of one tile ping-pongs between two
-// shared-memory buffers, a larger one between src and tmp in device memory,
-// its tiles in order after a histogram of the whole set.  The sorted ids go
-// to out on its 128-byte lines.
+// Sorts one slot's n > 0 ids with a block.  A set of one tile is sorted by
+// buckets in shared memory (sort_buckets).  Larger ones, and ids in narrow
+// groups: LSD radix, SORT_BITS bits a pass over the bits in which the ids
+// differ, in tiles of SORT_TILE ids; in a pass each thread takes SORT_PT ids at
+// most (a warp's are consecutive runs of 32), ranks them within its warp's digit
+// counts by ballots, and the block's scan of those counts places every id; a set
+// of one tile ping-pongs between two shared-memory buffers, a larger one between
+// src and tmp in device memory, its tiles in order after a histogram of the
+// whole set.  The sorted ids go to out on its 128-byte lines (ids written to
+// page-locked host memory from their buckets, out of line: 0.92 ms for 0.76).
 //
 // Why a block: a warp that sorts a set alone is a chain of dependent loads,
-// votes and shared-memory updates (67 rounds a pass at the street workload's
-// mean of 2,140 ids, 400 at its largest), and the last large set that starts
-// ends the batch.  Street workload, 16,384 sets, 35 M ids: finalize 1.42 ms
-// with a warp a set, 0.81 so (0.06 of it because the 140 MB go to page-locked
-// host memory).  Ranking bound: same-digit lanes from a match instruction
-// instead of a ballot a bit took 0.96 ms.
+// votes and shared-memory updates, and the last large set that starts ends the
+// batch.  Street workload, 16,384 sets, 35 M ids, finalize with a warp a set /
+// radix passes / buckets: 1.42 / 0.81 / 0.76 ms into page-locked host memory,
+// - / 0.78 / 0.47 into device memory.  The first is bound by the link to the
+// host (140 MB at 190 GB/s, as a copy of the same bytes: 0.74 ms), the second by
+// the block's barriers.
 namespace {
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int SORT_PT = SORT_TILE / SORT_THREADS;
 constexpr int SORT_DIGITS = 1 << SORT_BITS;
+constexpr int SORT_BUCKET_BITS = 12, SORT_BUCKETS = 1 << SORT_BUCKET_BITS, SORT_BUCKET_MAX = 32;
+static_assert(SORT_BUCKETS % SORT_THREADS == 0, "whole buckets a thread");
 static_assert(SORT_THREADS >= SORT_DIGITS && SORT_DIGITS % 32 == 0, "a thread a digit in the scans");
 static_assert(SORT_TILE % SORT_THREADS == 0 && SORT_TILE <= 65536, "whole rounds of ids, 16-bit counts");
 
 struct SortShared {
     unsigned key[2][SORT_TILE];
-    uint16_t cnt[SORT_WARPS][SORT_DIGITS];      // a warp's digit counts, then its first places
+    union {
+        uint16_t cnt[SORT_WARPS][SORT_DIGITS];  // a warp's digit counts, then its first places
+        unsigned bucket[SORT_BUCKETS];          // a bucket's count, then its first place
+    };
     unsigned base[SORT_DIGITS];                 // tiled sets: where a digit's next id goes
     unsigned place[SORT_DIGITS];                // where the tile's first id of a digit goes
     unsigned ws[SORT_WARPS], mn, mx;
@@ -813,18 +820,79 @@ __device__ __forceinline__ unsigned sort_scan(unsigned v, SortShared& sh)
     return b + x - v;
 }
 
+// Sorts a tile's ids into sh.key[0] by buckets: their range is cut into
+// SORT_BUCKETS equal parts, each id goes to its part (an atomic to count it and
+// one to place it, a scan between) and from there to its rank among the few in
+// that part.  False, with the ids untouched, when a part holds more than
+// SORT_BUCKET_MAX (ids in narrow groups): the digits' passes are left.
+__device__ __forceinline__ bool sort_buckets(SortShared& sh, const int* src, unsigned mn, int bits, int n)
+{
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    unsigned *at = sh.bucket, *key = sh.key[1];
+    const int shift = max(0, bits - SORT_BUCKET_BITS);
+    constexpr int PER = SORT_BUCKETS / SORT_THREADS;
+    for (int i = tid; i < SORT_BUCKETS; i += SORT_THREADS) at[i] = 0u;
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < n; i += SORT_THREADS) atomicAdd(&at[(okey(src[i]) - mn) >> shift], 1u);
+    __syncthreads();
+    unsigned c[PER], sum = 0u, top = 0u;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        c[j] = at[PER * tid + j];
+        sum += c[j];
+        top = max(top, c[j]);
+    }
+    if (__syncthreads_or(top > SORT_BUCKET_MAX)) return false;
+    unsigned x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sh.ws[w] = x;
+    __syncthreads();
+    x -= sum;
+#pragma unroll
+    for (int j = 0; j < SORT_WARPS; ++j) x += j < w ? sh.ws[j] : 0u;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        at[PER * tid + j] = x;
+        x += c[j];
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < n; i += SORT_THREADS) {
+        const unsigned k = okey(src[i]);
+        key[atomicAdd(&at[(k - mn) >> shift], 1u)] = k;
+    }
+    __syncthreads();
+    // at[b] is now the end of bucket b
+    for (int i = tid; i < n; i += SORT_THREADS) {
+        const unsigned k = key[i], b = (k - mn) >> shift;
+        const int i0 = b ? (int)at[b - 1] : 0, i1 = (int)at[b];
+        int r = i0;
+        for (int j = i0; j < i1; ++j) {
+            const unsigned o = key[j];
+            r += o < k || (o == k && j < i);
+        }
+        sh.key[0][r] = k;
+    }
+    __syncthreads();
+    return true;
+}
+
 __device__ __forceinline__ void sort_slot(SortShared& sh, const unsigned* src0, unsigned* tmp, unsigned* out, int n)
 {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     unsigned* src = (unsigned*)src0;
     const bool one = n <= SORT_TILE;
-    // keys with the ids' order, their range, and (one tile) their copy
+    // the range of the keys (unsigned, in the ids' order)
     unsigned mn = 0xffffffffu, mx = 0u;
     if (tid == 0) { sh.mn = 0xffffffffu; sh.mx = 0u; }
+#pragma unroll 4
     for (int i = tid; i < n; i += SORT_THREADS) {
         const unsigned k = okey((int)src[i]);
-        if (one) sh.key[0][i] = k;
-        else src[i] = k;
         mn = min(mn, k);
         mx = max(mx, k);
     }
@@ -835,7 +903,18 @@ __device__ __forceinline__ void sort_slot(SortShared& sh, const unsigned* src0, 
     __syncthreads();
     mn = sh.mn;
     const unsigned span = sh.mx - mn;
-    const int passes = span ? (32 - __clz((int)span) + SORT_BITS - 1) / SORT_BITS : 0;
+    const int bits = span ? 32 - __clz((int)span) : 0;
+    int passes = (bits + SORT_BITS - 1) / SORT_BITS;
+    if (one && span && sort_buckets(sh, (const int*)src, mn, bits, n)) {
+        passes = 0;
+    } else {
+        for (int i = tid; i < n; i += SORT_THREADS) {
+            const unsigned k = okey((int)src[i]);
+            if (one) sh.key[0][i] = k;
+            else src[i] = k;
+        }
+        __syncthreads();
+    }
     int cur = 0;                        // one tile: the buffer that holds the keys
     unsigned *a = src, *b = tmp;        // more: the arrays, a holding the keys
     for (int p = 0; p < passes; ++p) {

@@ -144,9 +144,10 @@ struct FinScan {
 // slots taken after each block's first).  Launched for batches whose largest k
 // gives SORT_MIN_MEAN results on average: below it large sets are few, and the
 // launch would cost more than their warps' sorts.
-// (finalize of the street workload, ms, threads / tile: 256 / 4096 0.84,
-// 256 / 8192 0.94, 512 / 4096 0.87, 512 / 8192 0.81, 1024 / 12288 1.03)
-constexpr int SORT_BITS = 8, SORT_THREADS = 512, SORT_TILE = 8192;
+// (finalize of the street workload, ms into host / device memory, by threads /
+// tile / blocks an SM: 1024 / 16384 / 1 0.756 / 0.471, 1024 / 12288 / 1 0.770 /
+// 0.485, 512 / 12288 / 2 0.770 / 0.405, 512 / 8192 / 2 0.793 / 0.489)
+constexpr int SORT_BITS = 8, SORT_THREADS = 1024, SORT_TILE = 16384;
 constexpr int SORT_MIN_MEAN = 1024;
 __global__ void sort_large_kernel(int* res_pool, const long long* cand_off, const int* reg_len, const int* res_count,
                                   const int* out_off, int* out, int* stage, long long out_cap, const int* list,

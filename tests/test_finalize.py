@@ -57,3 +57,23 @@ def test_regions_past_the_pool(nq):
             got, off = idx.query_batch_flat(np.zeros(nq, np.int32), 3, mode)
             assert np.array_equal(off, n * np.arange(nq + 1))
             assert np.array_equal(got.reshape(nq, n), np.tile(np.arange(n, dtype=np.int32), (nq, 1)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [513, 5000, 12_288, 16_384, 16_385])
+@pytest.mark.parametrize("kind", ["even", "groups", "equal", "pairs", "two ends"])
+def test_ids_in_groups(n, kind):
+    """Ids spread evenly, in narrow groups (a part of their range holds many),
+    all the same, each twice, and at both ends of the int32 range."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n, dtype=np.int64)
+    ids = {"even": i * 37 - 1000, "groups": (i // 200) * 1_000_003 + i % 200, "equal": np.full(n, -7, np.int64),
+           "pairs": (i // 2) * 101, "two ends": np.where(i % 2 == 0, -2**31 + i, 2**31 - 1 - i)}[kind]
+    ids = rng.permutation(ids).astype(np.int32)
+    qs = np.zeros(3, np.int32)
+    with _index(n, ids, 0) as idx:
+        for mode in ("fp32", "fp64"):
+            for _ in range(2):
+                got, off = idx.query_batch_flat(qs, 2, mode)
+                assert np.array_equal(off, n * np.arange(4))
+                assert np.array_equal(got, np.tile(np.sort(ids), 3))
