@@ -185,6 +185,7 @@ struct rknn_index {
     int* d_fidin = nullptr;     // facility ids as given, for snapshots (null: 0, 1, ...)
     float fac_per_cell = 2.0f, usr_per_cell = 8.0f;
     int vupt = VERIFY_UPT;         // verification: users per lane per work item
+    bool vupt_auto = true;         // (neither given nor tuned)
     int vwarps = VERIFY_WARPS;     // verification: warps per block
     int skip_coincident = 1;
     int zone_vertex_test = 0;   // see rknn_index_opts.zone_vertex_test
@@ -647,6 +648,13 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     // more warps (a lone FP64 query's evaluations are bound by one warp's
     // FP64 issue rate)
     if (nq <= 16 && b.vupt > 2) b.vupt = 2;
+    // and so does FP64 while items (a query has about 2 k users per facility
+    // of candidates) are fewer than warps: uniform k=10, calls of 100 / 500 /
+    // 1000 / 2000 queries 84 / 91 / 100 / 129 us with four users a lane, 73 / 82 /
+    // 95 / 126 with two; street layout, 500 queries of 2,700: 481 against 491
+    if (mode == MODE_FP64 && ix->vupt_auto &&
+        (double)nq * std::max(1.0, 2.0 * kmax * (double)ix->nu / (double)ix->nf / VERIFY_CHUNK) < 24.0 * ix->num_sms)
+        b.vupt = 2;
     // batches with more slots than the GPU has verification warps (3,648): a
     // warp takes up to four parts of a slot in turn and finds the slot, its
     // segments and half-planes once (verification of 16,384 queries, one part
@@ -1275,7 +1283,7 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
         return bail(fail(RKNN_ERR_ARG, "users_per_thread must be 2, 4 or 8"));
     if (o.verify_warps != 0 && o.verify_warps != 4 && o.verify_warps != 8 && o.verify_warps != 16)
         return bail(fail(RKNN_ERR_ARG, "verify_warps must be 4, 8 or 16"));
-    if (o.users_per_thread) ix->vupt = o.users_per_thread;
+    if (o.users_per_thread) { ix->vupt = o.users_per_thread; ix->vupt_auto = false; }
     if (o.verify_warps) ix->vwarps = o.verify_warps;
     cudaStream_t st = ix->stream;
     CKB(dalloc(ix->d_fin, nf));
@@ -2581,6 +2589,9 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
         s = build_grids(ix, r.fac_per_cell, r.usr_per_cell);
     }
     if (s != RKNN_OK) return s;
+    const bool auto0 = ix->vupt_auto;
+    bool shaped = false;            // a trial's shape is the best
+    ix->vupt_auto = false;
     for (int upt : upts)
         for (int vw : vws) {
             ix->vupt = upt;
@@ -2594,6 +2605,7 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
                 r.best_ms = ms;
                 r.users_per_thread = upt;
                 r.verify_warps = vw;
+                shaped = true;
             }
         }
     {
@@ -2602,6 +2614,7 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
     }
     if (s != RKNN_OK) return s;
     ix->vupt = r.users_per_thread;
+    ix->vupt_auto = auto0 && !shaped;
     ix->vwarps = r.verify_warps;
     ix->plan_cache.reset();
     *result = r;
