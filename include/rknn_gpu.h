@@ -96,7 +96,7 @@ typedef struct {
     int64_t bisectors;      /* influence-zone bisectors created */
     int64_t zone_vertices_max;
     int64_t zone_candidates;/* bisector intersections considered (slice filter:
-                               facilities offered to the slice heaps) */
+                               facilities offered to the slices' bounds) */
     int64_t zone_fp64;      /* intersections computed in double precision */
     int64_t candidates;     /* users tested against the half-planes */
     int64_t plane_evals;    /* (user, half-plane) evaluations, and (box of users, half-plane) ones */
@@ -110,7 +110,7 @@ typedef struct {
                                candidate intersections, dedup, counts/erase/append, epilogue.
                                The slice filter fills 0 facility stream, and within it 1
                                slice-bound offers, 3 ring stop tests, 4 cell ranges, 5 facility
-                               items (with 1); 2 user-cell ring scan, 7 half-planes and
+                               items (with 1); 2 user rows, 7 half-planes and
                                segments, 6 the verification of the query's users when
                                the filter does it (warp 0's share) */
     int64_t zone_points;    /* facilities taken from the zone search's queue */

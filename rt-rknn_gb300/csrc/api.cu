@@ -1,16 +1,18 @@
 // C ABI of the engine (include/rknn_gpu.h): index creation, single-query
 // and batched queries, device-resident batches, statistics.
 //
-// One query batch is five kernels on the index's stream, captured once per
+// One query batch is a few kernels on the index's stream, captured once per
 // batch shape into a CUDA graph and replayed:
-//   zone_kernel      one warp per query (persistent, queries in descending-k
-//                    order): influence zone, half-planes, candidate segments
-//   plan_kernel      candidate and work-item offsets
-//   verify_kernel    persistent warps over 128-user work items: half-plane
-//                    filter, exact recount, warp-aggregated result append
-//   scan_counts      result offsets
-//   finalize_kernel  one warp per query (the block for large sets): sort its
-//                    ids into the output
+//   slice_kernel / zone_kernel  the filter (persistent, queries in descending-k
+//                    order): half-planes, candidate segments; small FP32 batches
+//                    verify their users here
+//   plan_kernel      result regions and work-item offsets
+//   verify_kernel    persistent warps over work items of users: half-plane
+//                    tests, warp-aggregated result append, survivor list
+//   recount_kernel   exact count of the survivors
+//   scan_counts      result offsets (finalize's own work up to 4096 queries)
+//   finalize_kernel  one warp per query: sort its ids into the output
+//   sort_large       a block per large set, in batches that expect them
 #include "../../include/rknn_gpu.h"
 #include "index.cuh"
 #include "rknn_common.cuh"

@@ -1,4 +1,4 @@
-// Angular-slice filter: one warp per query, for large k.
+// Angular-slice filter: one or two warps per query.
 //
 // The influence zone of rknn-inf keeps every arrangement vertex below level
 // k (about 3.4 k^2 of them), which outgrows shared memory beyond k ~ 35.
@@ -12,7 +12,8 @@
 //     degrees): every point of P farther than that from q is strictly nearer
 //     to f than to q.  With unit directions e1, e2 at the slice's edges the
 //     arc is |f-q|^2 / (2 min((f-q).e1, (f-q).e2));
-//   * each lane keeps the k smallest arcs of its slice in a max-heap; the
+//   * each lane keeps the k smallest arcs of its slice (a sorted list of
+//     registers, beyond k = 32 a max-heap in shared memory); the
 //     k-th smallest, R(P), bounds the results: a user of P farther than R(P)
 //     from q has k facilities strictly nearer than q;
 //   * facilities stream in ring by ring from q's cell; a facility at
@@ -25,11 +26,10 @@
 // the user test, so the kept region contains every result.  The verification
 // kernel decides exactly; this filter only bounds its work.
 //
-// Outputs are those of the zone kernel: half-planes of the nearest
-// facilities (the first caps.lc streamed) for the verification's filter, and
-// the user-cell segments of the kept region (a ring scan over user cells; the
-// region {u : |u-q| <= R(slice of u)} is star-shaped around q, so a full ring
-// of pruned cells closes it).
+// Outputs are those of the zone kernel: half-planes of the facilities that can
+// decide a user (up to caps.lc, in ring order) for the verification's filter,
+// and the user segments of the kept region {u : |u-q| <= R(slice of u)}, a range
+// of cells for each user row.
 #include "rknn_common.cuh"
 #include "zone.cuh"
 #include "verify_item.cuh"
@@ -327,7 +327,7 @@ __device__ __forceinline__ void fuse_verify(const ZoneArgs& A, int s, const char
 // facilities are among the two lists' k smallest), computed identically in
 // both warps, and the stream's budget is read from a shared count between
 // the same barriers.  At the end warp 0 writes the half-planes while warp 1
-// scans the user cells.
+// finds the user rows.
 template <int KR, int NWQ>
 __device__ __forceinline__ void slice_body(const ZoneArgs& A)
 {

@@ -58,7 +58,7 @@ namespace {
 // tk/tc[0 .. m), m <= 32: from the end on, each old entry moves past the new
 // ones greater than it, 32 at a time, and each new one counts the old and new
 // ones greater than itself.  Entries beyond cap are not taken (*over is set).
-// Codes are unique, so the sequence of entries taken is a heap's.
+// Codes are unique, so the order of the entries does not depend on the merges.
 __device__ __forceinline__ void wq_merge(uint64_t* K, uint32_t* C, int& n, const uint64_t* tk, const uint32_t* tc,
                                          int m, int cap, bool& over)
 {
@@ -194,8 +194,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
         const float2 qf = A.fxy[GX(qpos, A.nf, 101)];
         const double qx = qf.x, qy = qf.y;
         const uint32_t ku = (uint32_t)k;
-        // Warp-uniform scalars live in registers (identical in every lane);
-        // lane 0 alone touches the heap and broadcasts what it changes.
+        // Warp-uniform scalars live in registers (identical in every lane).
         int nV = 4, nL = 0, nP = 0, nCons = -1, flags = 0;
         double nearb = DBL_MAX;
         float nearf = INFINITY;         // nearb rounded up
@@ -297,7 +296,7 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
             PHASE(1);
             // Rule 1 prunes this entry.  Every entry still queued has a key
             // >= this one, and every cell not yet expanded lies beyond the
-            // heap's top (the expansion loop above guarantees it), so rule 1
+            // queue's head (the expansion loop above guarantees it), so rule 1
             // prunes all of them as well and the zone is final: stop here
             // instead of draining the queue.
             bool r1;

@@ -11,8 +11,8 @@
 //     every thread at once (each entry's new place is its rank among the old
 //     entries plus its rank within the batch), and the queue's head is read
 //     by every thread, so a pop needs no broadcast.  Entries are ordered by
-//     (squared distance, code) as in the heap of zone.cu; codes are unique,
-//     so the pop sequence is the heap's;
+//     (squared distance, code) as in zone.cu; codes are unique, so both
+//     kernels take the same sequence;
 //   * the loops over vertices and candidates run over the block's threads
 //     (ordered compactions keep the reference's vertex order);
 //   * a candidate intersection's certified pre-discard and its count over the

@@ -189,7 +189,7 @@ struct Arr {
 // ---- priority queue ---------------------------------------------------------
 // Keys are squared distances (non-negative doubles), stored as their bit
 // patterns: for non-negative doubles the integer order is the numeric order,
-// so the heap needs no floating-point comparison.
+// so the queue needs no floating-point comparison.
 __device__ __forceinline__ bool pq_less(uint64_t k1, uint32_t c1, uint64_t k2, uint32_t c2)
 {
     return k1 < k2 || (k1 == k2 && c1 < c2);
