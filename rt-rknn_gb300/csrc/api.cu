@@ -102,6 +102,8 @@ constexpr int FUSE_CAND = 4096;
 // segments kept in shared memory for a slot's verification (slots with more
 // read them from L1)
 constexpr int SEG_STAGE_MAX = 130;
+// cells a side from which a facility grid can be sparse (zone_launch)
+constexpr int SPARSE_SIDE = 64;
 // most queries of a batch whose ids finalize also writes to page-locked staging
 constexpr int TWIN_MAX = 16;
 constexpr int ZB_VSTATS_INTS = 32;  // room for the statistics after them
@@ -188,6 +190,8 @@ struct rknn_index {
     float fac_per_cell = 2.0f, usr_per_cell = 8.0f;
     int vupt = VERIFY_UPT;         // verification: users per lane per work item
     bool vupt_auto = true;         // (neither given nor tuned)
+    bool sparse = false;           // a large facility grid with under half the cells filled that uniform
+                                   // points would fill
     int vwarps = VERIFY_WARPS;     // verification: warps per block
     int skip_coincident = 1;
     int zone_vertex_test = 0;   // see rknn_index_opts.zone_vertex_test
@@ -372,11 +376,17 @@ ZoneLaunch zone_launch(rknn_index* ix, const ZoneCaps& c, int nq, bool slice = f
     if (kr > 0) {
         // two warps per query (shorter chains) when every query of the class
         // keeps a block resident; one warp each otherwise (more queries in
-        // flight)
+        // flight), and on a sparse facility grid, where far rings are taken by
+        // blocks of cells, which the two-warp kernels do not do (clustered
+        // layout, 17 % of the cells filled, calls of 10 / 100 / 500 / 1000
+        // queries: 613 / 839 / 1097 / 1555 us with two warps, 342 / 233 / 844 /
+        // 722 with one; uniform and street layouts, 85 % filled: up to 10 %
+        // slower with one, as are clustered ones on 32 cells a side, whose far
+        // rings are few; on 50 both take the same)
         size_t smem2 = slice_own_bytes(L.slice, 2, kr);
         if (fuse) smem2 = fuse_layout(smem2, fuse_sc, fuse_ss).bytes;
         const int per2 = occupancy(ix, (const void*)slice_fn(kmax, true), 64, smem2);
-        if ((long long)nq <= (long long)per2 * ix->num_sms) {
+        if (!ix->sparse && (long long)nq <= (long long)per2 * ix->num_sms) {
             L.smem = smem2;
             L.threads = 64;
             L.grid = std::max(1, nq);
@@ -1137,9 +1147,13 @@ rknn_status build_grids(rknn_index* ix, float fac_per_cell, float usr_per_cell)
         char* p = nullptr;
         ~Scratch() { cudaFree(p); }
     } ws;
-    CK(dalloc(ws.p, std::max(grid_sort_bytes((int)nf, ix->gf), grid_sort_bytes((int)nu, ix->gu))));
+    const size_t sort_bytes = std::max(grid_sort_bytes((int)nf, ix->gf), grid_sort_bytes((int)nu, ix->gu));
+    CK(dalloc(ws.p, sort_bytes + sizeof(int)));
+    int* d_filled = (int*)(ws.p + sort_bytes);
+    int filled = 0;
     CK(grid_sort(ix->d_fin, nullptr, (int)nf, ix->gf, ws.p, ix->d_fxy, ix->d_fidx, ix->d_fpos, ix->d_fstart, st));
-    CK(cell_mbrs(ix->d_fxy, ix->d_fstart, ix->gf, ix->d_fmbr, st));
+    CK(cell_mbrs(ix->d_fxy, ix->d_fstart, ix->gf, ix->d_fmbr, d_filled, st));
+    CK(cudaMemcpyAsync(&filled, d_filled, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(grid_sort(ix->d_uin, ix->d_uidin, (int)nu, ix->gu, ws.p, ix->d_uxy, ix->d_uid, nullptr, ix->d_ustart, st));
     if (ix->order_est) {
         ix->h_fstart.resize(ncf + 1);
@@ -1148,6 +1162,8 @@ rknn_status build_grids(rknn_index* ix, float fac_per_cell, float usr_per_cell)
         CK(cudaMemcpyAsync(ix->h_ustart.data(), ix->d_ustart, sizeof(int) * (ncu + 1), cudaMemcpyDeviceToHost, st));
     }
     CK(cudaStreamSynchronize(st));
+    ix->sparse = std::max(ix->gf.gx, ix->gf.gy) >= SPARSE_SIDE &&
+                 filled < 0.5 * (double)ncf * (1.0 - std::exp(-(double)nf / (double)ncf));
     return RKNN_OK;
 }
 

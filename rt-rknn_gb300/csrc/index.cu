@@ -228,9 +228,12 @@ __global__ void __launch_bounds__(ST_THREADS) k_starts(const float2* xy, int n, 
     }
 }
 
-__global__ void k_mbr(const float2* xy, const int* start, int nc, float4* mbr)
+// Box of each cell's points; *filled counts the cells that have any.
+__global__ void k_mbr(const float2* xy, const int* start, int nc, float4* mbr, int* filled)
 {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = __syncthreads_count(c < nc && start[c + 1] > start[c]);
+    if (threadIdx.x == 0 && n) atomicAdd(filled, n);
     if (c >= nc) return;
     float4 r = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
     for (int i = start[c]; i < start[c + 1]; ++i) {
@@ -362,10 +365,12 @@ cudaError_t grid_sort(const float2* d_xy, const int* d_ids, int n, const Grid& g
     return cudaGetLastError();
 }
 
-cudaError_t cell_mbrs(const float2* xy_s, const int* start, const Grid& g, float4* mbr, cudaStream_t st)
+cudaError_t cell_mbrs(const float2* xy_s, const int* start, const Grid& g, float4* mbr, int* filled, cudaStream_t st)
 {
     int nc = g.gx * g.gy;
-    k_mbr<<<nblk(nc, 256), 256, 0, st>>>(xy_s, start, nc, mbr);
+    const cudaError_t e = cudaMemsetAsync(filled, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    k_mbr<<<nblk(nc, 256), 256, 0, st>>>(xy_s, start, nc, mbr, filled);
     return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@ size_t grid_sort_bytes(int n, const Grid& g);
 cudaError_t grid_sort(const float2* d_xy, const int* d_ids, int n, const Grid& g, char* ws,
                       float2* xy_s, int* ids_s, int* pos_of, int* start, cudaStream_t st);
 
-cudaError_t cell_mbrs(const float2* xy_s, const int* start, const Grid& g, float4* mbr, cudaStream_t st);
+// Boxes of the cells' points, and (*filled, on the device) how many cells have any.
+cudaError_t cell_mbrs(const float2* xy_s, const int* start, const Grid& g, float4* mbr, int* filled, cudaStream_t st);
 
 }  // namespace rknn

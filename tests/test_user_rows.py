@@ -47,3 +47,25 @@ def test_regions_match_oracle(engine, layout):
             if layout != "corner":
                 for got, w in zip(idx.query_batch(big, k, "fp32"), want * (big.size // qs.size)):
                     assert np.array_equal(got, w), (layout, k)
+
+
+@pytest.mark.parametrize("spread", [0.2, 3.0, 14.0, 25.0, 300.0])
+def test_clustered_facilities(engine, spread):
+    """Facility grids from nearly empty to uniformly filled: small batches take
+    one warp a query below half the uniform filling, two above."""
+    rng = np.random.default_rng(int(10 * spread))
+    centre = rng.uniform(0, 1000, (60, 2))
+    f = centre[rng.integers(60, size=12_000)] + spread * rng.standard_normal((12_000, 2))
+    u = np.concatenate([centre[rng.integers(60, size=30_000)] + 2 * spread * rng.standard_normal((30_000, 2)),
+                        rng.uniform(0, 1000, (10_000, 2))])
+    f, u = f.astype(np.float32), u.astype(np.float32)
+    ds = datagen.Dataset(f, u, np.arange(12_000, dtype=np.int32), np.arange(12_000, 52_000, dtype=np.int32))
+    o = O.Oracle.of(ds)
+    qs = np.arange(0, 12_000, 299, dtype=np.int32)
+    with engine.Index.of(ds) as idx:
+        for k in (1, 10, 31):
+            want = [o.query(int(q), k) for q in qs]
+            for mode in ("fp32", "fp64"):
+                for n in (1, qs.size):
+                    for got, w in zip(idx.query_batch(qs[:n], k, mode), want):
+                        assert np.array_equal(got, w), (spread, k, mode, n)
