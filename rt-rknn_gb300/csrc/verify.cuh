@@ -8,7 +8,11 @@ constexpr int VERIFY_UPT = 4;                       // default users per lane pe
 constexpr int VERIFY_CHUNK = 32 * VERIFY_UPT;       // default users per work item
 constexpr int VERIFY_WARPS = 8;                     // default warps per block
 constexpr int VERIFY_SAMPLES = 1024;                // work-item offsets cached per block
-constexpr int BOX_MIN_CAND = 512;                   // FP32: candidates from which boxes come first
+// FP32: candidates from which boxes come first (verification, ms, with the line
+// at 384 / 512 / 768: uniform 16,384 queries of 400 candidates 0.395 / 0.277 /
+// 0.254, of 640 - / 0.682 / 0.526; street layout - / 1.482 / 1.497; calls of the
+// street and clustered layouts with k to 100 and of k=25 1-2 % slower at 768)
+constexpr int BOX_MIN_CAND = 512;
 // Most queries of an influence-zone batch, and candidates of a query, that go
 // to the recount without a half-plane test.  The zone's half-planes reject
 // about half of the candidates and accept none (its pruning may have dropped a

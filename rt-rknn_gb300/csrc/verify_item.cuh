@@ -177,10 +177,35 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
     sweep((const float4*)sp, ns);
     if constexpr (COMPACT)
         if (!stopped && ns < nb) sweep(gp, nb);
-#pragma unroll
-    for (int t = 0; t < UPT; ++t)
-        und[t] = rmin[t] <= __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f))) || lim[t] > rho2;
     evals += (unsigned)(m * nvalid);
+    bool again = false;
+#pragma unroll
+    for (int t = 0; t < UPT; ++t) {
+        und[t] = rmin[t] <= __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
+        again |= und[t] && cnt[t] < k && !(lim[t] > rho2);
+    }
+    if constexpr (COMPACT)
+        if (__any_sync(FULL, again)) {
+            // some are too close to call for a user that they would leave a
+            // result: count them; below k with all of them it is one (ties on
+            // bisectors; clustered layout, 2000 queries: recount 142 -> 45 us,
+            // the call 897 -> 793)
+            int nc[UPT];
+#pragma unroll
+            for (int t = 0; t < UPT; ++t) nc[t] = 0;
+#pragma unroll 1
+            for (int i = 0; i < m; ++i) {
+                const float4 p = i < ns ? ((const float4*)sp)[i] : gp[i];
+#pragma unroll
+                for (int t = 0; t < UPT; ++t)
+                    nc[t] += __float_as_uint(fmaf(p.x, x[t], fmaf(p.y, y[t], p.z)) + bu[t]) <=
+                             __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
+            }
+#pragma unroll
+            for (int t = 0; t < UPT; ++t) und[t] = und[t] && cnt[t] + nc[t] >= k;
+        }
+#pragma unroll
+    for (int t = 0; t < UPT; ++t) und[t] |= lim[t] > rho2;
 }
 
 // Exclusive block-wide prefix sum; *total receives the block's sum.
