@@ -65,6 +65,11 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
     return cnt;
 }
 
+// A float evaluation bound 8u (2F'(X + Y) + F'^2) below this keeps the sum in
+// parentheses, and with it every intermediate of m(u) in float, below 2.2e37.
+// From it on m(u) may overflow on the way to a small value.
+constexpr float BOUND_MAX = 1e31f;
+
 // Above 4|u - q|^2 with margin, for the user at offset (x, y) from q.
 __device__ __forceinline__ float user_lim(float x, float y)
 {
