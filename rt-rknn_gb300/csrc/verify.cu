@@ -234,7 +234,7 @@ __device__ __forceinline__ int group_exact_count(const Counted& d, const VerifyA
     // the disc's radius, above |u - q|
     const float ddx = ux - qx, ddy = uy - qy;
     const float Dq = fmaf(ddx, ddx, ddy * ddy);
-    const float r = sqrtf(Dq) * (1.0f + 4e-6f) + slack;
+    const float r = disc_radius(Dq, slack);
     Near64 near;
     if (F64) near = near64(ux, uy, qx, qy);
     if (G > 1) {
@@ -252,7 +252,8 @@ __device__ __forceinline__ int group_exact_count(const Counted& d, const VerifyA
         if (cy <= cy1) {
             const float ylo = g.y0 + (float)cy * g.cs - ym, yhi = g.y0 + (float)(cy + 1) * g.cs + ym;
             const float dyn = fmaxf(fmaxf(ylo - uy, uy - yhi), 0.0f) * (1.0f - 1e-6f);
-            const float w = sqrtf(fmaxf(fmaf(r, r, -dyn * dyn), 0.0f)) * (1.0f + 1e-6f) + slack;
+            // (r^2 - dyn^2 as a product: the squares overflow from 1.8e19 on)
+            const float w = sqrtf(fmaxf((r - dyn) * (r + dyn), MIN_SQUARE)) * (1.0f + 1e-6f) + slack;
             const int cx0 = cell_coord(ux - w, g.x0, g.inv, g.gx), cx1 = cell_coord(ux + w, g.x0, g.inv, g.gx);
             f0 = A.fstart[VX(cy * g.gx + cx0, A.ncf + 1, 211)];
             len = A.fstart[VX(cy * g.gx + cx1 + 1, A.ncf + 1, 212)] - f0;

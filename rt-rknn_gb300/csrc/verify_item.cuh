@@ -30,6 +30,16 @@ __device__ __forceinline__ long long vck(const VerifyArgs& A, long long i, long 
 #define VX(i, n, id) (i)
 #endif
 
+// Squares below this are rounded as subnormals, with errors beyond any relative
+// margin: an upper bound of a root takes it in their place.
+constexpr float MIN_SQUARE = 1e-36f;
+
+// Above |u - q|, from its float square (infinite where that overflowed).
+__device__ __forceinline__ float disc_radius(float Dq, float slack)
+{
+    return sqrtf(fmaxf(Dq, MIN_SQUARE)) * (1.0f + 4e-6f) + slack;
+}
+
 template <typename T>
 __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, const VerifyArgs& A,
                                            unsigned long long& fac, unsigned long long& rech)
@@ -40,7 +50,7 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
     // the radius of the cells looked at, above |u - q|
     const float ddx = ux - qx, ddy = uy - qy;
     const float Dq = fmaf(ddx, ddx, ddy * ddy);
-    const float r = sqrtf(Dq) * (1.0f + 4e-6f) + slack;
+    const float r = disc_radius(Dq, slack);
     Near64 near;
     if (sizeof(T) == 8) near = near64(ux, uy, qx, qy);
     const Grid& g = A.gf;
