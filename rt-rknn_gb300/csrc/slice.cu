@@ -68,7 +68,7 @@ __device__ __forceinline__ float upper_arc(float vx, float vy, float e1x, float 
     const float l1 = fabsf(vx) + fabsf(vy);
     const float dmin = fminf(d1, d2) - 8.0f * kU32 * l1 - 1e-37f;
     if (!(dmin > 0.0f)) return INFINITY;
-    const float num = fmaf(vx, vx, vy * vy) * (1.0f + 8.0f * kU32);
+    const float num = fmaf(vx, vx, fmaf(vy, vy, vitem::SQUARE_ERR)) * (1.0f + 8.0f * kU32);
     const float den = 2.0f * dmin;
     // __fdividef is within 2 ulp for denominators in [2^-126, 2^126]: a
     // 2^-20 relative inflation covers it; outside that range divide exactly
@@ -87,7 +87,7 @@ __device__ __forceinline__ float upper_arc_fast(float vx, float vy, float e1x, f
     const float d1 = fmaf(vx, e1x, vy * e1y), d2 = fmaf(vx, e2x, vy * e2y);
     const float l1 = fabsf(vx) + fabsf(vy);
     const float dmin = fminf(d1, d2) - 8.0f * kU32 * l1 - 1e-37f;
-    const float num = fmaf(vx, vx, vy * vy);
+    const float num = fmaf(vx, vx, fmaf(vy, vy, vitem::SQUARE_ERR));
     // num (1 + 8u) / (2 dmin), the quotient rounded up by 2^-20
     constexpr float C = 0.5f * (1.0f + 8.0f * kU32) * (1.0f + 0x1p-20f) * (1.0f + 4.0f * kU32);
     return (dmin > 0x1p-100f && dmin < 0x1p100f) ? __fdividef(num, dmin) * C : INFINITY;
@@ -128,21 +128,24 @@ __device__ __forceinline__ float box_bound(float X0, float X1, float Y0, float Y
     return r;
 }
 
+// Whether an offset (vx, vy) lies beyond twice a reach or need r.  |v|^2 / 4 is
+// made from quartered factors, rounded down: it overflows only where r^2 does
+// or |v| > 2r, and then an infinite r^2 is not exceeded.  What underflows on the
+// left is below SQUARE_ERR on the right (0 >= 0 dropped facilities that decide
+// users where offsets are below about 1e-23).
+__device__ __forceinline__ bool beyond(float vx, float vy, float r)
+{
+    constexpr float C = 0.25f * (1.0f - 8.0f * kU32);
+    return fmaf(C * vx, vx, (C * vy) * vy) > fmaf(r, r, vitem::SQUARE_ERR);
+}
+
 // Whether every facility in a box (relative to q, not around it) lies beyond
 // twice the need of its slice (Ns: the slices' need).
 __device__ __forceinline__ bool box_idle(float X0, float X1, float Y0, float Y1, const float* Ns)
 {
     const float dx = fmaxf(fmaxf(X0, -X1), 0.0f), dy = fmaxf(fmaxf(Y0, -Y1), 0.0f);
-    const float L2 = fmaf(dx, dx, dy * dy) * (1.0f - 4e-6f);     // |box - q|^2, rounded down
     const float R = box_bound(X0, X1, Y0, Y1, Ns);
-    return R < INFINITY && 0.25f * L2 > R * R * (1.0f + 4e-6f);
-}
-
-// Whether a facility at offset (vx, vy), |v|^2 = d2, lies beyond twice a reach
-// or need.
-__device__ __forceinline__ bool beyond(float d2, float r)
-{
-    return 0.25f * d2 * (1.0f - 4.0f * kU32) >= r * r;
+    return beyond(dx * (1.0f - 2e-6f), dy * (1.0f - 2e-6f), R * (1.0f + 2e-6f));
 }
 
 // Cell ri of the square ring at Chebyshev distance ring around (qcx, qcy):
@@ -258,7 +261,7 @@ __device__ __forceinline__ int trim_planes(const float2* fxy, int nf, int* lpos,
             dx = f.x - q.x;
             dy = f.y - q.y;
         }
-        const bool keep = m < n && !beyond(fmaf(dx, dx, dy * dy), Ns[slice_of(dx, dy)]);
+        const bool keep = m < n && !beyond(dx, dy, Ns[slice_of(dx, dy)]);
         const unsigned km = __ballot_sync(FULL, keep);          // (every lane has read its entry)
         if (keep) lpos[k + __popc(km & ((1u << lane) - 1))] = pos;
         k += __popc(km);
@@ -454,7 +457,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 // inside the cone (or near its edges: then the corner only raises the bound)
                 const float c1 = e1x * dy - e1y * dx, c2 = dx * e2y - dy * e2x;
                 const float tol = 1e-5f * (fabsf(dx) + fabsf(dy));
-                if (c1 >= -tol && c2 >= -tol) clip = fmaxf(clip, sqrtf(fmaf(dx, dx, dy * dy)));
+                if (c1 >= -tol && c2 >= -tol) clip = fmaxf(clip, sqrtf(fmaf(dx, dx, fmaf(dy, dy, vitem::SQUARE_ERR))));
             }
             clip = clip * (1.0f + 1e-5f) + 1e-30f;
         }
@@ -596,9 +599,8 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 }
                 const int sj = slice_of(vx, vy);
                 const float rj = Rs[sj], nj = Ns[sj];
-                const float d2 = fmaf(vx, vx, vy * vy);
-                const bool hp = ok && !beyond(d2, nj);
-                unsigned m = __ballot_sync(FULL, ok && !beyond(d2, rj));
+                const bool hp = ok && !beyond(vx, vy, nj);
+                unsigned m = __ballot_sync(FULL, ok && !beyond(vx, vy, rj));
                 // half-planes: the first LC of them, in ring order
                 const unsigned pm = __ballot_sync(FULL, hp);
                 int at0 = nL;       // this batch's first half-plane slot
@@ -821,7 +823,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 dy = f.y - qf.y;
             }
             const float c = fmaf(dx, dx, dy * dy);
-            const bool keep = m < nL && !beyond(c, Ns[slice_of(dx, dy)]);
+            const bool keep = m < nL && !beyond(dx, dy, Ns[slice_of(dx, dy)]);
             const unsigned km = __ballot_sync(FULL, keep);      // (every lane has read its entry)
             if (keep) {
                 const int o = nk + __popc(km & ((1u << lane) - 1));
@@ -864,7 +866,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         }
         // in float, rounded up (the constants carry a 2e-6 margin over their
         // own rounding); an overflow to +inf only makes every test undecided
-        const float Fp = __fadd_ru(__fmul_ru(__fsqrt_ru(__fmul_ru(cmax, 1.0f + 1e-5f)), 1.0f + 1e-6f), 1e-30f);
+        const float Fp = __fadd_ru(__fmul_ru(__fsqrt_ru(__fmaf_ru(cmax, 1.0f + 1e-5f, vitem::SQUARE_ERR)), 1.0f + 1e-6f), 1e-30f);
         const float Fp2 = __fmul_ru(Fp, Fp);
         k2f = __fmul_ru(Fp, 16.0f * kU32 * (1.0f + 2e-6f));
         kf2 = __fadd_ru(__fmul_ru(Fp2, 8.0f * kU32 * (1.0f + 2e-6f)), 1e-30f);
@@ -932,7 +934,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                     const float lo = fmaxf(ypos ? Y0 : -Y1, 0.0f), hi = fminf(ypos ? Y1 : -Y0, Ymax);
                     if (lo > hi) continue;
                     const float xa = lo * cotB;
-                    const float xc = sqrtf((R - lo) * (R + lo)) * (1.0f + 1e-6f);   // (lo <= hi <= R)
+                    const float xc = sqrtf(fmaf(R - lo, R + lo, vitem::SQUARE_ERR)) * (1.0f + 1e-6f);   // (lo <= hi <= R)
                     const float xb = fminf(fminf(hi * cotA, Xmax), xc);     // (0 times infinity: xb from the others)
                     const int c0 = cell_coord(xpos ? qf.x + xa - delta : qf.x - xb - delta, gu.x0, gu.inv, gu.gx);
                     const int c1 = cell_coord(xpos ? qf.x + xb + delta : qf.x - xa + delta, gu.x0, gu.inv, gu.gx);

@@ -34,6 +34,10 @@ __device__ __forceinline__ long long vck(const VerifyArgs& A, long long i, long 
 // margin: an upper bound of a root takes it in their place.
 constexpr float MIN_SQUARE = 1e-36f;
 
+// Above the error of a sum of two such squares, and lost in any sum of larger
+// ones: added to a square that has to be an upper bound.
+constexpr float SQUARE_ERR = 0x1p-125f;
+
 // Above |u - q|, from its float square (infinite where that overflowed).
 __device__ __forceinline__ float disc_radius(float Dq, float slack)
 {
@@ -361,7 +365,7 @@ __device__ __forceinline__ void item_users(const VerifyArgs& A, const QDesc& d, 
             if (!valid[t]) continue;
             const float dx = u[t].x - d.qx, dy = u[t].y - d.qy;
             const float Rs = Rq[slice_of(dx, dy)];
-            if (fmaf(dx, dx, dy * dy) * (1.0f - 1e-6f) > Rs * Rs) valid[t] = false;
+            if (fmaf(dx, dx, dy * dy) * (1.0f - 1e-6f) > fmaf(Rs, Rs, SQUARE_ERR)) valid[t] = false;
         }
     }
 }

@@ -32,13 +32,13 @@ def _points(layout):
     exact and changes no result: the unscaled set is the oracle's."""
     rng = np.random.default_rng(3)
     if layout == "far":                     # users around few facilities, up to three times as far out
-        f, u = 1.3 * rng.random((30, 2)) - 0.65, 3.2 * rng.random((20_000, 2)) - 1.6
+        f, u = 1.3 * rng.random((30, 2)) - 0.65, 3.2 * rng.random((3000, 2)) - 1.6
     elif layout == "clustered":
         c = rng.random((20, 2))
-        f = c[rng.integers(20, size=6000)] + 0.01 * rng.standard_normal((6000, 2))
-        u = c[rng.integers(20, size=20_000)] + 0.02 * rng.standard_normal((20_000, 2))
+        f = c[rng.integers(20, size=1500)] + 0.01 * rng.standard_normal((1500, 2))
+        u = c[rng.integers(20, size=3000)] + 0.02 * rng.standard_normal((3000, 2))
     else:
-        f, u = rng.random((2000, 2)) - 0.5, rng.random((20_000, 2)) - 0.5
+        f, u = rng.random((600, 2)) - 0.5, rng.random((3000, 2)) - 0.5
     return (np.round(v * 2.0**23) / 2.0**23 for v in (f, u))
 
 
@@ -69,3 +69,10 @@ def test_scaled_points_zone_fp64(engine, points, e):
     """Through the zone, whose candidates the exact count decides: listed whole
     in small batches, behind the boxes in larger ones."""
     _check(engine, points, e, "inf", ("fp64",), (1, 40))
+
+
+@pytest.mark.parametrize("e,modes", [(-90, ("fp32", "fp64")), (-72, ("fp32", "fp64")), (-66, ("fp32", "fp64")),
+                                     (64, ("fp64",)), (66, ("fp64",)), (90, ("fp64",))])
+def test_scaled_points_slice(engine, points, e, modes):
+    """Through the slice filter, two warps a query and one."""
+    _check(engine, points, e, "slice", modes, (1, 40, 1400))
