@@ -329,7 +329,7 @@ __device__ __forceinline__ void filter_boxed(const VerifyArgs& A, const QDesc& d
                     bb = __double_as_longlong(f2d_bits(
                         __fmaf_ru(__double2float_ru(d.k2f64), ax, __double2float_ru(d.kf264))));
                 } else {
-                    bu = fmaf(d.k2f, fabsf(xs) + fabsf(ys), d.kf2);
+                    bu = user_bound(d, xs, ys);
                     bu2 = min(__float_as_uint(__fmul_ru(bu, 2.0f * (1.0f + 0x1p-20f))), 0x7f800000u);
                 }
                 // a lane's counts over its half-planes, and the sums over those
@@ -405,6 +405,9 @@ __device__ __forceinline__ void filter_boxed(const VerifyArgs& A, const QDesc& d
                     __syncwarp();
                 }
                 evals += base < INT_MAX / 2 ? ne : 0;
+                // an infinite bound decides nothing
+                if constexpr (!F64)
+                    if (!(bu < INFINITY)) later = nb;
                 // back to the users' own lanes
                 const int ce = base + (int)(sum & 0x7ffu);
                 state = (ce < k ? 1 : 0) |

@@ -90,6 +90,14 @@ __device__ __forceinline__ float user_lim(float x, float y)
     return 4.0f * fmaf(x, x, y * y) * (1.0f + 1e-4f) + 1e-30f;
 }
 
+// The FP32 evaluation bound of the user at offset (x, y), infinite from
+// BOUND_MAX on: no half-plane is certain for the user then.
+__device__ __forceinline__ float user_bound(const QDesc& d, float x, float y)
+{
+    const float b = fmaf(d.k2f, fabsf(x) + fabsf(y), d.kf2);
+    return b < BOUND_MAX ? b : INFINITY;
+}
+
 // Stage 1, FP32, over the slot's first nb half-planes: cnt = certified
 // violations (the loop leaves once every lane's users reached k), und =
 // half-planes the bound could not decide.  sp: the first ns of them staged;
@@ -119,7 +127,7 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
         x[t] = u[t].x - d.qx;
         y[t] = u[t].y - d.qy;
         lim[t] = user_lim(x[t], y[t]);
-        bu[t] = fmaf(d.k2f, fabsf(x[t]) + fabsf(y[t]), d.kf2);
+        bu[t] = user_bound(d, x[t], y[t]);
     }
     const int k = d.k;
     int m = 0;
@@ -198,9 +206,12 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
         if (!stopped && ns < nb) sweep(gp, nb);
     evals += (unsigned)(m * nvalid);
     bool again = false;
+    unsigned top[UPT];
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {
-        und[t] = rmin[t] <= __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
+        // (an infinite bound: r is infinite or, where m overflowed, a NaN)
+        top[t] = bu[t] < INFINITY ? __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f))) : 0x7fffffffu;
+        und[t] = rmin[t] <= top[t];
         again |= und[t] && cnt[t] < k && !(lim[t] > rho2);
     }
     if constexpr (COMPACT)
@@ -217,8 +228,7 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
                 const float4 p = i < ns ? ((const float4*)sp)[i] : gp[i];
 #pragma unroll
                 for (int t = 0; t < UPT; ++t)
-                    nc[t] += __float_as_uint(fmaf(p.x, x[t], fmaf(p.y, y[t], p.z)) + bu[t]) <=
-                             __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
+                    nc[t] += __float_as_uint(fmaf(p.x, x[t], fmaf(p.y, y[t], p.z)) + bu[t]) <= top[t];
             }
 #pragma unroll
             for (int t = 0; t < UPT; ++t) und[t] = und[t] && cnt[t] + nc[t] >= k;

@@ -76,3 +76,11 @@ def test_scaled_points_zone_fp64(engine, points, e):
 def test_scaled_points_slice(engine, points, e, modes):
     """Through the slice filter, two warps a query and one."""
     _check(engine, points, e, "slice", modes, (1, 40, 1400))
+
+
+@pytest.mark.parametrize("filter", ["slice", "inf"])
+@pytest.mark.parametrize("e", [64, 66, 90])
+def test_scaled_points_fp32(engine, points, e, filter):
+    """Float evaluations that overflow decide nothing, user by user (in the
+    filter's own blocks and in the verification kernel) and behind boxes."""
+    _check(engine, points, e, filter, ("fp32",), (1, 40) if filter == "inf" else (1, 40, 1400))
