@@ -578,7 +578,8 @@ struct ZClass {
 // Capacities of the slice filter: a k-entry heap per slice, half-planes of
 // the nearest facilities for the verification (no more than it uses, so
 // that all of them take part in its exact shortcut).
-ZoneCaps slice_caps(int kmax)
+// lc_most and rm: less room, for callers that count their memory.
+ZoneCaps slice_caps(int kmax, int lc_most = VERIFY_PLANES_MAX, int rm = 128)
 {
     ZoneCaps c;
     c.vc = std::max(1, kmax);
@@ -590,10 +591,10 @@ ZoneCaps slice_caps(int kmax)
     // distance to q.  Street workload, k up to 100: 68 users a query recounted
     // with at most 512 (0.81 ms FP32, 2.31 FP64), 2 with 768 (0.03), at 0.04
     // ms more in the filter.
-    const long long most = std::min<long long>(std::max<long long>(8LL * c.vc, 512), VERIFY_PLANES_MAX);
+    const long long most = std::min<long long>(std::max<long long>(8LL * c.vc, 512), lc_most);
     c.lc = (int)std::max<long long>(1, std::min<long long>(24LL * c.vc + 60, most));
     c.pc = 0;
-    c.rm = 128;
+    c.rm = rm;
     return c;
 }
 
@@ -604,6 +605,14 @@ bool use_slice(rknn_index* ix, int kmax)
     const size_t budget = std::min<size_t>(ix->smem_optin, 200 * 1024) - 1024;
     if (slice_layout(slice_caps(kmax)).bytes > budget) return false;    // k beyond the heaps' room
     return ix->filter == RKNN_FILTER_SLICE || kmax >= ix->slice_min_k;
+}
+
+// The slice filter's capacities within the influence zone's (fewer half-planes:
+// more users reach the exact count).
+ZoneCaps lean_caps(rknn_index* ix, int kmax)
+{
+    const ZoneCaps z = caps_fit(ix, caps_for(kmax));
+    return slice_caps(kmax, std::min(z.lc, VERIFY_PLANES_MAX), z.rm);
 }
 
 // Launch geometry of one batch, computed before any stream capture.
@@ -626,7 +635,9 @@ struct BatchPlan {
 
 // k_sorted: the batch's k in processing order (descending) when use_order,
 // else null (every query in one class sized for kmax).
-BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int* k_sorted, int kmax)
+// lean: slice classes take the room of the scratch estimate (scratch_per_query).
+BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int* k_sorted, int kmax,
+                     bool lean = false)
 {
     BatchPlan b;
     b.nq = nq;
@@ -648,7 +659,9 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.key = {nq, mode, use_order ? 1 : 0};
     for (auto& c : b.cls) {
         c.slice = use_slice(ix, c.kmax);
-        c.caps = c.slice ? slice_caps(c.kmax) : caps_fit(ix, caps_for(c.kmax));
+        if (!c.slice) c.caps = caps_fit(ix, caps_for(c.kmax));
+        else if (lean) c.caps = lean_caps(ix, c.kmax);
+        else c.caps = slice_caps(c.kmax);
         b.pstride = std::max(b.pstride, c.caps.lc);
         b.key.push_back(c.n);
         b.key.push_back(c.kmax);
@@ -704,6 +717,7 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.key.push_back(b.sort_grid);
     b.key.push_back(b.vupt);
     b.key.push_back(b.vwarps);
+    b.key.push_back(b.pstride);
     return b;
 }
 
@@ -2143,12 +2157,19 @@ int pad_pow2(int n)
 
 // Scratch a batch slot uses per query at a given largest k: half-planes and
 // bisector positions, segments, descriptors and offsets, and the result
-// pool's starting share (two 4096-entry int arrays).
-long long scratch_per_query(rknn_index* ix, int kmax)
+// pool's starting share (two 4096-entry int arrays).  lean: with the influence
+// zone's capacities, which a slice batch can be kept to.
+long long scratch_per_query(rknn_index* ix, int kmax, bool lean)
 {
-    const ZoneCaps c = caps_fit(ix, caps_for(kmax));
-    return 20LL * c.lc + 8LL * (2 * c.rm + 2) + (long long)sizeof(QDesc) + (long long)sizeof(ZStats) + 32 +
-           2LL * 4 * 4096;
+    ZoneCaps c = caps_fit(ix, caps_for(kmax));
+    if (!lean && ix->filter != RKNN_FILTER_INF) {
+        // (a smaller k of the batch may take the slice filter where kmax does not)
+        const ZoneCaps f = slice_caps(kmax);
+        c.lc = std::max(c.lc, f.lc);
+        c.rm = std::max(c.rm, f.rm);
+    }
+    return 20LL * c.lc + 8LL * (2 * c.rm + 2) + (long long)sizeof(QDesc) + (long long)sizeof(ZStats) +
+           (lean ? 32 : 176) + 2LL * 4 * 4096;
 }
 
 }  // namespace
@@ -2211,7 +2232,9 @@ rknn_status slot_launch(rknn_server* sv, Slot& sl, int inject)
         ksorted[i] = order[i] < nq ? sl.reqs[order[i]]->k : 1;
         kmax = std::max(kmax, ksorted[i]);
     }
-    sl.plan = plan_batch(ix, nqp, sl.reqs[0]->mode, true, ksorted.data(), kmax);
+    // (only a request on its own can need more than the budget, see below)
+    const bool lean = nqp * scratch_per_query(ix, kmax, false) > sv->o.scratch_bytes;
+    sl.plan = plan_batch(ix, nqp, sl.reqs[0]->mode, true, ksorted.data(), kmax, lean);
     Workspace& w = sl.ws;
     if (inject == INJECT_OOM) w.inject_oom = true;
     rknn_status s = ensure_ws(w, nqp, plan_caps(sl.plan), std::max<long long>(w.pool_cap, (long long)nqp * 4096));
@@ -2293,9 +2316,10 @@ void serve_loop(rknn_server* sv)
                 ReqPtr r = *it;
                 if (r->mode != mode) { ++it; continue; }
                 const int km = std::max(kmax, (int)r->k);
-                // a request's own estimate never exceeds the budget (submit
-                // refuses such requests), so the first one always fits
-                const long long need = (long long)pad_pow2((int)sl.reqs.size() + 1) * scratch_per_query(sv->ix, km);
+                // a request's own lean estimate never exceeds the budget (submit
+                // refuses such requests), so the first one always fits; others
+                // join it while the batch fits with all its room
+                const long long need = (long long)pad_pow2((int)sl.reqs.size() + 1) * scratch_per_query(sv->ix, km, false);
                 if (!sl.reqs.empty() && need > budget) break;
                 sl.reqs.push_back(r);
                 kmax = km;
@@ -2405,10 +2429,10 @@ rknn_status rknn_serve_submit(rknn_server* sv, int32_t q, int32_t k, int32_t mod
                                       std::to_string(sv->ix->nf) + ")");
     if (k <= 0) return fail(RKNN_ERR_ARG, "k must be a positive integer");
     if (mode != RKNN_MODE_FP32 && mode != RKNN_MODE_FP64) return fail(RKNN_ERR_ARG, "bad mode");
-    // admission: a request whose scratch estimate alone (as a batch of its
+    // admission: a request whose lean scratch estimate alone (as a batch of its
     // own) exceeds the server's budget is refused, so that no batch passes
     // the budget
-    const long long need1 = (long long)pad_pow2(1) * scratch_per_query(sv->ix, k);
+    const long long need1 = (long long)pad_pow2(1) * scratch_per_query(sv->ix, k, true);
     if (need1 > sv->o.scratch_bytes)
         return fail(RKNN_ERR_CAPACITY, "request needs about " + std::to_string(need1) +
                                            " bytes of scratch, more than the server's scratch_bytes (" +

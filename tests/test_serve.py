@@ -136,3 +136,27 @@ def test_request_beyond_the_scratch_budget_is_refused(engine, served):
     with engine.Server(idx, slots=1, max_batch=8, scratch_bytes=8 << 20) as srv:
         t = srv.submit(q, 5, "fp32")
         assert np.array_equal(srv.wait(t), orc.query(q, 5))
+
+
+def test_batches_keep_to_the_scratch_budget(engine, served):
+    """64 queries at k = 10 need 300 half-planes and 258 segments each, 2.63 MB
+    with their result shares: a budget of 2.56 MB admits 32 a batch."""
+    ds, idx, _ = served
+    n = 2000
+    qs = np.random.default_rng(13).integers(0, ds.nf, n).astype(np.int32)
+    with engine.Server(idx, slots=1, max_batch=4096, scratch_bytes=64 * 40_000) as srv:
+        lat, nres = srv.replay(qs, np.full(n, 10, np.int32), "fp32", np.zeros(n))
+        st = srv.stats()
+    assert st["completed"] == n and st["mean_batch"] <= 32
+    assert [len(x) for x in idx.query_batch(qs, 10, "fp32")] == nres.tolist()
+
+
+@pytest.mark.parametrize("k", [1, 10, 40])
+def test_lean_batches(engine, served, k):
+    """A budget between a request's estimate and what the slice filter would
+    take: the request is admitted and runs with fewer half-planes."""
+    ds, idx, orc = served
+    with engine.Server(idx, slots=1, scratch_bytes=32 * (20 * (6 * k + 40) + 34_100)) as srv:
+        for q in ds.queries[:4]:
+            for mode in ("fp32", "fp64"):
+                assert np.array_equal(srv.wait(srv.submit(int(q), k, mode)), orc.query(int(q), k)), (int(q), k, mode)
