@@ -659,8 +659,11 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.key = {nq, mode, use_order ? 1 : 0};
     for (auto& c : b.cls) {
         c.slice = use_slice(ix, c.kmax);
+        // batches of millions: memory bounds their size (at k=100 44 KB a query
+        // with this room, 51 with all of it)
         if (!c.slice) c.caps = caps_fit(ix, caps_for(c.kmax));
         else if (lean) c.caps = lean_caps(ix, c.kmax);
+        else if (nq > 1 << 20) c.caps = slice_caps(c.kmax, 512, 64);
         else c.caps = slice_caps(c.kmax);
         b.pstride = std::max(b.pstride, c.caps.lc);
         b.key.push_back(c.n);

@@ -160,3 +160,18 @@ def test_lean_batches(engine, served, k):
         for q in ds.queries[:4]:
             for mode in ("fp32", "fp64"):
                 assert np.array_equal(srv.wait(srv.submit(int(q), k, mode)), orc.query(int(q), k)), (int(q), k, mode)
+
+
+def test_batch_of_more_than_a_million(engine):
+    """Beyond 2^20 queries the filter's capacities are smaller."""
+    ds = datagen.uniform(50, 2000, seed=33, nq=50, k=1)
+    o = O.Oracle.of(ds)
+    n = (1 << 20) + 33
+    with engine.Index.of(ds) as idx:
+        for k in (1, 12):
+            got, off = idx.query_batch_flat(np.arange(n, dtype=np.int32) % 50, k, "fp32")
+            w = [o.query(q, k) for q in range(50)]
+            m = np.diff(off)
+            assert np.array_equal(m, np.resize([x.size for x in w], n))
+            for i in (0, 1, 49, 50, n // 2, n - 1):
+                assert np.array_equal(got[off[i]:off[i + 1]], w[i % 50]), (k, i)
