@@ -156,7 +156,7 @@ struct Workspace {
     std::map<GraphKey, CachedGraph> graphs;
     cudaStream_t aux[NAUX] = {};
     cudaEvent_t fork = nullptr, join[NAUX] = {};
-    bool inject_oom = false;       // failure test hook: the next ensure_ws fails (host only)
+    int inject_oom = 0;            // failure test hook: the n-th ensure_ws from now fails (host only)
 };
 
 }  // namespace
@@ -449,10 +449,9 @@ rknn_status grow_ws(Workspace& w, int nqc, int lc, int sc);
 rknn_status ensure_ws(Workspace& w, int nq, const ZoneCaps& caps, long long pool_need)
 {
     const int seg_cap = 2 * caps.rm + 2;
-    if (w.inject_oom) {
+    if (w.inject_oom > 0 && --w.inject_oom == 0) {
         // failure test hook (rknn_serve_inject_fault): this growth fails as
         // a cudaMalloc would, after the old arrays were released
-        w.inject_oom = false;
         free_ws(w);
         return fail(RKNN_ERR_OOM, "workspace growth failed (injected for a failure test)");
     }
@@ -1594,6 +1593,26 @@ rknn_status rknn_debug_zone_stats(rknn_index* ix, void* out, int32_t nq)
     return RKNN_OK;
 }
 
+// Failure test hook: the n-th sizing of the index's workspace from now fails as
+// an allocation would (made on the host); 0 takes it back.  shape: the
+// verification's users per lane, warps per block and whether the former are
+// chosen automatically.  Not part of the public header.
+rknn_status rknn_debug_fail_workspace(rknn_index* ix, int32_t n)
+{
+    if (!ix || n < 0) return fail(RKNN_ERR_ARG, "bad argument");
+    std::lock_guard<std::mutex> lk(ix->mu);
+    ix->ws.inject_oom = n;
+    return RKNN_OK;
+}
+rknn_status rknn_debug_shape(rknn_index* ix, int32_t* shape)
+{
+    if (!ix || !shape) return fail(RKNN_ERR_ARG, "null argument");
+    shape[0] = ix->vupt;
+    shape[1] = ix->vwarps;
+    shape[2] = ix->vupt_auto;
+    return RKNN_OK;
+}
+
 rknn_status rknn_set_stream(rknn_index* ix, void* stream)
 {
     if (!ix) return fail(RKNN_ERR_ARG, "index is null");
@@ -2239,7 +2258,7 @@ rknn_status slot_launch(rknn_server* sv, Slot& sl, int inject)
     const bool lean = nqp * scratch_per_query(ix, kmax, false) > sv->o.scratch_bytes;
     sl.plan = plan_batch(ix, nqp, sl.reqs[0]->mode, true, ksorted.data(), kmax, lean);
     Workspace& w = sl.ws;
-    if (inject == INJECT_OOM) w.inject_oom = true;
+    if (inject == INJECT_OOM) w.inject_oom = 1;
     rknn_status s = ensure_ws(w, nqp, plan_caps(sl.plan), std::max<long long>(w.pool_cap, (long long)nqp * 4096));
     if (s != RKNN_OK) return s;
     for (int i = 0; i < nqp; ++i) {
@@ -2603,6 +2622,26 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
     };
     const float fpc0 = ix->fac_per_cell, upc0 = ix->usr_per_cell;
     const int upt0 = ix->vupt, vw0 = ix->vwarps;
+    const bool auto0 = ix->vupt_auto;
+    // a failing return leaves the densities and the shape of the entry
+    struct Restore {
+        rknn_index* ix;
+        float fpc, upc;
+        int upt, vw;
+        bool automatic, done;
+        ~Restore()
+        {
+            if (done) return;
+            const std::string err = g_err;
+            std::lock_guard<std::mutex> lk(ix->mu);
+            ix->vupt = upt;
+            ix->vwarps = vw;
+            ix->vupt_auto = automatic;
+            ix->plan_cache.reset();
+            if (ix->fac_per_cell != fpc || ix->usr_per_cell != upc || !ix->d_ustart) build_grids(ix, fpc, upc);
+            g_err = err;
+        }
+    } restore{ix, fpc0, upc0, upt0, vw0, auto0, false};
     rknn_tune_result r{};
     r.fac_per_cell = fpc0; r.usr_per_cell = upc0; r.users_per_thread = upt0; r.verify_warps = vw0;
     s = time_batch(r.default_ms);
@@ -2634,7 +2673,6 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
         s = build_grids(ix, r.fac_per_cell, r.usr_per_cell);
     }
     if (s != RKNN_OK) return s;
-    const bool auto0 = ix->vupt_auto;
     bool shaped = false;            // a trial's shape is the best
     ix->vupt_auto = false;
     for (int upt : upts)
@@ -2662,6 +2700,7 @@ extern "C" rknn_status rknn_index_tune(rknn_index* ix, const int32_t* q, const i
     ix->vupt_auto = auto0 && !shaped;
     ix->vwarps = r.verify_warps;
     ix->plan_cache.reset();
+    restore.done = true;
     *result = r;
     return RKNN_OK;
 }
