@@ -1896,6 +1896,15 @@ rknn_status rknn_last_stats(rknn_index* ix, rknn_query_stats* stats)
     return collect_stats(c, ix->last_nq, stats);
 }
 
+namespace {
+// out[i] = table[at[i]]
+__global__ void gather_kernel(const int* table, const int* at, int n, int* out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = table[at[i]];
+}
+}  // namespace
+
 rknn_status rknn_last_zone(rknn_index* ix, int32_t slot, int32_t* bis_fac, int32_t cap, int32_t* n_bis,
                            int32_t* flags)
 {
@@ -1903,17 +1912,21 @@ rknn_status rknn_last_zone(rknn_index* ix, int32_t slot, int32_t* bis_fac, int32
     std::lock_guard<std::mutex> lk(ix->mu);
     if (slot < 0 || slot >= ix->last_nq) return fail(RKNN_ERR_ARG, "slot out of range");
     Workspace& w = ix->ws;
+    if (!w.d_qd || !w.d_surv) return fail(RKNN_ERR_STATE, "the last call left no workspace");
     QDesc d;
-    CK(cudaMemcpy(&d, w.d_qd + slot, sizeof(QDesc), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&d, w.d_qd + slot, sizeof(QDesc), cudaMemcpyDeviceToHost, ix->stream));
+    CK(cudaStreamSynchronize(ix->stream));
     *n_bis = d.nb;
     if (flags) *flags = d.flags;
     int n = std::min(d.nb, cap);
     if (n > 0 && bis_fac) {
-        std::vector<int> pos(n);
-        CK(cudaMemcpy(pos.data(), w.d_bispos + (size_t)slot * ix->last_lc, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        std::vector<int> fidx(ix->nf);      // cell-sorted position -> facility input index
-        CK(cudaMemcpy(fidx.data(), ix->d_fidx, sizeof(int) * fidx.size(), cudaMemcpyDeviceToHost));
-        for (int i = 0; i < n; ++i) bis_fac[i] = fidx[pos[i]];
+        // translated on the device, in the survivor list (at least 4 M entries,
+        // idle between batches)
+        int* out = (int*)w.d_surv;
+        gather_kernel<<<(n + 255) / 256, 256, 0, ix->stream>>>(ix->d_fidx, w.d_bispos + (size_t)slot * ix->last_lc, n, out);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(bis_fac, out, sizeof(int) * n, cudaMemcpyDeviceToHost, ix->stream));
+        CK(cudaStreamSynchronize(ix->stream));
     }
     return RKNN_OK;
 }
