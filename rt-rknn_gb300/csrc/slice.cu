@@ -128,15 +128,14 @@ __device__ __forceinline__ float box_bound(float X0, float X1, float Y0, float Y
     return r;
 }
 
-// Whether an offset (vx, vy) lies beyond twice a reach or need r.  |v|^2 / 4 is
-// made from quartered factors, rounded down: it overflows only where r^2 does
-// or |v| > 2r, and then an infinite r^2 is not exceeded.  What underflows on the
-// left is below SQUARE_ERR on the right (0 >= 0 dropped facilities that decide
-// users where offsets are below about 1e-23).
-__device__ __forceinline__ bool beyond(float vx, float vy, float r)
+// Whether an offset of squared length d2 (float) lies beyond twice a reach or
+// need r.  A d2 that overflowed counts as the largest float: the left side is a
+// lower bound in any case.  What underflows there is below SQUARE_ERR on the
+// right (0 >= 0 dropped facilities that decide users where offsets are below
+// about 1e-23).
+__device__ __forceinline__ bool beyond(float d2, float r)
 {
-    constexpr float C = 0.25f * (1.0f - 8.0f * kU32);
-    return fmaf(C * vx, vx, (C * vy) * vy) > fmaf(r, r, vitem::SQUARE_ERR);
+    return 0.25f * (1.0f - 8.0f * kU32) * fminf(d2, FLT_MAX) > fmaf(r, r, vitem::SQUARE_ERR);
 }
 
 // Whether every facility in a box (relative to q, not around it) lies beyond
@@ -145,7 +144,7 @@ __device__ __forceinline__ bool box_idle(float X0, float X1, float Y0, float Y1,
 {
     const float dx = fmaxf(fmaxf(X0, -X1), 0.0f), dy = fmaxf(fmaxf(Y0, -Y1), 0.0f);
     const float R = box_bound(X0, X1, Y0, Y1, Ns);
-    return beyond(dx * (1.0f - 2e-6f), dy * (1.0f - 2e-6f), R * (1.0f + 2e-6f));
+    return beyond(fmaf(dx, dx, dy * dy) * (1.0f - 8e-6f), R);
 }
 
 // Cell ri of the square ring at Chebyshev distance ring around (qcx, qcy):
@@ -261,7 +260,7 @@ __device__ __forceinline__ int trim_planes(const float2* fxy, int nf, int* lpos,
             dx = f.x - q.x;
             dy = f.y - q.y;
         }
-        const bool keep = m < n && !beyond(dx, dy, Ns[slice_of(dx, dy)]);
+        const bool keep = m < n && !beyond(fmaf(dx, dx, dy * dy), Ns[slice_of(dx, dy)]);
         const unsigned km = __ballot_sync(FULL, keep);          // (every lane has read its entry)
         if (keep) lpos[k + __popc(km & ((1u << lane) - 1))] = pos;
         k += __popc(km);
@@ -599,8 +598,9 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 }
                 const int sj = slice_of(vx, vy);
                 const float rj = Rs[sj], nj = Ns[sj];
-                const bool hp = ok && !beyond(vx, vy, nj);
-                unsigned m = __ballot_sync(FULL, ok && !beyond(vx, vy, rj));
+                const float d2 = fmaf(vx, vx, vy * vy);
+                const bool hp = ok && !beyond(d2, nj);
+                unsigned m = __ballot_sync(FULL, ok && !beyond(d2, rj));
                 // half-planes: the first LC of them, in ring order
                 const unsigned pm = __ballot_sync(FULL, hp);
                 int at0 = nL;       // this batch's first half-plane slot
@@ -823,7 +823,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
                 dy = f.y - qf.y;
             }
             const float c = fmaf(dx, dx, dy * dy);
-            const bool keep = m < nL && !beyond(dx, dy, Ns[slice_of(dx, dy)]);
+            const bool keep = m < nL && !beyond(c, Ns[slice_of(dx, dy)]);
             const unsigned km = __ballot_sync(FULL, keep);      // (every lane has read its entry)
             if (keep) {
                 const int o = nk + __popc(km & ((1u << lane) - 1));
