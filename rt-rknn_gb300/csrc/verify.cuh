@@ -8,11 +8,18 @@ constexpr int VERIFY_UPT = 4;                       // default users per lane pe
 constexpr int VERIFY_CHUNK = 32 * VERIFY_UPT;       // default users per work item
 constexpr int VERIFY_WARPS = 8;                     // default warps per block
 constexpr int VERIFY_SAMPLES = 1024;                // work-item offsets cached per block
-// FP32: candidates from which boxes come first (verification, ms, with the line
-// at 384 / 512 / 768: uniform 16,384 queries of 400 candidates 0.395 / 0.277 /
-// 0.254, of 640 - / 0.682 / 0.526; street layout - / 1.482 / 1.497; calls of the
-// street and clustered layouts with k to 100 and of k=25 1-2 % slower at 768)
-constexpr int BOX_MIN_CAND = 512;
+// FP32: whether boxes come first in a slot of n candidates.  Measured over 128
+// users (ns of verification, 16,384 queries), user by user costs about 1 + 0.14 k
+// (each user meets some 6 k half-planes before it is decided) and with boxes
+// about 2.6 + 105 k / n (the fewer users a facility has, the wider their boxes):
+// uniform layout with 10 users a facility k=60 9.9 / 9.9, k=80 13.0 / 10.9, with
+// 50 k=7 1.9 / 3.7, k=24 3.9 / 4.1, street layout k=6 2.0 / 3.4, k=20 3.3 / 3.5.
+// The line lies where both cost the same on these and on the clustered layout
+// (k=16 160 / 162 us, k=32 297 / 272).
+__host__ __device__ __forceinline__ bool boxes_first(int k, int n)
+{
+    return (float)k * (float)(n - 750) > 16.0f * (float)n;
+}
 // Most queries of an influence-zone batch, and candidates of a query, that go
 // to the recount without a half-plane test.  The zone's half-planes reject
 // about half of the candidates and accept none (its pruning may have dropped a
