@@ -198,7 +198,7 @@ struct rknn_index {
     int filter = RKNN_FILTER_AUTO;
     int slice_min_k = 1;
     int num_sms = 0;
-    int recount_grid = 0;       // one wave of recount_kernel blocks
+    int recount_grid = 0, recount64_grid = 0;   // one wave of recount_kernel's blocks
     bool pdl = true;            // programmatic dependent launch between the batch kernels
     // the last uniform-k host batch's plan, reused by the next batch of the
     // same size, mode and k (dropped when the grids or the verification's
@@ -861,7 +861,8 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     mark(2);
     CK(launch_k(verify_fn(b.mode, b.vupt), b.vgrid, b.vwarps * 32, b.vsmem, st, pdl && (ncls == 1 || !b.fuse), va));
     mark(3);
-    CK(launch_k(b.mode == MODE_FP64 ? recount64_kernel : recount_kernel, ix->recount_grid, 256, 0, st, pdl, va));
+    if (b.mode == MODE_FP64) CK(launch_k(recount64_kernel, ix->recount64_grid, 256, 0, st, pdl, va));
+    else CK(launch_k(recount_kernel, ix->recount_grid, 256, 0, st, pdl, va));
     mark(4);
     // the output offsets: in finalize itself for batches of up to
     // FIN_SCAN_MAX slots, else by the scan kernel
@@ -1301,6 +1302,9 @@ rknn_status rknn_index_create(const float* fxy, const int32_t* fid, int64_t nf, 
         int per = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, recount_kernel, 256, 0);
         ix->recount_grid = std::max(1, per) * ix->num_sms;
+        per = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, recount64_kernel, 256, 0);
+        ix->recount64_grid = std::max(1, per) * ix->num_sms;
     }
     CKB(allow_dynamic_smem((const void*)slice_kernel, optin));
     CKB(allow_dynamic_smem((const void*)sort_large_kernel, optin));

@@ -310,7 +310,7 @@ __device__ __forceinline__ int group_exact_count(const Counted& d, const VerifyA
 // the count's latency, not its work, bounds a small batch.  sc: one shared
 // counter per group.
 template <bool F64>
-__device__ __forceinline__ void recount_listed(const VerifyArgs& A, VCount& vc, int* sc)
+__device__ __forceinline__ void recount_listed(const VerifyArgs& A, VCount& vc, int* sc, Counted* run_c, int2* run_e)
 {
     const int lane = threadIdx.x & 31;
     const int n = min(*A.surv_count, A.surv_cap);
@@ -326,7 +326,8 @@ __device__ __forceinline__ void recount_listed(const VerifyArgs& A, VCount& vc, 
     // short runs where survivors are few, up to 32 where the queue's counter
     // would be the bound.  Survivors of one query are neighbours in the list
     // and alike, so a run takes every nruns-th.  A run's records are loaded by
-    // its lanes at once.  Clustered workload, 209 k survivors: 0.64 ms with
+    // its lanes at once and kept in shared memory, where the count's registers
+    // leave room for more warps.  Clustered workload, 209 k survivors: 0.64 ms with
     // fixed shares, 0.51 with runs of neighbours, 0.46 so; uniform zone batch,
     // 101 k alike ones: 66, 68 and 68 us.
     const int run = G == 1 ? max(1, min(32, n / (8 * nw))) : 1;
@@ -335,24 +336,23 @@ __device__ __forceinline__ void recount_listed(const VerifyArgs& A, VCount& vc, 
     int r = blockIdx.x * gpb + gid;
     while (r < nruns) {
         const int m = (n - 1 - r) / nruns + 1;
-        int2 e = make_int2(-1, 0);
-        float2 u = make_float2(0.f, 0.f), q = u;
-        int qpos = 0, k = 0;
+        __syncwarp();                    // the last run's records have been read
         if (lane < m) {
-            e = A.surv[VX(r + lane * nruns, A.surv_cap, 215)];
+            const int2 e = A.surv[VX(r + lane * nruns, A.surv_cap, 215)];
+            Counted c = {};
             if (e.x >= 0) {
                 const QDesc* d = A.qd + e.x;
-                u = A.uxy[VX(e.y, A.nu, 216)];
-                q = make_float2(d->qx, d->qy);
-                qpos = d->qpos;
-                k = d->k;
+                const float2 u = A.uxy[VX(e.y, A.nu, 216)];
+                c = {u.x, u.y, d->qx, d->qy, d->qpos, d->k};
             }
+            run_c[lane] = c;
+            run_e[lane] = e;
         }
+        __syncwarp();
         for (int j = 0; j < m; ++j) {
-            const int slot = __shfl_sync(FULL, e.x, j), pos = __shfl_sync(FULL, e.y, j);
+            const int slot = run_e[j].x, pos = run_e[j].y;
             if (slot < 0) continue;      // the group's warps skip it alike
-            const Counted c = {__shfl_sync(FULL, u.x, j), __shfl_sync(FULL, u.y, j), __shfl_sync(FULL, q.x, j),
-                               __shfl_sync(FULL, q.y, j), __shfl_sync(FULL, qpos, j), __shfl_sync(FULL, k, j)};
+            const Counted c = run_c[j];
             const int cnt = group_exact_count<F64>(c, A, G, gi, 1 + gid, sc + gid, s_fac, s_rech);
             if (cnt < c.k && gi == 0 && lane == 0) {
                 const int at = atomicAdd(A.res_count + slot, 1);
@@ -377,12 +377,19 @@ __device__ __forceinline__ void recount_body(const VerifyArgs& A)
     pdl_wait();
     pdl_trigger();
     __shared__ int sc[8];
+    __shared__ Counted run_c[8][32];
+    __shared__ int2 run_e[8][32];
     VCount vc = {};
-    recount_listed<F64>(A, vc, sc);
+    recount_listed<F64>(A, vc, sc, run_c[threadIdx.x >> 5], run_e[threadIdx.x >> 5]);
     vc.flush(A.vstats);
 }
 
-__global__ void __launch_bounds__(256) recount_kernel(VerifyArgs A) { recount_body<false>(A); }
+// FP32 with four blocks an SM (64 registers, spills in the exact predicate's
+// rare call), FP64 with three (79): FP32 waits for its loads, FP64 for its pipe.
+// ms, four / three blocks: FP32 uniform k=500, 400 queries 2.50 / 3.15, street
+// zones k=25, 1000 queries 1.00 / 1.26; FP64 the same 2.72 / 2.72 (a grid of four
+// blocks an SM over three resident ones: 2.74, and 4 us more on small batches).
+__global__ void __launch_bounds__(256, 4) recount_kernel(VerifyArgs A) { recount_body<false>(A); }
 __global__ void __launch_bounds__(256) recount64_kernel(VerifyArgs A) { recount_body<true>(A); }
 
 // ---------------------------------------------------------------- scans
