@@ -324,13 +324,17 @@ __device__ __forceinline__ void recount_listed(const VerifyArgs& A, VCount& vc, 
     // by its number and later ones from a queue (a survivor far from every
     // facility walks a large disc, so shares fixed beforehand end unevenly);
     // short runs where survivors are few, up to 32 where the queue's counter
-    // would be the bound.  Survivors of one query are neighbours in the list
-    // and alike, so a run takes every nruns-th.  A run's records are loaded by
-    // its lanes at once and kept in shared memory, where the count's registers
-    // leave room for more warps.  Clustered workload, 209 k survivors: 0.64 ms with
-    // fixed shares, 0.51 with runs of neighbours, 0.46 so; uniform zone batch,
-    // 101 k alike ones: 66, 68 and 68 us.
-    const int run = G == 1 ? max(1, min(32, n / (8 * nw))) : 1;
+    // would be the bound: about three runs a warp in FP32, eight in FP64, whose
+    // counts are longer (zone batches of 50 k / 100 k / 250 k survivors, us, with
+    // eight / four / three / two: FP32 57 / 47 / 45 / 45, 70 / 61 / 61 / 64, 127 /
+    // 119 / 123 / 135, FP64 70 / 65 / 64 / 68, 115 / 111 / 119 / 127, 283 / 297 /
+    // 307 / 324; fixed shares took 43, 66 and 131 in FP32).  Survivors of one
+    // query are neighbours in the list and alike, so a run takes every nruns-th.
+    // A run's records are loaded by its lanes at once and kept in shared memory,
+    // where the count's registers leave room for more warps.  Clustered workload,
+    // 209 k survivors (eight runs a warp): 0.64 ms with fixed shares, 0.51 with
+    // runs of neighbours, 0.46 so.
+    const int run = G == 1 ? max(1, min(32, n / ((F64 ? 8 : 3) * nw))) : 1;
     const int nruns = (n + run - 1) / run;
     const int ngroups = gridDim.x * gpb;
     int r = blockIdx.x * gpb + gid;
