@@ -624,6 +624,7 @@ struct BatchPlan {
     int seg_stage = 0;          // user segments it stages per warp
     int vupt = VERIFY_UPT, vwarps = VERIFY_WARPS;
     int list_cand = -1;         // see LIST_CAND
+    bool box_batch = false;     // see BOX_MIN_CAND
     int parts = 1;              // parts of 32 vupt users in a verification work item
     bool fuse = false;          // the slice filter verifies its own slots (FP32, every class a slice class)
     size_t vsmem = 0;
@@ -693,6 +694,7 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
     if (nq <= LIST_QUERIES && std::none_of(b.cls.begin(), b.cls.end(), [](const ZClass& c) { return c.slice; }))
         b.list_cand = LIST_CAND;
+    b.box_batch = boxes_first(kmax / 2, (int)std::min(1e9, 1.5 * kmax * (double)ix->nu / (double)ix->nf));
     int rm = 0;
     for (auto& c : b.cls) rm = std::max(rm, c.caps.rm);
     b.seg_stage = std::min(2 * rm + 2, SEG_STAGE_MAX);
@@ -717,6 +719,7 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     if ((long long)kmax * ix->nu >= (long long)SORT_MIN_MEAN * ix->nf)
         b.sort_grid = std::min(nq, occupancy(ix, (const void*)sort_large_kernel, SORT_THREADS, sort_large_smem()) * ix->num_sms);
     b.key.push_back(b.sort_grid);
+    b.key.push_back(b.box_batch);
     b.key.push_back(b.vupt);
     b.key.push_back(b.vwarps);
     b.key.push_back(b.pstride);
@@ -787,6 +790,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     va.stage_cap = b.stage_cap;
     va.parts = b.parts;
     va.list_cand = b.list_cand;
+    va.box_batch = b.box_batch;
     va.segs = w.d_segs; va.seg_cap = w.seg_cap; va.seg_stage = b.seg_stage;
     va.chunk_off = w.d_chunk_off; va.cand_off = w.d_cand_off; va.reg_len = w.d_reg_len; va.nq = nq;
     va.uxy = ix->d_uxy; va.uid = ix->d_uid; va.fxy = ix->d_fxy; va.fstart = ix->d_fstart; va.gf = ix->gf;

@@ -20,6 +20,14 @@ __host__ __device__ __forceinline__ bool boxes_first(int k, int n)
 {
     return (float)k * (float)(n - 750) > 16.0f * (float)n;
 }
+// A batch whose largest k is beyond that line by a factor of two, at the 1.5
+// candidates for each of the users that k facilities have (1.4 to 1.5 on uniform
+// and street layouts), takes the boxes from this many candidates on instead:
+// slots of both kinds side by side miss the instruction caches (verification of
+// 16,384 queries of k from 1 to a largest one, us, so / by the line: street layout
+// k to 24 547 / 416, to 50 864 / 997, to 100 1488 / 1787, 50 users a facility
+// k to 32 432 / 346, to 64 684 / 746, clustered k to 50 860 / 839, to 100 1743 / 1840).
+constexpr int BOX_MIN_CAND = 512;
 // Most queries of an influence-zone batch, and candidates of a query, that go
 // to the recount without a half-plane test.  The zone's half-planes reject
 // about half of the candidates and accept none (its pruning may have dropped a
@@ -42,6 +50,7 @@ struct VerifyArgs {
     int stage_cap;           // half-planes used per slot, at most 1024 (the first ones;
                              // fewer only means more users reach the exact recount)
     int list_cand = -1;      // slots of up to this many candidates go to the recount whole
+    bool box_batch = false;  // FP32: see BOX_MIN_CAND
     int parts = 1;           // parts of 32 * (users per lane) users in a work item
     const int2* segs;        // [slot][seg_cap]
     int seg_cap;
