@@ -161,6 +161,7 @@ struct QDesc {
     int nb;            // bisector half-planes stored
     int nseg;          // user segments stored
     float k2f, kf2;    // per-user FP32 bound: 8u(2F'(|x'|+|y'|) + F'^2) = k2f*(|x'|+|y'|) + kf2
+                       // (kf2 infinite: see filter_bound)
     double k2f64, kf264;
     int ncand;         // users in all segments
     int flags;         // RKNN_QF_* bits
@@ -168,6 +169,16 @@ struct QDesc {
                        // (0 when unknown): a user with 2|u-q| <= rho is decided by them
     int pad;
 };
+
+// kf2, or infinity when a float evaluation of a half-plane may overflow for a user
+// at |x'| + |y'| <= span: it may then do so on the way to a small value of either
+// sign, so in float nothing is certain for the query's users (FP32 counts all of
+// them exactly).  Below 1e31 the sum 2F'span + F'^2, and with it every
+// intermediate, stays below 2.2e37.
+__device__ __forceinline__ float filter_bound(float k2f, float kf2, float span)
+{
+    return fmaf(k2f, span, kf2) < 1e31f ? kf2 : __int_as_float(0x7f800000);
+}
 
 // QDesc.flags
 constexpr int QF_ZONE_V_OVERFLOW = 1;    // vertex capacity reached: zone stopped early

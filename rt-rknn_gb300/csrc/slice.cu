@@ -870,6 +870,7 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         const float Fp2 = __fmul_ru(Fp, Fp);
         k2f = __fmul_ru(Fp, 16.0f * kU32 * (1.0f + 2e-6f));
         kf2 = __fadd_ru(__fmul_ru(Fp2, 8.0f * kU32 * (1.0f + 2e-6f)), 1e-30f);
+        kf2 = filter_bound(k2f, kf2, (bx1 - bx0) + (by1 - by0));
         k2f64 = (double)__fmul_ru(Fp, 16.0f * (float)kU64 * (1.0f + 2e-6f));
         kf264 = (double)__fmul_ru(Fp2, 8.0f * (float)kU64 * (1.0f + 2e-6f)) + 1e-300;
         }   // half-planes

@@ -120,7 +120,7 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
             __syncwarp();
             const float4* src = A.planes + (size_t)s * A.lc;
             const int nst = min(d.nb, A.stage_cap);
-            listed = A.list_cand >= d.ncand;
+            listed = A.list_cand >= d.ncand || (!F64 && !(d.kf2 < INFINITY));
             boxed = listed || F64 || (A.box_batch ? d.ncand >= BOX_MIN_CAND : boxes_first(d.k, d.ncand));
             if (listed) {
                 // no half-planes needed

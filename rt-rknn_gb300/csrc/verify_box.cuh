@@ -37,7 +37,7 @@ __device__ __forceinline__ float warp_fmax(float v)
 }
 
 // A box of user offsets from q: centre, half extents (rounded up) and the FP32
-// evaluation bound of its users (infinite from BOUND_MAX on).
+// evaluation bound of its users.
 struct UserBox {
     float cx, cy, hx, hy, b;
 };
@@ -49,8 +49,7 @@ __device__ __forceinline__ UserBox make_box(const QDesc& d, float x0, float x1, 
     r.cy = 0.5f * y0 + 0.5f * y1;
     r.hx = fmaxf(__fsub_ru(x1, r.cx), __fsub_ru(r.cx, x0));
     r.hy = fmaxf(__fsub_ru(y1, r.cy), __fsub_ru(r.cy, y0));
-    const float b = __fmaf_ru(d.k2f, __fadd_ru(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1))), d.kf2);
-    r.b = b < BOUND_MAX ? b : INFINITY;
+    r.b = __fmaf_ru(d.k2f, __fadd_ru(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1))), d.kf2);
     return r;
 }
 
@@ -63,9 +62,9 @@ __device__ __forceinline__ UserBox make_box(const QDesc& d, float x0, float x1, 
 // x and y, 2u|a|X + 2u|b|Y + 5u|c|; the two FMAs below add u|a|X + 2u|b|Y +
 // 2u|c|.  With |a|, |b| <= 2F' and |c| <= F'^2 that is at most
 // 8uF'(X + Y) + 7uF'^2, below the box's bound 8u (2F'(X + Y) + F'^2).
-// Nothing overflows below BOUND_MAX; from it on the box's bound is infinite,
-// which leaves the pair undecided whatever overflows (mc + r < -inf is false,
-// and so is mc - r > inf; NaNs compare false).
+// Where something may overflow the bound is infinite (filter_bound), which
+// leaves the pair undecided (mc + r < -inf is false, and so is mc - r > inf; NaNs
+// compare false).
 // NO_PLANE is neither (and undecided where the bound overflows: callers mask
 // the lanes that hold it).
 #define NO_PLANE make_float4(0.0f, 0.0f, INFINITY, 0.0f)
@@ -329,7 +328,7 @@ __device__ __forceinline__ void filter_boxed(const VerifyArgs& A, const QDesc& d
                     bb = __double_as_longlong(f2d_bits(
                         __fmaf_ru(__double2float_ru(d.k2f64), ax, __double2float_ru(d.kf264))));
                 } else {
-                    bu = user_bound(d, xs, ys);
+                    bu = fmaf(d.k2f, fabsf(xs) + fabsf(ys), d.kf2);
                     bu2 = min(__float_as_uint(__fmul_ru(bu, 2.0f * (1.0f + 0x1p-20f))), 0x7f800000u);
                 }
                 // a lane's counts over its half-planes, and the sums over those
@@ -405,9 +404,6 @@ __device__ __forceinline__ void filter_boxed(const VerifyArgs& A, const QDesc& d
                     __syncwarp();
                 }
                 evals += base < INT_MAX / 2 ? ne : 0;
-                // an infinite bound decides nothing
-                if constexpr (!F64)
-                    if (!(bu < INFINITY)) later = nb;
                 // back to the users' own lanes
                 const int ce = base + (int)(sum & 0x7ffu);
                 state = (ce < k ? 1 : 0) |

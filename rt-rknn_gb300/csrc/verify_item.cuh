@@ -79,23 +79,10 @@ __device__ __forceinline__ int exact_count(float ux, float uy, const QDesc& d, c
     return cnt;
 }
 
-// A float evaluation bound 8u (2F'(X + Y) + F'^2) below this keeps the sum in
-// parentheses, and with it every intermediate of m(u) in float, below 2.2e37.
-// From it on m(u) may overflow on the way to a small value.
-constexpr float BOUND_MAX = 1e31f;
-
 // Above 4|u - q|^2 with margin, for the user at offset (x, y) from q.
 __device__ __forceinline__ float user_lim(float x, float y)
 {
     return 4.0f * fmaf(x, x, y * y) * (1.0f + 1e-4f) + 1e-30f;
-}
-
-// The FP32 evaluation bound of the user at offset (x, y), infinite from
-// BOUND_MAX on: no half-plane is certain for the user then.
-__device__ __forceinline__ float user_bound(const QDesc& d, float x, float y)
-{
-    const float b = fmaf(d.k2f, fabsf(x) + fabsf(y), d.kf2);
-    return b < BOUND_MAX ? b : INFINITY;
 }
 
 // Stage 1, FP32, over the slot's first nb half-planes: cnt = certified
@@ -127,7 +114,7 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
         x[t] = u[t].x - d.qx;
         y[t] = u[t].y - d.qy;
         lim[t] = user_lim(x[t], y[t]);
-        bu[t] = user_bound(d, x[t], y[t]);
+        bu[t] = fmaf(d.k2f, fabsf(x[t]) + fabsf(y[t]), d.kf2);
     }
     const int k = d.k;
     int m = 0;
@@ -206,12 +193,9 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
         if (!stopped && ns < nb) sweep(gp, nb);
     evals += (unsigned)(m * nvalid);
     bool again = false;
-    unsigned top[UPT];
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {
-        // (an infinite bound: r is infinite or, where m overflowed, a NaN)
-        top[t] = bu[t] < INFINITY ? __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f))) : 0x7fffffffu;
-        und[t] = rmin[t] <= top[t];
+        und[t] = rmin[t] <= __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
         again |= und[t] && cnt[t] < k && !(lim[t] > rho2);
     }
     if constexpr (COMPACT)
@@ -228,7 +212,8 @@ __device__ __forceinline__ void filter_users(const QDesc& d, int nb, const char*
                 const float4 p = i < ns ? ((const float4*)sp)[i] : gp[i];
 #pragma unroll
                 for (int t = 0; t < UPT; ++t)
-                    nc[t] += __float_as_uint(fmaf(p.x, x[t], fmaf(p.y, y[t], p.z)) + bu[t]) <= top[t];
+                    nc[t] += __float_as_uint(fmaf(p.x, x[t], fmaf(p.y, y[t], p.z)) + bu[t]) <=
+                             __float_as_uint(__fmul_ru(bu[t], 2.0f * (1.0f + 0x1p-20f)));
             }
 #pragma unroll
             for (int t = 0; t < UPT; ++t) und[t] = und[t] && cnt[t] + nc[t] >= k;
@@ -506,7 +491,12 @@ __device__ __forceinline__ void verify_item(const VerifyArgs& A, const QDesc& d,
     bool valid[UPT];
     item_users<UPT>(A, d, s, v0, sg, sr, region_in >= 0, pos, u, valid, vc);
     int cnt[UPT], und[UPT];
-    filter_users<UPT, COMPACT>(d, nbs, sp, ns, gp, u, valid, cnt, und, vc.evals, item_rho2(d, nbs));
+    if (d.kf2 < INFINITY) {
+        filter_users<UPT, COMPACT>(d, nbs, sp, ns, gp, u, valid, cnt, und, vc.evals, item_rho2(d, nbs));
+    } else {
+#pragma unroll
+        for (int t = 0; t < UPT; ++t) { cnt[t] = 0; und[t] = 1; }       // counted exactly
+    }
     bool direct[UPT], surv[UPT];
 #pragma unroll
     for (int t = 0; t < UPT; ++t) {

@@ -840,7 +840,8 @@ __device__ __forceinline__ void zone_body(const ZoneArgs& A)
         const double Fp = sqrt(cmax) * (1.0 + 1e-6) + 1e-30;
         // per-user bound 8u (2F'(|x'|+|y'|) + F'^2)
         const float k2f = (float)(8.0 * (double)kU32 * 2.0 * Fp * (1.0 + 1e-6));
-        const float kf2 = (float)(8.0 * (double)kU32 * Fp * Fp * (1.0 + 1e-6)) + 1e-30f;
+        const float kf2 = filter_bound(k2f, (float)(8.0 * (double)kU32 * Fp * Fp * (1.0 + 1e-6)) + 1e-30f,
+                                       (fsx1 - fsx0) + (fsy1 - fsy0));
         const double k2f64 = 8.0 * kU64 * 2.0 * Fp * (1.0 + 1e-6);
         const double kf264 = 8.0 * kU64 * Fp * Fp * (1.0 + 1e-6) + 1e-300;
         WSYNC();
