@@ -683,12 +683,6 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     if (mode == MODE_FP64 && ix->vupt_auto &&
         (double)nq * std::max(1.0, 2.0 * kmax * (double)ix->nu / (double)ix->nf / VERIFY_CHUNK) < 24.0 * ix->num_sms)
         b.vupt = 2;
-    // batches with more slots than the GPU has verification warps (3,648): a
-    // warp takes up to four parts of a slot in turn and finds the slot, its
-    // segments and half-planes once (verification of 16,384 queries, one part
-    // against four: street layout 1.92 -> 1.75 ms FP32, 3.20 -> 2.94 FP64;
-    // uniform k=10 139 -> 134 us); smaller batches need the items
-    b.parts = nq >= 16384 ? 4 : nq >= 8192 ? 2 : 1;
     // (half-planes beyond these are left out: the filter weakens, the exact
     // recount still decides)
     b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
@@ -716,6 +710,15 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     b.vsmem = (size_t)b.vwarps * verify_warp_bytes(b.stage_cap, b.seg_stage);
     const int vper = occupancy(ix, (const void*)verify_fn(mode, b.vupt), b.vwarps * 32, b.vsmem);
     b.vgrid = vper * ix->num_sms;
+    // slots that outnumber the resident verification warps (3,648 of them) several
+    // times: a warp takes two or four parts of a slot in turn and finds the slot,
+    // its segments and half-planes once (verification, us, one / two / four parts:
+    // street layout k=10 7,500 queries 242 / 215 / 209, 15,000 467 / 414 / 395, FP64
+    // 903 / 848 / 819; uniform k=10 15,000 94 / 86 / 84; but FP64 uniform k=40 735 /
+    // 756 / 805 at 7,500 and 422 / 453 / 496 at 4,000, where the warps need the
+    // items)
+    const int per_warp = nq / (b.vgrid * b.vwarps);
+    b.parts = per_warp >= 4 ? 4 : per_warp >= 2 ? 2 : 1;
     if ((long long)kmax * ix->nu >= (long long)SORT_MIN_MEAN * ix->nf)
         b.sort_grid = std::min(nq, occupancy(ix, (const void*)sort_large_kernel, SORT_THREADS, sort_large_smem()) * ix->num_sms);
     b.key.push_back(b.sort_grid);

@@ -28,3 +28,19 @@ def test_both_sides_of_the_line(engine, nf, nu, ks):
                     kk = rng.choice(ks, n).astype(np.int32) if mixed else np.full(n, k, np.int32)
                     for q, k1, got in zip(qs, kk, idx.query_batch(qs, kk, "fp32")):
                         assert np.array_equal(got, want[(int(q), int(k1))]), (int(q), int(k1), n)
+
+
+@pytest.mark.parametrize("nq", [7295, 7296, 14_591, 14_592])
+def test_parts_of_an_item(engine, nq):
+    """Items of one, two and four parts on either side of where the queries
+    outnumber the resident warps (3,648 at these half-planes) two and four times."""
+    ds = datagen.uniform(900, 30_011, seed=76, nq=40, k=1)
+    o = O.Oracle.of(ds)
+    want = {k: [o.query(int(q), k) for q in ds.queries] for k in (2, 9, 35)}
+    with engine.Index.of(ds) as idx:
+        for k, w in want.items():
+            for mode in ("fp32", "fp64"):
+                got, off = idx.query_batch_flat(np.resize(ds.queries, nq).astype(np.int32), k, mode)
+                assert np.array_equal(np.diff(off), np.resize([x.size for x in w], nq)), (nq, k, mode)
+                for i in [*range(40), *range(nq - 40, nq)]:
+                    assert np.array_equal(got[off[i]:off[i + 1]], w[i % 40]), (nq, k, mode, i)
