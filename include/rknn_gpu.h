@@ -259,7 +259,7 @@ rknn_status rknn_last_kernel_ms(rknn_index* idx, double* ms);
  * are submitted; whenever one of the server's slots is free, the worker
  * forms a batch from the queue (first come first served, one mode per batch,
  * as many requests as max_batch and the slot's scratch budget admit, the
- * budget charged by each request's scratch estimate from its k) and launches
+ * budget charged by what the batch's queries take at its largest k) and launches
  * it on the slot's own stream while earlier batches are still running, so
  * the work of several batches overlaps on the GPU.  A request's result does
  * not depend on the batch it ran in. */
@@ -290,8 +290,9 @@ rknn_status rknn_serve_start(rknn_index* idx, const rknn_serve_opts* opts, rknn_
 /* Queue one request; *ticket identifies it in rknn_serve_wait.  Thread-safe.
  * Admission rule: a request whose scratch estimate on its own (a batch of
  * one, padded as batches are) exceeds the server's scratch_bytes is refused
- * with RKNN_ERR_CAPACITY, so no batch passes the budget; other requests are
- * combined first come first served while the batch's estimate fits. */
+ * with RKNN_ERR_CAPACITY, so no batch passes the budget (a request that fits
+ * only by that estimate runs within it, with fewer half-planes); other requests
+ * are combined first come first served while the batch fits. */
 rknn_status rknn_serve_submit(rknn_server* srv, int32_t q_index, int32_t k, int32_t mode,
                               uint64_t* ticket);
 

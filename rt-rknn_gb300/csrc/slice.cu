@@ -721,7 +721,9 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
         // as one range each: a query next to an empty direction walks far
         // through mostly empty cells, a load's latency for 32 of them.  (Later
         // than the rings that ordinary queries reach, where whole blocks would
-        // stream too many facilities.)  Clustered workload, 2000 queries:
+        // stream too many facilities: those that get there stream up to 24 %
+        // more of them, the filter of 1500 uniform queries at k=1000 30.8 ->
+        // 30.6 ms, at k=1400 44.9 -> 45.3.)  Clustered workload, 2000 queries:
         // filter 1.06 -> 0.56 ms, the slowest query 2.2 -> 1.2 M cycles.  One
         // warp a query only: with this code the two-warp kernels' ordinary
         // queries take 4 % longer (single FP32 queries 453 -> 473 us for
@@ -1067,8 +1069,9 @@ __device__ __forceinline__ void slice_body(const ZoneArgs& A)
 #undef SLICE_KTH
 
 // The one-warp variants' registers are capped where more queries in flight pay
-// for shorter chains (filter of 16,384 uniform queries at k=10: 133 registers
-// 254 us, 121 (16 blocks an SM) 212, 104 (18) 196, 20 blocks 196, 24 201).
+// for shorter chains (filter of 16,384 uniform queries at k=10 by blocks an SM:
+// uncapped 254 us, 16 212, 18 196, 20 196, 24 201; at 18, 96 registers, r10 spills
+// 4 bytes and r12 16).
 __global__ void __launch_bounds__(32, 1) slice_kernel(ZoneArgs A) { slice_body<0, 1>(A); }
 __global__ void __launch_bounds__(32, 18) slice_kernel_r4(ZoneArgs A) { slice_body<4, 1>(A); }
 __global__ void __launch_bounds__(32, 18) slice_kernel_r8(ZoneArgs A) { slice_body<8, 1>(A); }

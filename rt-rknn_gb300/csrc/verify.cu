@@ -12,9 +12,9 @@
 // exceeds the float (or double) evaluation error of m_f (at most
 // 4.01u(|a x'| + |b y'| + |c|)).  Lanes own users (coalesced float2 loads,
 // four per lane); the warp leaves the half-plane loop as soon as every lane
-// has k certified violations for all its users (__all_sync).  In slots of many
-// candidates, and in FP64 always, the users' bounding boxes are tested first
-// (verify_box.cuh).
+// has k certified violations for all its users (__all_sync).  Where it is
+// cheaper (boxes_first), and in FP64 always, the users' bounding boxes are tested
+// first (verify_box.cuh).
 //
 // Stage 2 (exact count).  Users that survive stage 1 go to a survivor list,
 // and recount_kernel counts each one exactly, a warp (or a group of up to
@@ -192,10 +192,11 @@ __device__ __forceinline__ void verify_body(const VerifyArgs& A)
 
 // The verification kernel with 2, 4 or 8 users per lane per work item
 // (32 * UPT users per item), for either precision mode; blocks of up to 16
-// warps.  80 registers (24 warps an SM): FP64 needs the warps to issue beside
-// the FP64 pipe (street layout with 126 / 80 / 64 registers: 2.49 / 2.27 /
-// 2.25 ms; 1000 uniform queries: 41 / 43 / 45 us), FP32 with 64 spills more
-// (1.46 -> 1.54 ms).
+// warps.  80 registers (24 warps an SM), which spill about 25 registers each
+// (94 bytes of stores and 176 of loads a thread in FP32, 104 and 164 in FP64):
+// FP64 needs the warps to issue beside the FP64 pipe (street layout with 126 / 80 /
+// 64 registers: 2.49 / 2.27 / 2.25 ms; 1000 uniform queries: 41 / 43 / 45 us), FP32
+// with 64 spills still more (1.46 -> 1.54 ms).
 __global__ void __maxnreg__(80) verify_kernel(VerifyArgs a) { verify_body<4, false>(a); }
 __global__ void __maxnreg__(80) verify_kernel_u2(VerifyArgs a) { verify_body<2, false>(a); }
 __global__ void __launch_bounds__(512) verify_kernel_u8(VerifyArgs a) { verify_body<8, false>(a); }

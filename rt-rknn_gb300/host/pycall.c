@@ -3,8 +3,9 @@
 // rknn_serve_wait.  The ctypes route costs microseconds a call in Python (a
 // pointer object per array, conversion of up to nine arguments), a large share
 // of the host time of a 1000-query call and most of a served request's; these
-// parse the arguments in C and release the interpreter lock around the call.  rknn.py uses it when it was built (the CPython headers are needed)
-// and ctypes otherwise: both call the same C entry points.
+// parse the arguments in C and release the interpreter lock around the call.
+// rknn.py uses them when they were built (the CPython headers are needed) and
+// ctypes otherwise: both call the same C entry points.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>

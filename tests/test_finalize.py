@@ -3,7 +3,7 @@
 With one facility every user is in its result set, so a set has exactly as
 many ids as there are users, whatever k: the sizes here sit at the edges of
 the sort's classes (32, 64, 128, 256 and 512 ids, and the block's radix sort
-beyond, by tiles of 8192).  Beside a few hundred facilities far from every
+beyond, by tiles of 16,384).  Beside a few hundred facilities far from every
 user the same sets are few in their batch, and warps sort the large ones.
 """
 import numpy as np
