@@ -686,7 +686,7 @@ BatchPlan plan_batch(rknn_index* ix, int nq, int mode, bool use_order, const int
     // (half-planes beyond these are left out: the filter weakens, the exact
     // recount still decides)
     b.stage_cap = std::max(1, std::min(b.pstride, VERIFY_PLANES_MAX));
-    if (nq <= LIST_QUERIES && std::none_of(b.cls.begin(), b.cls.end(), [](const ZClass& c) { return c.slice; }))
+    if (mode == MODE_FP64 && nq <= LIST_QUERIES && std::none_of(b.cls.begin(), b.cls.end(), [](const ZClass& c) { return c.slice; }))
         b.list_cand = LIST_CAND;
     b.box_batch = boxes_first(kmax / 2, (int)std::min(1e9, 1.5 * kmax * (double)ix->nu / (double)ix->nf));
     int rm = 0;

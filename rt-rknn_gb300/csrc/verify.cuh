@@ -28,14 +28,16 @@ __host__ __device__ __forceinline__ bool boxes_first(int k, int n)
 // k to 24 547 / 416, to 50 864 / 997, to 100 1488 / 1787, 50 users a facility
 // k to 32 432 / 346, to 64 684 / 746, clustered k to 50 860 / 839, to 100 1743 / 1840).
 constexpr int BOX_MIN_CAND = 512;
-// Most queries of an influence-zone batch, and candidates of a query, that go
-// to the recount without a half-plane test.  The zone's half-planes reject
+// Most queries of an FP64 influence-zone batch, and candidates of a query, that
+// go to the recount without a half-plane test.  The zone's half-planes reject
 // about half of the candidates and accept none (its pruning may have dropped a
 // needed facility, so those left are counted anyway), and a few queries leave
 // most warps idle: counting all candidates takes the recount no longer, and the
 // half-plane tests' chain is saved (one FP64 query at k=10: verification
 // 26 -> 8 us; single queries at k=10, uniform 499 -> 468 us, clustered 571 -> 538,
-// street 522 -> 490, ten at a time 563 -> 530, 1146 -> 1138, 646 -> 609).
+// street 522 -> 490, ten at a time 563 -> 530, 1146 -> 1138, 646 -> 609).  In FP32
+// the chain is short: one query takes 406 us either way, sixteen with 50 users a
+// facility at k=3 229 listed, 223 tested.
 constexpr int LIST_QUERIES = 16, LIST_CAND = 4096;
 constexpr int VERIFY_PLANES_MAX = 1024;             // half-planes used per slot (32 box masks of 32)
 constexpr int FIN_WARPS = 8;                        // finalize: slots per block (one warp each)
