@@ -794,6 +794,7 @@ rknn_status enqueue(rknn_index* ix, Ctx& c, const BatchPlan& b, bool events = fa
     va.parts = b.parts;
     va.list_cand = b.list_cand;
     va.box_batch = b.box_batch;
+    va.alike = std::none_of(b.cls.begin(), b.cls.end(), [](const ZClass& z) { return z.slice; });
     va.segs = w.d_segs; va.seg_cap = w.seg_cap; va.seg_stage = b.seg_stage;
     va.chunk_off = w.d_chunk_off; va.cand_off = w.d_cand_off; va.reg_len = w.d_reg_len; va.nq = nq;
     va.uxy = ix->d_uxy; va.uid = ix->d_uid; va.fxy = ix->d_fxy; va.fstart = ix->d_fstart; va.gf = ix->gf;

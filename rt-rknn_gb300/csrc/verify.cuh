@@ -81,6 +81,7 @@ struct VerifyArgs {
     int surv_cap;            // 0: no list (the verification kernel recounts in-warp)
     int* surv_count;
     int* recount_counter = nullptr;    // recount_kernel's queue
+    bool alike = false;      // an influence-zone batch: its survivors cost much the same
     int* fault;              // checked builds: {flag, array id, index, size, line}
     // slots to verify: chunk_off indexes deflist[0 .. *ndef) when deflist is
     // set (the fused slice filter verified the others), else slots 0 .. nq
